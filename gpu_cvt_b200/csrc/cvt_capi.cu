@@ -1022,13 +1022,76 @@ __global__ void k_fill_int(int* p, int n, int v) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) p[i] = v;
 }
-__global__ void k_f32_to_f64(const float* a, double* b, long n) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = (double)a[i];
+
+// Place the sites of new segments in internal order: thread t takes the t-th
+// of their cell-ordered copy (id: caller index), the site slot base + t, and
+// gives the slot its initial state.
+template <class T>
+__global__ void k_place_sites(EngineArgs<T> a, int parity, int n, const Pt4<float>* __restrict__ ordered, int base, int seg,
+                              const int* __restrict__ raw_seg, int* __restrict__ site_seg, uint32_t* __restrict__ internal_of) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const Pt4<float> p = ordered[t];
+  const int g = base + t;
+  const uint32_t caller = (uint32_t)base + p.id;
+  a.S[parity][g] = Pt4<T>{(T)p.x, (T)p.y, (T)p.z, caller};
+  internal_of[caller] = (uint32_t)g;
+  site_seg[g] = raw_seg ? raw_seg[p.id] : seg;
+#pragma unroll
+  for (int k = 0; k < kKProj; ++k) a.knnv[k * a.stride + g] = -1;
+  a.frozen[g] = a.streak[g] = a.tier[g] = a.same[g] = 0;
+  a.kth[g] = -1.f;
+  if (a.cand_rho) a.cand_rho[g] = -1.f;  // no candidate list yet
 }
-__global__ void k_f64_to_f32(const double* a, float* b, long n) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = (float)a[i];
+
+// segment of every site of a freshly filled engine (segments in site order)
+__global__ void k_raw_segments(const SegDev* __restrict__ segs, int nseg, int n, int* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int lo = 0, hi = nseg - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (segs[mid].site_base <= i) lo = mid; else hi = mid - 1;
+  }
+  out[i] = lo;
+}
+
+// Sites of the slots [first, first + n) in the caller's order, as O, at out +
+// 3 * (caller index - first).  A segment's current buffer follows from its
+// placement parity and the iterations it has done (a segment stopped by its
+// stop rule keeps its sites where its last iteration wrote them).
+template <class T, class O>
+__global__ void k_export_sites(EngineArgs<T> a, int first, int n, O* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int s = a.site_seg[first + i];
+  if (s < 0) return;
+  const SegDev& sd = a.segs[s];
+  const Pt4<T> p = a.S[(sd.p0 + sd.iter) & 1][first + i];
+  st3(out, (long)p.id - first, V3<O>{(O)p.x, (O)p.y, (O)p.z});
+}
+
+// The per-site state of one segment in the caller's order and indices (any
+// pointer may be NULL).
+template <class T>
+__global__ void k_export_state(EngineArgs<T> a, int seg, uint32_t* __restrict__ knn, int* __restrict__ knnv,
+                               uint8_t* __restrict__ frozen, uint8_t* __restrict__ tier) {
+  const SegDev& sd = a.segs[seg];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= sd.n_sites) return;
+  const int base = sd.site_base, g = base + i;
+  const Pt4<T>* S = a.S[(sd.p0 + sd.iter) & 1];
+  const size_t o = S[g].id - (uint32_t)base;
+  if (knn)
+    for (int t = 0; t < a.K; ++t) {
+      const uint32_t j = a.list[t * a.stride + g];
+      // before the first iteration there is no list yet
+      knn[o * a.K + t] = sd.iter == 0 ? 0u : j == 0xffffffffu ? j : S[j].id - (uint32_t)base;
+    }
+  if (knnv)
+    for (int k = 0; k < kKProj; ++k) knnv[o * kKProj + k] = a.knnv[k * a.stride + g];
+  if (frozen) frozen[o] = a.frozen[g];
+  if (tier) tier[o] = a.tier[g];
 }
 
 struct cvt_engine {
@@ -1055,7 +1118,8 @@ struct cvt_engine {
   MeshDev* d_meshes = nullptr;
   int* d_site_seg = nullptr;
   void* d_S[2] = {nullptr, nullptr};
-  uint32_t* d_knn = nullptr;
+  uint32_t* d_internal_of = nullptr;
+  uint32_t* d_list = nullptr;   // list_len() entries per site: the K-list, with knn_reuse the candidate list
   uint8_t* d_same = nullptr;
   float* d_kth = nullptr;
   int* d_act = nullptr;
@@ -1077,19 +1141,18 @@ struct cvt_engine {
                                   // [2] BVH stack overflows of the projection (never expected)
   int num_sms = 148;
   void* d_cent = nullptr;
-  uint32_t* d_cand = nullptr;   // candidate lists (knn_reuse): cand_len(K) global ids per site
   float* d_cand_rho = nullptr;
   float* d_cand_D = nullptr;
-  int* d_srch = nullptr;          // sites left for a full KNN search, srch_cap slots per verify warp
-  float* d_srch_thr = nullptr;    // per slot: the check's bound on the site's MM-th distance
-  int* d_srch_n = nullptr;
-  int srch_cap = 0;
+  int* d_srch = nullptr;          // count, sites left for a full KNN search
+  float* d_srch_thr = nullptr;    // the check's bound on each one's MM-th distance
   unsigned long long* d_blockmax = nullptr;  // per cell slot: coarse-block motion of the last step
   // graphs
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-  // fork / join of the frame-vertex search, which runs on a second stream
-  // while the site KNN runs: for eager iterations and for graph captures
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_cfork = nullptr, ev_cjoin = nullptr;
+  // fork / joins of the second stream, which builds the grid beside the list
+  // check and finds the frame vertices beside the KNN: for eager iterations
+  // and for graph captures
+  cudaEvent_t ev_fork = nullptr, ev_grid = nullptr, ev_join = nullptr;
+  cudaEvent_t ev_cfork = nullptr, ev_cgrid = nullptr, ev_cjoin = nullptr;
   int graph_nodes = 0;
   long long last_launches = 0;
 };
@@ -1161,7 +1224,7 @@ static void engine_free(cvt_engine* e) {
   if (!e) return;
   for (int k = 0; k < 2; ++k)
     if (e->gexec[k]) graph_cache_put(graph_key(e), e->gexec[k]);
-  for (cudaEvent_t ev : {e->ev_fork, e->ev_join, e->ev_cfork, e->ev_cjoin})
+  for (cudaEvent_t ev : {e->ev_fork, e->ev_grid, e->ev_join, e->ev_cfork, e->ev_cgrid, e->ev_cjoin})
     if (ev) cudaEventDestroy(ev);
   dev_free_sync(e->arena);
   delete e;
@@ -1176,6 +1239,9 @@ static constexpr int cand_len(int k) { return k + 16 > 64 ? 64 : k + 16; }
 // sized for the candidate list's length made its full searches cheaper but
 // the coarse motion blocks coarser, which kept fewer lists: slower overall.)
 static double grid_neighbours(const cvt_params_t& p) { return (double)(p.k + 1); }
+
+static size_t pt_bytes(const cvt_engine* e) { return e->f64 ? sizeof(Pt4<double>) : sizeof(Pt4<float>); }
+template <class T> static EngineArgs<T> engine_args(cvt_engine* e);
 
 static bool k_supported(int k) { return k == 8 || k == 12 || k == 16 || k == 20 || k == 24 || k == 32; }
 
@@ -1212,7 +1278,7 @@ extern "C" cvt_status_t cvt_engine_create(const cvt_params_t* p, int max_segment
   e->site_alloc.init(max_sites);
   e->cell_alloc.init(max_cells);
   const size_t tsz = e->f64 ? sizeof(double) : sizeof(float);
-  const size_t psz = e->f64 ? sizeof(Pt4<double>) : sizeof(Pt4<float>);
+  const size_t psz = pt_bytes(e);
   cudaError_t err = cudaSuccess;
 #define ECK(x)                                                                               \
   do {                                                                                       \
@@ -1230,8 +1296,9 @@ extern "C" cvt_status_t cvt_engine_create(const cvt_params_t* p, int max_segment
   ar.add(&e->d_active, max_segments);
   ar.add(&e->d_meshes, max_segments);
   ar.add(&e->d_site_seg, ns);
-  for (int k = 0; k < 2; ++k) ar.add(reinterpret_cast<char**>(&e->d_S[k]), tsz * 3 * ns);
-  ar.add(&e->d_knn, (size_t)e->K * ns);
+  for (int k = 0; k < 2; ++k) ar.add(reinterpret_cast<char**>(&e->d_S[k]), psz * ns);
+  ar.add(&e->d_internal_of, ns);
+  ar.add(&e->d_list, (size_t)(q.knn_reuse ? cand_len(e->K) : e->K) * ns);
   ar.add(&e->d_same, ns);
   ar.add(&e->d_kth, ns);
   ar.add(&e->d_act, ns);
@@ -1252,13 +1319,10 @@ extern "C" cvt_status_t cvt_engine_create(const cvt_params_t* p, int max_segment
   ar.add(&e->d_tickets, 3);  // scan ticket, bookkeeping ticket, BVH stack overflows
   ar.add(reinterpret_cast<char**>(&e->d_cent), tsz * 3 * ns);
   if (q.knn_reuse) {
-    ar.add(&e->d_cand, (size_t)cand_len(e->K) * ns);
     ar.add(&e->d_cand_rho, ns);
     ar.add(&e->d_cand_D, ns);
-    e->srch_cap = (int)cdiv((long)ns, (long)e->num_sms * kKnnVerifyWarpsPerSM) + 2;  // two sites per warp step
-    ar.add(&e->d_srch, (size_t)e->srch_cap * e->num_sms * kKnnVerifyWarpsPerSM);
-    ar.add(&e->d_srch_thr, (size_t)e->srch_cap * e->num_sms * kKnnVerifyWarpsPerSM);
-    ar.add(&e->d_srch_n, (size_t)e->num_sms * kKnnVerifyWarpsPerSM);
+    ar.add(&e->d_srch, ns + 1);
+    ar.add(&e->d_srch_thr, ns);
     ar.add(&e->d_blockmax, (size_t)max_cells);
   }
   ECK(ar.commit(&e->arena));
@@ -1267,7 +1331,7 @@ extern "C" cvt_status_t cvt_engine_create(const cvt_params_t* p, int max_segment
   k_fill_int<<<cdiv((long)ns, 256), 256>>>(e->d_site_seg, (int)ns, -1);
   LAUNCHED(1);
   ECK(cudaGetLastError());
-  for (cudaEvent_t* ev : {&e->ev_fork, &e->ev_join, &e->ev_cfork, &e->ev_cjoin})
+  for (cudaEvent_t* ev : {&e->ev_fork, &e->ev_grid, &e->ev_join, &e->ev_cfork, &e->ev_cgrid, &e->ev_cjoin})
     ECK(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
   ECK(cudaDeviceSynchronize());
 #undef ECK
@@ -1282,14 +1346,26 @@ extern "C" cvt_status_t cvt_engine_destroy(cvt_engine_t e) {
   return CVT_OK;
 }
 
-// defer_tables: leave the segment's entries of the device tables (segment,
-// grid geometry, mesh view, active flag) and the final wait to the caller,
-// which uploads the tables of many segments at once (each small copy from
-// pageable host memory waits for the stream); the sites buffer must then
-// stay valid until the stream has passed this segment's copy.
+// The sites of n consecutive slots from base on, cell-ordered copy in
+// `ordered`, into the engine with their initial state (k_place_sites).
+static cvt_status_t place_sites(cvt_engine* e, const Pt4<float>* ordered, int n, int base, int seg, const int* raw_seg,
+                                cudaStream_t st) {
+  if (e->f64)
+    k_place_sites<double><<<cdiv(n, 256), 256, 0, st>>>(engine_args<double>(e), e->parity, n, ordered, base, seg, raw_seg,
+                                                       e->d_site_seg, e->d_internal_of);
+  else
+    k_place_sites<float><<<cdiv(n, 256), 256, 0, st>>>(engine_args<float>(e), e->parity, n, ordered, base, seg, raw_seg,
+                                                      e->d_site_seg, e->d_internal_of);
+  CKLAUNCH();
+  return CVT_OK;
+}
+
+// raw (remesh_batch): only reserve the segment's slots and cells in the host
+// mirrors of a freshly created engine; the caller has all segments' sites in
+// one device array and places them at once (place_all_segments).
 static cvt_status_t add_segment_impl(cvt_engine* e, cvt_mesh_t mesh, const float* sites, int n, int sites_on_device,
-                                     int* seg_id, cudaStream_t st, bool defer_tables) {
-  if (!e || !mesh || !sites || n < 1 || !seg_id) return fail(CVT_ERR_INVALID, "cvt_engine_add_segment: bad arguments");
+                                     int* seg_id, cudaStream_t st, bool reserve_only) {
+  if (!e || !mesh || (!sites && !reserve_only) || n < 1 || !seg_id) return fail(CVT_ERR_INVALID, "cvt_engine_add_segment: bad arguments");
   int s = -1;
   for (int k = 0; k < e->max_seg; ++k) if (!e->active[k] && !e->seg_mesh[k]) { s = k; break; }
   if (s < 0) return fail(CVT_ERR_CAPACITY, "cvt_engine_add_segment: no free segment slot");
@@ -1315,6 +1391,7 @@ static cvt_status_t add_segment_impl(cvt_engine* e, cvt_mesh_t mesh, const float
   sd.kth_est = (float)(2.0 * (e->K + 1) * (double)mesh->area / (M_PI * (double)n));
   sd.stop_motion2 = -1.f;
   sd.stop_iters = 0;
+  sd.p0 = e->parity;
   MeshDev md = mesh->dev();
   static const int kStreak1[6] = {5, 10, 15, 20, 25, 25};  // main.cu:22, 543-553
   static const int kStreak2[6] = {5, 10, 15, 20, 25, 10};  // main.cu:39, 554-563
@@ -1330,47 +1407,30 @@ static cvt_status_t add_segment_impl(cvt_engine* e, cvt_mesh_t mesh, const float
   e->seg_cells[s] = cells;
   e->host_iters[s] = 0;
   e->seg_p0[s] = e->parity;
-  const size_t tsz = e->f64 ? sizeof(double) : sizeof(float);
-  if (!defer_tables) {
-    CK(cudaMemcpyAsync(e->d_segs + s, &e->segs[s], sizeof(SegDev), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(e->d_geom + s, &e->geom[s], sizeof(GridGeom), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(e->d_meshes + s, &md, sizeof(MeshDev), cudaMemcpyHostToDevice, st));
-  }
-  char* Sdst = (char*)e->d_S[e->parity] + tsz * 3 * (size_t)base;
-  if (!e->f64) {
-    CK(cudaMemcpyAsync(Sdst, sites, sizeof(float) * 3 * (size_t)n,
-                       sites_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
-  } else {
-    const float* src = sites;
+  *seg_id = s;
+  if (reserve_only) return CVT_OK;
+  CK(cudaMemcpyAsync(e->d_segs + s, &e->segs[s], sizeof(SegDev), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(e->d_geom + s, &e->geom[s], sizeof(GridGeom), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(e->d_meshes + s, &md, sizeof(MeshDev), cudaMemcpyHostToDevice, st));
+  {
     Scratch sc(st);
+    const float* src = sites;
     if (!sites_on_device) {
       float* tmp;
       CK(sc.get(&tmp, 3 * (size_t)n));
       CK(cudaMemcpyAsync(tmp, sites, sizeof(float) * 3 * (size_t)n, cudaMemcpyHostToDevice, st));
       src = tmp;
     }
-    k_f32_to_f64<<<cdiv(3L * n, 256), 256, 0, st>>>(src, (double*)Sdst, 3L * n);
-    CKLAUNCH();
+    GridGeom own = g;
+    own.cell_base = 0;
+    PointGrid pg;
+    cvt_status_t r = build_point_grid(sc, src, n, 0.f, &own, pg);
+    if (r == CVT_OK) r = place_sites(e, pg.sorted, n, base, s, nullptr, st);
+    if (r != CVT_OK) return r;
   }
-  k_fill_int<<<cdiv(n, 256), 256, 0, st>>>(e->d_site_seg + base, n, s);
-  CKLAUNCH();
-  k_fill_int<<<cdiv(5L * n, 256), 256, 0, st>>>(e->d_knnv + 5L * base, 5 * n, -1);
-  CKLAUNCH();
-  CK(cudaMemsetAsync(e->d_frozen + base, 0, n, st));
-  CK(cudaMemsetAsync(e->d_streak + base, 0, n, st));
-  CK(cudaMemsetAsync(e->d_tier + base, 0, n, st));
-  CK(cudaMemsetAsync(e->d_knn + (size_t)e->K * base, 0, sizeof(uint32_t) * e->K * (size_t)n, st));
-  CK(cudaMemsetAsync(e->d_same + base, 0, n, st));
-  k_fill_int<<<cdiv(n, 256), 256, 0, st>>>(reinterpret_cast<int*>(e->d_kth) + base, n, (int)0xbf800000);  // -1.0f
-  CKLAUNCH();
-  if (e->d_cand_rho) {  // no candidate lists yet; no motion recorded in the segment's blocks
-    k_fill_int<<<cdiv(n, 256), 256, 0, st>>>(reinterpret_cast<int*>(e->d_cand_rho) + base, n, (int)0xbf800000);
-    CKLAUNCH();
+  if (e->d_blockmax)  // no motion recorded in the segment's blocks
     CK(cudaMemsetAsync(e->d_blockmax + cbase, 0, sizeof(unsigned long long) * (size_t)cells, st));
-  }
   CK(cudaMemsetAsync(e->d_stats + (size_t)s * kStatsRing * kStatsWords, 0, sizeof(int) * kStatsRing * kStatsWords, st));
-  *seg_id = s;
-  if (defer_tables) return CVT_OK;
   CK(cudaMemcpyAsync(e->d_active + s, &e->active[s], sizeof(int), cudaMemcpyHostToDevice, st));
   // the host mirrors above are read by the async copies; keep them stable
   CK(cudaStreamSynchronize(st));
@@ -1382,9 +1442,11 @@ extern "C" cvt_status_t cvt_engine_add_segment(cvt_engine_t e, cvt_mesh_t mesh, 
   return add_segment_impl(e, mesh, sites, n, sites_on_device, seg_id, S_(stream), false);
 }
 
-// The device tables of every segment slot from the host mirrors, in four
-// copies, then a wait (after add_segment_impl with defer_tables).
-static cvt_status_t upload_segment_tables(cvt_engine* e, cudaStream_t st) {
+// Fill a freshly created engine whose segments were reserved in slot order:
+// the device tables from the host mirrors in four copies (each small copy
+// from pageable memory waits for the stream), and every segment's sites (raw:
+// n sites in slot order) through one grid build over all of them.
+static cvt_status_t place_all_segments(cvt_engine* e, const float* raw, int n, cudaStream_t st) {
   std::vector<MeshDev> md(e->max_seg);
   for (int k = 0; k < e->max_seg; ++k)
     if (e->seg_mesh[k]) md[k] = e->seg_mesh[k]->dev();
@@ -1392,6 +1454,23 @@ static cvt_status_t upload_segment_tables(cvt_engine* e, cudaStream_t st) {
   CK(cudaMemcpyAsync(e->d_geom, e->geom.data(), sizeof(GridGeom) * e->max_seg, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(e->d_meshes, md.data(), sizeof(MeshDev) * e->max_seg, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(e->d_active, e->active.data(), sizeof(int) * e->max_seg, cudaMemcpyHostToDevice, st));
+  Scratch sc(st);
+  int* seg;
+  int2* rank;
+  Pt4<float>* ordered;
+  CK(sc.get(&seg, (size_t)n));
+  CK(sc.get(&rank, (size_t)n));
+  CK(sc.get(&ordered, (size_t)n));
+  k_raw_segments<<<cdiv(n, 256), 256, 0, st>>>(e->d_segs, e->max_seg, n, seg);
+  CKLAUNCH();
+  // the engine's own cell arrays: the scan leaves the counts at zero again
+  k_grid_count<float><<<cdiv(n, 256), 256, 0, st>>>(n, raw, SegGrid{e->d_geom, seg, nullptr}, e->d_cell_count, rank);
+  CKLAUNCH();
+  LAUNCHED(launch_exclusive_scan(e->max_cells, e->d_cell_count, e->d_part, e->d_cell_start, st, true, e->d_tickets));
+  k_grid_scatter<float><<<cdiv(n, 256), 256, 0, st>>>(n, raw, rank, e->d_cell_start, ordered);
+  CKLAUNCH();
+  cvt_status_t r = place_sites(e, ordered, n, 0, -1, seg, st);
+  if (r != CVT_OK) return r;
   CK(cudaStreamSynchronize(st));
   return CVT_OK;
 }
@@ -1415,47 +1494,51 @@ constexpr int kCellCap = 16;
 template <class T> static EngineArgs<T> engine_args(cvt_engine* e) {
   EngineArgs<T> a;
   a.segs = e->d_segs; a.geom = e->d_geom; a.active = e->d_active; a.meshes = e->d_meshes; a.site_seg = e->d_site_seg;
-  a.S[0] = (T*)e->d_S[0]; a.S[1] = (T*)e->d_S[1];
-  a.knn = e->d_knn; a.same = e->d_same; a.kth = e->d_kth; a.act = e->d_act; a.act_count = e->d_act_count;
+  a.S[0] = (Pt4<T>*)e->d_S[0]; a.S[1] = (Pt4<T>*)e->d_S[1];
+  a.internal_of = e->d_internal_of; a.stride = (size_t)e->max_sites; a.list = e->d_list;
+  a.same = e->d_same; a.kth = e->d_kth; a.act = e->d_act; a.act_count = e->d_act_count;
   a.knnv = e->d_knnv; a.nnv = e->d_nnv;
   a.frozen = e->d_frozen; a.streak = e->d_streak; a.tier = e->d_tier;
-  a.cell_start = e->d_cell_start; a.sorted = (const Pt4<T>*)e->d_sorted; a.total_cells = e->max_cells;
+  a.cell_start = e->d_cell_start; a.sorted = (const Pt4<T>*)e->d_sorted;
   a.stats = e->d_stats; a.ovf = e->d_ovf; a.far = e->d_far; a.cent = (T*)e->d_cent; a.K = e->K;
+  a.n_sites = e->max_sites;
   a.proj_mode = e->p.proj_mode; a.bvh_ovf = reinterpret_cast<int*>(e->d_tickets + 2);
-  a.cand = e->d_cand; a.cand_rho = e->d_cand_rho; a.cand_D = e->d_cand_D; a.srch = e->d_srch; a.srch_thr = e->d_srch_thr; a.srch_n = e->d_srch_n; a.srch_cap = e->srch_cap; a.blockmax = e->d_blockmax;
+  a.cand_rho = e->d_cand_rho; a.cand_D = e->d_cand_D; a.srch = e->d_srch; a.srch_thr = e->d_srch_thr;
+  a.blockmax = e->d_blockmax;
   return a;
 }
 
-// the site KNN: with candidate lists, the check (one warp per active site)
-// and then the full searches of the sites it left (a grid-stride kernel);
-// without, the full searches of every active site.  Returns the launches.
-template <class T, int KK, int MM, int BS>
-static int launch_site_knn_b(const EngineArgs<T>& a, int parity, int nsites, int nsm, cudaStream_t st) {
-  (void)nsites;
-  const int vgrid = nsm * (kKnnVerifyWarpsPerSM * 32 / BS);  // the shape a.srch_cap is sized for
-  int L = 0;
-  if constexpr (MM > 0) {
-    k_knn_verify<T, KK, MM, BS><<<vgrid, BS, 0, st>>>(a, parity);
-    L++;
-  }
-  k_knn_search<T, KK, MM, BS><<<nsm * (kKnnSearchWarpsPerSM * 32 / BS), BS, 0, st>>>(a, parity,
-                                                                                    nsm * kKnnVerifyWarpsPerSM);
-  return L + 1;
+// the list check (with candidate lists): the sites it proves need no search
+template <class T, int KK> static void launch_verify(const EngineArgs<T>& a, int parity, int ns, cudaStream_t st) {
+  k_knn_verify<T, KK, cand_len(KK)><<<cdiv(ns, kVerifyThreads), kVerifyThreads, 0, st>>>(a, parity);
 }
 
+// the full searches: of the sites the check left, or of every active site
 template <class T, int KK, int MM>
-static int launch_site_knn_m(const EngineArgs<T>& a, int parity, int nsites, int bs, int nsm, cudaStream_t st) {
-  if (bs == 64) return launch_site_knn_b<T, KK, MM, 64>(a, parity, nsites, nsm, st);
-  if (bs == 256) return launch_site_knn_b<T, KK, MM, 256>(a, parity, nsites, nsm, st);
-  return launch_site_knn_b<T, KK, MM, 128>(a, parity, nsites, nsm, st);
+static void launch_search_m(const EngineArgs<T>& a, int parity, int bs, int nsm, cudaStream_t st) {
+  const int warps = nsm * kKnnSearchWarpsPerSM;
+  if (bs == 64) k_knn_search<T, KK, MM, 64><<<warps * 32 / 64, 64, 0, st>>>(a, parity);
+  else if (bs == 256) k_knn_search<T, KK, MM, 256><<<warps * 32 / 256, 256, 0, st>>>(a, parity);
+  else k_knn_search<T, KK, MM, 128><<<warps * 32 / 128, 128, 0, st>>>(a, parity);
+}
+template <class T, int KK>
+static void launch_search(const EngineArgs<T>& a, int parity, int bs, bool reuse, int nsm, cudaStream_t st) {
+  if (reuse) launch_search_m<T, KK, cand_len(KK)>(a, parity, bs, nsm, st);
+  else launch_search_m<T, KK, 0>(a, parity, bs, nsm, st);
 }
 
-template <class T, int KK>
-static int launch_site_knn(const EngineArgs<T>& a, int parity, int nsites, int bs, bool reuse, int nsm,
-                           cudaStream_t st) {
-  if (reuse) return launch_site_knn_m<T, KK, cand_len(KK)>(a, parity, nsites, bs, nsm, st);
-  return launch_site_knn_m<T, KK, 0>(a, parity, nsites, bs, nsm, st);
-}
+// FN<T, k>(args...) for the engine's k
+#define K_DISPATCH(k, FN, T, ...)              \
+  do {                                         \
+    switch (k) {                               \
+      case 8: FN<T, 8>(__VA_ARGS__); break;    \
+      case 12: FN<T, 12>(__VA_ARGS__); break;  \
+      case 16: FN<T, 16>(__VA_ARGS__); break;  \
+      case 20: FN<T, 20>(__VA_ARGS__); break;  \
+      case 24: FN<T, 24>(__VA_ARGS__); break;  \
+      default: FN<T, 32>(__VA_ARGS__); break;  \
+    }                                          \
+  } while (0)
 
 template <int PROF, int FRAME>
 static void launch_site_clip_f(const EngineArgs<typename PT<PROF>::T>& a, int parity, int ns, int bs, int nsm,
@@ -1498,52 +1581,51 @@ static void launch_site_proj(const EngineArgs<typename PT<PROF>::T>& a, int pari
 // the second branch of an iteration: its stream and the fork / join events
 struct Branch {
   cudaStream_t side;
-  cudaEvent_t fork, join;
+  cudaEvent_t fork, grid, join;
 };
 
 // ev (optional, 6 events): recorded before the grid build, after it, after
-// the KNN kernel, after the clip kernels, after the projection kernels and
-// after the bookkeeping kernel
+// the KNN kernels, after the clip kernels, after the projection kernels and
+// after the bookkeeping kernel.  With events the grid is built on the main
+// stream, so that its time is its own.
 template <int PROF>
 static cvt_status_t enqueue_iteration_t(cvt_engine* e, int parity, cudaStream_t st, const Branch& br, int* nlaunch,
                                         cudaEvent_t* ev) {
   using T = typename PT<PROF>::T;
-  using PP = typename PT<PROF>::PP;
   EngineArgs<T> a = engine_args<T>(e);
-  const int ns = e->max_sites;
+  const int ns = a.n_sites;
   int L = 0;
   if (ev) CK(cudaEventRecord(ev[0], st));
-  // d_cell_count is all zero here: set at creation, cleared by the scan
-  k_grid_count<T><<<cdiv(ns, 256), 256, 0, st>>>(ns, (const T*)e->d_S[parity], SegGrid{e->d_geom, e->d_site_seg, e->d_active},
-                                                 e->d_cell_count, e->d_cellrank);
+  // d_cell_count is all zero here (set at creation, cleared by the scan), as
+  // are the active and search counts (reset by the bookkeeping)
+  k_site_count<T><<<cdiv(ns, kCountThreads), kCountThreads, 0, st>>>(a, parity, e->d_cell_count, e->d_cellrank);
   L++;
-  L += launch_exclusive_scan(e->max_cells, e->d_cell_count, e->d_part, e->d_cell_start, st, true, e->d_tickets);
-  k_grid_scatter<T><<<cdiv(ns, 256), 256, 0, st>>>(ns, (const T*)e->d_S[parity], e->d_cellrank, e->d_cell_start,
-                                                   (Pt4<T>*)e->d_sorted);
+  // The grid is first read by the full searches and the frame vertices by the
+  // clip: both run on the side stream while the check and the searches run.
+  cudaStream_t gs = ev ? st : br.side;
+  if (!ev) {
+    CK(cudaEventRecord(br.fork, st));
+    CK(cudaStreamWaitEvent(br.side, br.fork, 0));
+  }
+  L += launch_exclusive_scan(e->max_cells, e->d_cell_count, e->d_part, e->d_cell_start, gs, true, e->d_tickets);
+  k_site_scatter<T><<<cdiv(ns, 256), 256, 0, gs>>>(a, parity, e->d_cellrank, (Pt4<T>*)e->d_sorted);
   L++;
-  // cell_start[max_cells] is the number of gridded sites (read on the device)
-  a.total_cells = e->max_cells;
-  // d_act_count is zero here: set at creation, reset by the bookkeeping
-  k_active_list<T><<<cdiv(ns, kActiveListThreads), kActiveListThreads, 0, st>>>(a);
-  L++;
-  // the frame vertices are first read by the clip: search them on the side
-  // stream while the site KNN runs
-  CK(cudaEventRecord(br.fork, st));
-  CK(cudaStreamWaitEvent(br.side, br.fork, 0));
-  k_frame_vertex<T><<<cdiv(ns, 128), 128, 0, br.side>>>(a);
+  CK(cudaEventRecord(br.grid, gs));
+  if (ev) {
+    CK(cudaEventRecord(ev[1], st));
+    CK(cudaStreamWaitEvent(br.side, br.grid, 0));
+  }
+  k_frame_vertex<T><<<cdiv(ns, 128), 128, 0, br.side>>>(a, parity);
   CK(cudaEventRecord(br.join, br.side));
   L++;
-  if (ev) CK(cudaEventRecord(ev[1], st));
   const bool reuse = e->p.knn_reuse != 0;
-  const int nsm = e->num_sms;
-  switch (e->K) {
-    case 8: L += launch_site_knn<T, 8>(a, parity, ns, e->p.knn_block, reuse, nsm, st); break;
-    case 12: L += launch_site_knn<T, 12>(a, parity, ns, e->p.knn_block, reuse, nsm, st); break;
-    case 16: L += launch_site_knn<T, 16>(a, parity, ns, e->p.knn_block, reuse, nsm, st); break;
-    case 20: L += launch_site_knn<T, 20>(a, parity, ns, e->p.knn_block, reuse, nsm, st); break;
-    case 24: L += launch_site_knn<T, 24>(a, parity, ns, e->p.knn_block, reuse, nsm, st); break;
-    default: L += launch_site_knn<T, 32>(a, parity, ns, e->p.knn_block, reuse, nsm, st); break;
+  if (reuse) {
+    K_DISPATCH(e->K, launch_verify, T, a, parity, ns, st);
+    L++;
   }
+  CK(cudaStreamWaitEvent(st, br.grid, 0));
+  K_DISPATCH(e->K, launch_search, T, a, parity, e->p.knn_block, reuse, e->num_sms, st);
+  L++;
   if (ev) CK(cudaEventRecord(ev[2], st));
   CK(cudaStreamWaitEvent(st, br.join, 0));
   launch_site_clip<PROF>(a, parity, ns, e->p.clip_block, e->p.frame_mode, e->num_sms, st);
@@ -1585,7 +1667,7 @@ extern "C" cvt_status_t cvt_engine_run(cvt_engine_t e, int iters, void* stream) 
   long long launches = 0;
   ThreadStreams* ts = nullptr;
   if (iters > 0) CK(thread_streams(&ts));
-  const Branch eager{ts ? ts->side : nullptr, e->ev_fork, e->ev_join};
+  const Branch eager{ts ? ts->side : nullptr, e->ev_fork, e->ev_grid, e->ev_join};
   e->last_launches = 0;
   for (int it = 0; it < iters; ++it) {
     const int par = e->parity;
@@ -1609,7 +1691,7 @@ extern "C" cvt_status_t cvt_engine_run(cvt_engine_t e, int iters, void* stream) 
     if (capture) {
       int ng = 0;
       CK(cudaStreamBeginCapture(ts->cap, cudaStreamCaptureModeThreadLocal));
-      cvt_status_t q = enqueue_iteration(e, par, ts->cap, Branch{ts->cap_side, e->ev_cfork, e->ev_cjoin}, &ng);
+      cvt_status_t q = enqueue_iteration(e, par, ts->cap, Branch{ts->cap_side, e->ev_cfork, e->ev_cgrid, e->ev_cjoin}, &ng);
       cudaGraph_t gr = nullptr;
       cudaError_t ce = cudaStreamEndCapture(ts->cap, &gr);
       if (q != CVT_OK) { if (gr) cudaGraphDestroy(gr); return q; }
@@ -1634,7 +1716,7 @@ extern "C" cvt_status_t cvt_engine_profile(cvt_engine_t e, int iters, float* ms,
   double acc[5] = {0, 0, 0, 0, 0};
   for (int it = 0; it < iters; ++it) {
     int nl = 0;
-    s = enqueue_iteration(e, e->parity, st, Branch{ts->side, e->ev_fork, e->ev_join}, &nl, ev);
+    s = enqueue_iteration(e, e->parity, st, Branch{ts->side, e->ev_fork, e->ev_grid, e->ev_join}, &nl, ev);
     if (s != CVT_OK) break;
     LAUNCHED(nl);
     e->parity ^= 1;
@@ -1673,18 +1755,15 @@ extern "C" cvt_status_t cvt_engine_get_sites(cvt_engine_t e, int s, float* out, 
   int par = 0;
   cvt_status_t ps = seg_sites_buffer(e, s, st, &par);
   if (ps != CVT_OK) return ps;
-  if (!e->f64) {
-    const float* src = (const float*)e->d_S[par] + 3 * (size_t)sd.site_base;
-    CK(cudaMemcpyAsync(out, src, sizeof(float) * cnt, out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
-  } else {
-    const double* src = (const double*)e->d_S[par] + 3 * (size_t)sd.site_base;
-    Scratch sc(st);
-    float* tmp = out;
-    if (!out_on_device) CK(sc.get(&tmp, cnt));
-    k_f64_to_f32<<<cdiv((long)cnt, 256), 256, 0, st>>>(src, tmp, (long)cnt);
-    CKLAUNCH();
-    if (!out_on_device) CK(cudaMemcpyAsync(out, tmp, sizeof(float) * cnt, cudaMemcpyDeviceToHost, st));
-  }
+  Scratch sc(st);
+  float* tmp = out;
+  if (!out_on_device) CK(sc.get(&tmp, cnt));
+  if (e->f64)
+    k_export_sites<<<cdiv(sd.n_sites, 256), 256, 0, st>>>(engine_args<double>(e), sd.site_base, sd.n_sites, tmp);
+  else
+    k_export_sites<<<cdiv(sd.n_sites, 256), 256, 0, st>>>(engine_args<float>(e), sd.site_base, sd.n_sites, tmp);
+  CKLAUNCH();
+  if (!out_on_device) CK(cudaMemcpyAsync(out, tmp, sizeof(float) * cnt, cudaMemcpyDeviceToHost, st));
   if (!out_on_device) CK(cudaStreamSynchronize(st));
   return CVT_OK;
 }
@@ -1697,8 +1776,12 @@ extern "C" cvt_status_t cvt_engine_get_sites_f64(cvt_engine_t e, int s, double* 
   int par = 0;
   cvt_status_t ps = seg_sites_buffer(e, s, st, &par);
   if (ps != CVT_OK) return ps;
-  const double* src = (const double*)e->d_S[par] + 3 * (size_t)sd.site_base;
-  CK(cudaMemcpyAsync(out, src, sizeof(double) * 3 * (size_t)sd.n_sites, cudaMemcpyDeviceToHost, st));
+  Scratch sc(st);
+  double* tmp;
+  CK(sc.get(&tmp, 3 * (size_t)sd.n_sites));
+  k_export_sites<<<cdiv(sd.n_sites, 256), 256, 0, st>>>(engine_args<double>(e), sd.site_base, sd.n_sites, tmp);
+  CKLAUNCH();
+  CK(cudaMemcpyAsync(out, tmp, sizeof(double) * 3 * (size_t)sd.n_sites, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   return CVT_OK;
 }
@@ -1708,13 +1791,22 @@ extern "C" cvt_status_t cvt_engine_get_state(cvt_engine_t e, int s, uint32_t* kn
   if (!e || s < 0 || s >= e->max_seg || !e->seg_mesh[s]) return fail(CVT_ERR_INVALID, "cvt_engine_get_state: bad segment");
   cudaStream_t st = S_(stream);
   const SegDev& sd = e->segs[s];
-  const size_t n = sd.n_sites, b = sd.site_base;
-  // the list of the last completed iteration sits in the buffer it wrote
-  const uint32_t* kl = e->d_knn;
-  if (knn) CK(cudaMemcpyAsync(knn, kl + (size_t)e->K * b, sizeof(uint32_t) * e->K * n, cudaMemcpyDeviceToHost, st));
-  if (knnv) CK(cudaMemcpyAsync(knnv, e->d_knnv + 5 * b, sizeof(int) * 5 * n, cudaMemcpyDeviceToHost, st));
-  if (frozen) CK(cudaMemcpyAsync(frozen, e->d_frozen + b, n, cudaMemcpyDeviceToHost, st));
-  if (tier) CK(cudaMemcpyAsync(tier, e->d_tier + b, n, cudaMemcpyDeviceToHost, st));
+  const size_t n = sd.n_sites;
+  Scratch sc(st);
+  uint32_t* tk = nullptr;
+  int* tv = nullptr;
+  uint8_t *tf = nullptr, *tt = nullptr;
+  if (knn) CK(sc.get(&tk, (size_t)e->K * n));
+  if (knnv) CK(sc.get(&tv, kKProj * n));
+  if (frozen) CK(sc.get(&tf, n));
+  if (tier) CK(sc.get(&tt, n));
+  if (e->f64) k_export_state<<<cdiv((long)n, 128), 128, 0, st>>>(engine_args<double>(e), s, tk, tv, tf, tt);
+  else k_export_state<<<cdiv((long)n, 128), 128, 0, st>>>(engine_args<float>(e), s, tk, tv, tf, tt);
+  CKLAUNCH();
+  if (knn) CK(cudaMemcpyAsync(knn, tk, sizeof(uint32_t) * e->K * n, cudaMemcpyDeviceToHost, st));
+  if (knnv) CK(cudaMemcpyAsync(knnv, tv, sizeof(int) * kKProj * n, cudaMemcpyDeviceToHost, st));
+  if (frozen) CK(cudaMemcpyAsync(frozen, tf, n, cudaMemcpyDeviceToHost, st));
+  if (tier) CK(cudaMemcpyAsync(tier, tt, n, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   return CVT_OK;
 }
@@ -1844,32 +1936,31 @@ extern "C" cvt_status_t cvt_remesh(const float* V, int nV, const int* F, int nF,
 // Host threads that ingest the meshes of one cvt_remesh_batch call.
 constexpr int kIngestThreads = 8;
 
-// Every segment's sites into its host array with one read of the segment
-// table and one wait at the end (cvt_engine_get_sites waits twice per
-// segment).
+// The sites of every reserved segment (slot order) from its host array.
+static cvt_status_t upload_and_place(cvt_engine* e, const int* seg, int n, const float* const* sites, const int* n_sites) {
+  cudaStream_t st = S_(nullptr);
+  Scratch sc(st);
+  float* raw;
+  CK(sc.get(&raw, 3 * (size_t)e->max_sites));
+  for (int i = 0; i < n; ++i)
+    CK(cudaMemcpyAsync(raw + 3 * (size_t)e->segs[seg[i]].site_base, sites[i], sizeof(float) * 3 * (size_t)n_sites[i],
+                       cudaMemcpyHostToDevice, st));
+  return place_all_segments(e, raw, e->max_sites, st);
+}
+
+// Every segment's sites into its host array: one kernel for all and one wait
+// at the end (cvt_engine_get_sites waits twice per segment).
 static cvt_status_t engine_get_sites_all(cvt_engine* e, const int* seg, int n, float* const* out) {
   cudaStream_t st = S_(nullptr);
-  std::vector<SegDev> hs(e->max_seg);
-  CK(cudaMemcpyAsync(hs.data(), e->d_segs, sizeof(SegDev) * e->max_seg, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  Scratch sc(st);
+  float* tmp;
+  CK(sc.get(&tmp, 3 * (size_t)e->max_sites));
+  if (e->f64) k_export_sites<<<cdiv(e->max_sites, 256), 256, 0, st>>>(engine_args<double>(e), 0, e->max_sites, tmp);
+  else k_export_sites<<<cdiv(e->max_sites, 256), 256, 0, st>>>(engine_args<float>(e), 0, e->max_sites, tmp);
+  CKLAUNCH();
   for (int i = 0; i < n; ++i) {
-    const int s = seg[i];
-    const SegDev& sd = e->segs[s];
-    e->host_iters[s] = hs[s].iter;
-    const int par = (e->seg_p0[s] + hs[s].iter) & 1;
-    const size_t cnt = 3 * (size_t)sd.n_sites;
-    if (!e->f64) {
-      const float* src = (const float*)e->d_S[par] + 3 * (size_t)sd.site_base;
-      CK(cudaMemcpyAsync(out[i], src, sizeof(float) * cnt, cudaMemcpyDeviceToHost, st));
-    } else {
-      const double* src = (const double*)e->d_S[par] + 3 * (size_t)sd.site_base;
-      Scratch sc(st);  // freed in stream order, after the copy
-      float* tmp;
-      CK(sc.get(&tmp, cnt));
-      k_f64_to_f32<<<cdiv((long)cnt, 256), 256, 0, st>>>(src, tmp, (long)cnt);
-      CKLAUNCH();
-      CK(cudaMemcpyAsync(out[i], tmp, sizeof(float) * cnt, cudaMemcpyDeviceToHost, st));
-    }
+    const SegDev& sd = e->segs[seg[i]];
+    CK(cudaMemcpyAsync(out[i], tmp + 3 * (size_t)sd.site_base, sizeof(float) * 3 * (size_t)sd.n_sites, cudaMemcpyDeviceToHost, st));
   }
   CK(cudaStreamSynchronize(st));
   return CVT_OK;
@@ -1927,13 +2018,10 @@ extern "C" cvt_status_t cvt_remesh_batch(int n_meshes, const float* const* V, co
   cvt_engine_t e = nullptr;
   if (s == CVT_OK) s = cvt_engine_create(p, n_meshes, (int)total_sites, (int)total_cells, &e);
   std::vector<int> seg(n_meshes, -1);
-  // segments added with their tables uploaded once for all
+  // every segment reserved, then all sites uploaded and placed at once
   for (int i = 0; i < n_meshes && s == CVT_OK; ++i)
-    s = add_segment_impl(e, meshes[i], sites_in[i], n_sites[i], 0, &seg[i], S_(nullptr), true);
-  if (e) {
-    const cvt_status_t u = upload_segment_tables(e, S_(nullptr));
-    if (s == CVT_OK) s = u;
-  }
+    s = add_segment_impl(e, meshes[i], nullptr, n_sites[i], 0, &seg[i], S_(nullptr), true);
+  if (s == CVT_OK) s = upload_and_place(e, seg.data(), n_meshes, sites_in, n_sites);
   if (s == CVT_OK) s = cvt_engine_run(e, iters, nullptr);
   if (s == CVT_OK) s = engine_get_sites_all(e, seg.data(), n_meshes, sites_out);
   if (e) cvt_engine_destroy(e);
@@ -1945,13 +2033,13 @@ extern "C" cvt_status_t cvt_remesh_batch(int n_meshes, const float* const* V, co
 // ---------------------------------------------------------------------------
 // evaluation: dual triangles, quality, Hausdorff (evaluate stage)
 // ---------------------------------------------------------------------------
-extern "C" cvt_status_t cvt_extract_faces(const float* S, const float* U, const float* V, const uint32_t* knn, int n, int K,
-                                          float R2, int* F_out, int max_faces, int* n_faces, void* stream) {
-  if (n < 0 || K < 1 || !n_faces || (n > 0 && (!S || !U || !V || !knn)) || (max_faces > 0 && !F_out))
-    return fail(CVT_ERR_INVALID, "cvt_extract_faces: bad arguments");
+// Dual triangles of n sites S with frames U, V and neighbours nb; the keys
+// hold nb.label() of the sites, and S_label are the positions by label.
+template <class NB>
+static cvt_status_t extract_faces(const float* S, const float* U, const float* V, const NB& nb, const float* S_label, int n,
+                                  int K, float R2, int* F_out, int max_faces, int* n_faces, cudaStream_t st) {
   *n_faces = 0;
   if (n == 0) return CVT_OK;
-  cudaStream_t st = S_(stream);
   Scratch sc(st);
   int* cnt;
   CK(sc.get(&cnt, 1));
@@ -1962,7 +2050,7 @@ extern "C" cvt_status_t cvt_extract_faces(const float* S, const float* U, const 
     Scratch ks(st);
     CK(ks.get(&keys, (size_t)cap));
     CK(cudaMemsetAsync(cnt, 0, sizeof(int), st));
-    k_face_keys<<<cdiv(n, 64), 64, 0, st>>>(S, U, V, knn, n, K, R2, 1e-8f, 1e-7f, keys, cnt, cap);
+    k_face_keys<<<cdiv(n, 64), 64, 0, st>>>(S, U, V, nb, n, K, R2, 1e-8f, 1e-7f, keys, cnt, cap);
     CKLAUNCH();
     CK(cudaMemcpyAsync(&nk, cnt, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -1992,7 +2080,7 @@ extern "C" cvt_status_t cvt_extract_faces(const float* S, const float* U, const 
       CK(sc.get(&keep, (size_t)nu));
       CK(sc.get(&pos, (size_t)nu + 1));
       CK(sc.get(&part, (size_t)scan_blocks(nu) + 2));
-      k_face_decode<<<cdiv(nu, 256), 256, 0, st>>>(uniq, nu, S, n, 1e-6f, tri, keep);
+      k_face_decode<<<cdiv(nu, 256), 256, 0, st>>>(uniq, nu, S_label, n, 1e-6f, tri, keep);
       CKLAUNCH();
       launch_exclusive_scan(nu, keep, part, pos, st);
       LAUNCHED(3);
@@ -2008,6 +2096,13 @@ extern "C" cvt_status_t cvt_extract_faces(const float* S, const float* U, const 
     cap = nk;  // retry with the exact key count
   }
   return fail(CVT_ERR_CUDA, "cvt_extract_faces: key count changed between passes");
+}
+
+extern "C" cvt_status_t cvt_extract_faces(const float* S, const float* U, const float* V, const uint32_t* knn, int n, int K,
+                                          float R2, int* F_out, int max_faces, int* n_faces, void* stream) {
+  if (n < 0 || K < 1 || !n_faces || (n > 0 && (!S || !U || !V || !knn)) || (max_faces > 0 && !F_out))
+    return fail(CVT_ERR_INVALID, "cvt_extract_faces: bad arguments");
+  return extract_faces(S, U, V, FaceRows{knn, K}, S, n, K, R2, F_out, max_faces, n_faces, S_(stream));
 }
 
 extern "C" cvt_status_t cvt_quality(const float* V, const int* F, int nF, float* out, void* stream) {
@@ -2043,18 +2138,22 @@ extern "C" cvt_status_t cvt_quality(const float* V, const int* F, int nF, float*
 
 // frames of the current sites (frozen sites keep their vertex list; the rest
 // take their nearest mesh vertex): main.cu:883-897
+// (Sf, U, Vv, label in internal order; Sc in the caller's)
 template <class T>
-__global__ void k_eval_frames(const T* __restrict__ S, int base, int n, const uint8_t* __restrict__ frozen,
-                              const int* __restrict__ knnv, int mode, MeshDev md, float* __restrict__ Sf,
-                              float* __restrict__ U, float* __restrict__ Vv) {
+__global__ void k_eval_frames(EngineArgs<T> a, int parity, int base, int n, int mode, MeshDev md, float* __restrict__ Sf,
+                              float* __restrict__ Sc, int* __restrict__ label, float* __restrict__ U, float* __restrict__ Vv) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int g = base + i;
-  V3<T> p = ld3(S, g);
+  const Pt4<T> me = a.S[parity][g];
+  const V3<T> p{me.x, me.y, me.z};
+  const int caller = (int)me.id - base;
   st3(Sf, i, cvt3<float>(p));
+  st3(Sc, caller, cvt3<float>(p));
+  label[i] = caller;
   int nn;
-  if (mode != 0 && frozen[g]) {
-    nn = knnv[(size_t)g * kKProj];
+  if (mode != 0 && a.frozen[g]) {
+    nn = a.knnv[g];
   } else {
     TopK<T, 1> v1;
     grid_knn<T, float, 1>(md.vg, md.vcell_start, md.vsorted, p, v1, [](uint32_t) { return true; });
@@ -2091,16 +2190,17 @@ static cvt_status_t engine_eval_impl(cvt_engine_t e, int s, cvt_eval_t* out, int
   cvt_status_t ps = seg_sites_buffer(e, s, st, &par);
   if (ps != CVT_OK) return ps;
   Scratch sc(st);
-  float *Sf, *U, *V;
+  float *Sf, *Sc, *U, *V;
+  int* label;
   CK(sc.get(&Sf, 3 * (size_t)n));
+  CK(sc.get(&Sc, 3 * (size_t)n));
+  CK(sc.get(&label, (size_t)n));
   CK(sc.get(&U, 3 * (size_t)n));
   CK(sc.get(&V, 3 * (size_t)n));
   if (e->f64)
-    k_eval_frames<double><<<cdiv(n, 128), 128, 0, st>>>((const double*)e->d_S[par], sd.site_base, n, e->d_frozen,
-                                                         e->d_knnv, sd.mode, m->dev(), Sf, U, V);
+    k_eval_frames<<<cdiv(n, 128), 128, 0, st>>>(engine_args<double>(e), par, sd.site_base, n, sd.mode, m->dev(), Sf, Sc, label, U, V);
   else
-    k_eval_frames<float><<<cdiv(n, 128), 128, 0, st>>>((const float*)e->d_S[par], sd.site_base, n, e->d_frozen,
-                                                        e->d_knnv, sd.mode, m->dev(), Sf, U, V);
+    k_eval_frames<<<cdiv(n, 128), 128, 0, st>>>(engine_args<float>(e), par, sd.site_base, n, sd.mode, m->dev(), Sf, Sc, label, U, V);
   CKLAUNCH();
   // R2 = longest bbox edge of the current sites (main.cu:899-909)
   int* bb;
@@ -2120,23 +2220,23 @@ static cvt_status_t engine_eval_impl(cvt_engine_t e, int s, cvt_eval_t* out, int
     std::memcpy(&hi[a], &q, 4);
   }
   float R2 = 2.0f * 0.5f * std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
-  const uint32_t* knn = e->d_knn + (size_t)e->K * sd.site_base;
+  const FaceColumns nb{e->d_list + sd.site_base, label, (size_t)e->max_sites, (uint32_t)sd.site_base};
   int max_faces = 4 * n + 64;
   int* Fc;
   CK(sc.get(&Fc, 3 * (size_t)max_faces));
   int nf = 0;
-  cvt_status_t r = cvt_extract_faces(Sf, U, V, knn, n, e->K, R2, Fc, max_faces, &nf, stream);
+  cvt_status_t r = extract_faces(Sf, U, V, nb, Sc, n, e->K, R2, Fc, max_faces, &nf, st);
   if (r == CVT_ERR_CAPACITY) {
     max_faces = nf;
     CK(sc.get(&Fc, 3 * (size_t)max_faces));
-    r = cvt_extract_faces(Sf, U, V, knn, n, e->K, R2, Fc, max_faces, &nf, stream);
+    r = extract_faces(Sf, U, V, nb, Sc, n, e->K, R2, Fc, max_faces, &nf, st);
   }
   if (r != CVT_OK) return r;
   float q[6];
-  r = cvt_quality(Sf, Fc, nf, q, stream);
+  r = cvt_quality(Sc, Fc, nf, q, stream);
   if (r != CVT_OK) return r;
   float dH = 0.f;
-  r = cvt_hausdorff_to_mesh(const_cast<cvt_mesh*>(m), Sf, n, Fc, nf, &dH, stream);
+  r = cvt_hausdorff_to_mesh(const_cast<cvt_mesh*>(m), Sc, n, Fc, nf, &dH, stream);
   if (r != CVT_OK) return r;
   if (n_faces_host) {
     *n_faces_host = nf;

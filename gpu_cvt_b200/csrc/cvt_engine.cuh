@@ -1,12 +1,13 @@
 // Fused Lloyd-iteration kernels over many (mesh, site set) segments.
 //
 // One iteration (main.cu:669-881 per segment) is:
-//   grid build over the sites of active segments (count -> scan -> scatter)
-//   k_active_list  the non-frozen sites
+//   k_site_count the cells of the sites of active segments, and the list of
+//                the non-frozen ones
+//   grid build   scan -> scatter, on a second stream beside k_knn_verify
 //   k_frame_vertex the mesh vertex nearest to each of them (its normal
-//                gives the frame, main.cu:685-700), on a second stream
+//                gives the frame, main.cu:685-700), on the second stream
 //                while the site KNN runs
-//   k_knn_verify per active site (one warp): the K-list from the site's
+//   k_knn_verify per active site (one thread): the K-list from the site's
 //                candidate list where its motion bound proves it exact
 //   k_knn_search the other active sites (one warp each): exact (K+1)-NN in
 //                the segment, drop self (site_knn.cuh:79), by one radius
@@ -32,6 +33,21 @@
 //                the last block of k_site_far
 // All sizes come from device memory, so the whole iteration is captured once
 // in a CUDA graph and relaunched while segments come and go.
+//
+// Site order.  A segment's sites are stored in the cell order of its grid at
+// the time it was placed ("internal" order; a Lloyd run moves sites by less
+// than a few cells, so neighbours in space stay neighbours in memory), with
+// the caller's index kept beside the position (Pt4::id) and the way back in
+// internal_of.  Every per-site kernel then reads and writes consecutive
+// sites, and a neighbour gather is one aligned 16-byte load (32 bytes in
+// FP64) from lines that its block has just read.  Ties are always broken by
+// the caller's indices, so no result depends on the internal order.  The
+// per-site lists are stored entry by entry (entry e of site g at
+// [e * stride + g]): one thread per site reads them coalesced.  With 12-byte
+// positions and row-major lists in the caller's order the gathers went to L2:
+// the 25-iteration run of 1M sites (K = 32, mixed) took 53.6 ms, with this
+// layout and the list check below 40.2; 100k sites, 100 iterations 23.7 and
+// 16.1 ms.
 #pragma once
 #include "cvt_grid.cuh"
 
@@ -80,6 +96,7 @@ struct SegDev {
   float thr2_tier[6];
   int need_tier[6];
   float step_motion;   // largest site motion of the segment's last iteration
+  int p0;              // buffer parity when the segment was placed
 };
 
 template <int PROF> struct PT;
@@ -93,36 +110,46 @@ template <class T> struct EngineArgs {
   const int* active;      // 0 free, 1 iterating, 2 stopped by its stop rule
   const MeshDev* meshes;
   const int* site_seg;
-  T* S[2];
-  uint32_t* knn;      // K neighbours per site (local indices), the current list
-  uint8_t* same;      // list unchanged vs the previous iteration (site KNN kernel)
+  Pt4<T>* S[2];               // positions in internal order, id = the site's caller index (+ site_base)
+  const uint32_t* internal_of;  // the way back: internal index of caller index (+ site_base)
+  size_t stride;              // sites the engine holds: entry e of site g's list at [e * stride + g]
+  // Neighbour list per site (internal indices, 0xffffffff: none): the K
+  // nearest in order, and with candidate lists (MM > 0) MM - K further ones
+  // in no order; the K-list is the candidate list's head.
+  uint32_t* list;
+  uint8_t* same;      // list unchanged vs the previous iteration (site KNN kernels)
   float* kth;         // last K-th neighbour's squared distance per site, < 0 unknown
-  int* act;           // sorted positions of the sites whose list is recomputed
+  int* act;           // the sites whose list is recomputed
   int* act_count;
-  int* knnv;
+  int* knnv;          // 5 nearest vertices, entry k of site g at [k * stride + g]
   int* nnv;
   uint8_t* frozen;
   uint8_t* streak;
   uint8_t* tier;
   const int* cell_start;
-  const Pt4<T>* sorted;
-  int total_cells;
+  const Pt4<T>* sorted;  // cell-ordered copy of the positions, id = caller index (+ site_base)
   int* stats;
   int* ovf;  // [0] = count, [1 + k] = overflowed site
   int* far;  // [0] = count, [1 + k] = site whose vertex search was deferred
   T* cent;   // centroid per site (3 values), k_site_clip -> k_site_proj
   int K;
+  int n_sites;    // site slots the launches cover (every placed segment lies below)
   int proj_mode;  // 0: one-ring of the KPROJ nearest vertices; 1: closest point through the BVH
   int* bvh_ovf;   // BVH traversal stack overflows (never expected: the tree depth is bounded)
-  uint32_t* cand;    // candidate list per site (global ids), MM entries (k_knn_verify / k_knn_search)
-  float* cand_rho;   // its MM-th distance when it was built, rounded down (< 0: no list; inf: every other site)
+  float* cand_rho;   // candidate list's MM-th distance when it was built, rounded down (< 0: no list; inf: every other site)
   float* cand_D;     // motion bound accumulated since it was built (k_knn_verify)
-  int* srch;         // per verify warp: srch_cap slots of sorted positions left for a full search
-  float* srch_thr;   // per slot: squared distance that the site's MM nearest lie within (< 0: unknown)
-  int* srch_n;       // per verify warp: slots used
-  int srch_cap;
+  int* srch;         // [0] = count, [1 + k] = site left for a full search
+  float* srch_thr;   // [k]: squared distance that the site's MM nearest lie within (< 0: unknown)
   unsigned long long* blockmax;  // per coarse block (cell slots of the segment): iteration << 32 | max motion bits
 };
+
+// Segment of site g when its segment is iterating, else -1.
+template <class T>
+__device__ __forceinline__ int active_seg(const EngineArgs<T>& a, int g) {
+  if (g >= a.n_sites) return -1;
+  const int s = __ldg(a.site_seg + g);
+  return s >= 0 && a.active[s] == 1 ? s : -1;
+}
 
 __device__ __forceinline__ float f32_ru(float x) { return x; }
 __device__ __forceinline__ float f32_ru(double x) { return __double2float_ru(x); }
@@ -210,6 +237,25 @@ __device__ __forceinline__ bool halfplane_contains_disk(Q a, Q b, Q c, Q r2) {
   return c > (Q)1e-18 && fmaT(a, a, b * b) * r2 * (Q)1.0001 < c * c;
 }
 
+// Neighbours of a site for clip_cell and pca_normal: id(t) is entry t of its
+// list, valid(id) whether it names a site, pos(id) that site's position.
+template <class T> struct RowNeighbours {  // row-major list of local indices into an AoS array
+  const T* S;
+  const uint32_t* row;
+  uint32_t n;
+  __device__ __forceinline__ uint32_t id(int t) const { return __ldg(row + t); }
+  __device__ __forceinline__ bool valid(uint32_t j) const { return j < n; }
+  __device__ __forceinline__ V3<T> pos(uint32_t j) const { return ld3(S, (long)j); }
+};
+template <class T> struct ListNeighbours {  // the engine's lists
+  const Pt4<T>* S;
+  const uint32_t* col;  // list + g
+  size_t stride;
+  __device__ __forceinline__ uint32_t id(int t) const { return __ldg(col + t * stride); }
+  __device__ __forceinline__ bool valid(uint32_t j) const { return j != 0xffffffffu; }
+  __device__ __forceinline__ V3<T> pos(uint32_t j) const { return ldp(S, j); }
+};
+
 // Clip the square [-R,R]^2 by the bisectors of the listed neighbours; returns
 // the vertex count (polygon in `cur` on return) or -1 on buffer overflow.
 //
@@ -223,9 +269,8 @@ __device__ __forceinline__ bool halfplane_contains_disk(Q a, Q b, Q c, Q r2) {
 // cut the polygon and the loop ends.  Both shortcuts only leave out clips
 // that would return their input unchanged: the result is the same bit for
 // bit as clipping by all K bisectors.
-template <int PROF>
-__device__ __forceinline__ int clip_cell(const typename PT<PROF>::T* __restrict__ S, int site_base, int n_sites,
-                                         V3<typename PT<PROF>::T> si, const uint32_t* __restrict__ row, int K,
+template <int PROF, class NB>
+__device__ __forceinline__ int clip_cell(const NB& nb, V3<typename PT<PROF>::T> si, int K,
                                          const Frame<typename PT<PROF>::T>& fr, float R,
                                          PolyRef<typename PT<PROF>::PP>& cur, PolyRef<typename PT<PROF>::PP>& nxt,
                                          int cap, bool row_sorted) {
@@ -238,8 +283,8 @@ __device__ __forceinline__ int clip_cell(const typename PT<PROF>::T* __restrict_
   Q r2 = (Q)2 * (Q)r * (Q)r * (Q)1.0001;
   bool ovf = false;
   // the next neighbour's position is loaded while the current one clips
-  uint32_t jn = __ldg(row);
-  V3<T> sn = jn < (uint32_t)n_sites ? ld3(S, (long)site_base + jn) : si;
+  uint32_t jn = nb.id(0);
+  V3<T> sn = nb.valid(jn) ? nb.pos(jn) : si;
   // Every lane runs all K trips; a finished lane only skips their bodies.  A
   // data-dependent `break` lets lanes leave at different trips, and the warp
   // then runs the rest of the site's work in fragments (measured 2x slower).
@@ -249,10 +294,10 @@ __device__ __forceinline__ int clip_cell(const typename PT<PROF>::T* __restrict_
     const uint32_t j = jn;
     const V3<T> sj = sn;
     if (t + 1 < K) {
-      jn = __ldg(row + t + 1);
-      if (jn < (uint32_t)n_sites) sn = ld3(S, (long)site_base + jn);
+      jn = nb.id(t + 1);
+      if (nb.valid(jn)) sn = nb.pos(jn);
     }
-    if (j >= (uint32_t)n_sites) continue;
+    if (!nb.valid(j)) continue;
     Q a, b, c;
     if (PROF == PROF_MIXED) {
       V3<double> d{(double)sj.x - (double)si.x, (double)sj.y - (double)si.y, (double)sj.z - (double)si.z};
@@ -305,17 +350,18 @@ __device__ inline void sym3_eigenvalues_d(const double C[9], double lam[3]) {
   lam[2] = C[0] + C[4] + C[8] - lam[0] - lam[1];
 }
 
-// normal(i) gives the unit normal of local site i as float[3]
-template <class NormalOf>
-__device__ inline int tier_of(int mode, int i, int n, int K, const uint32_t* row, NormalOf normal) {
+// normal(i) gives the unit normal of site i as float[3]; row(t) the t-th
+// listed neighbour of site i, or -1
+template <class RowOf, class NormalOf>
+__device__ inline int tier_of(int mode, int i, int K, RowOf row, NormalOf normal) {
   const double TH[4] = {0.15, 0.35, 0.55, 0.80};
   float ni[3];
   normal(i, ni);
   double sum = 0.0;
   int cnt = 0;
   for (int j = 0; j < K; ++j) {
-    int jj = (int)row[j];
-    if (jj < 0 || jj >= n) continue;
+    int jj = row(j);
+    if (jj < 0) continue;
     float nj[3];
     normal(jj, nj);
     double c = (double)ni[0] * (double)nj[0] + (double)ni[1] * (double)nj[1] + (double)ni[2] * (double)nj[2];
@@ -330,8 +376,8 @@ __device__ inline int tier_of(int mode, int i, int n, int K, const uint32_t* row
     double mean[3] = {0, 0, 0};
     int c2 = 0;
     for (int j = 0; j < K; ++j) {
-      int jj = (int)row[j];
-      if (jj < 0 || jj >= n) continue;
+      int jj = row(j);
+      if (jj < 0) continue;
       float nj[3];
       normal(jj, nj);
       for (int a = 0; a < 3; ++a) mean[a] += (double)nj[a];
@@ -341,8 +387,8 @@ __device__ inline int tier_of(int mode, int i, int n, int K, const uint32_t* row
       for (int a = 0; a < 3; ++a) mean[a] = __ddiv_rn(mean[a], (double)c2);
       double C[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
       for (int j = 0; j < K; ++j) {
-        int jj = (int)row[j];
-        if (jj < 0 || jj >= n) continue;
+        int jj = row(j);
+        if (jj < 0) continue;
         float nj[3];
         normal(jj, nj);
         double d[3] = {(double)nj[0] - mean[0], (double)nj[1] - mean[1], (double)nj[2] - mean[2]};
@@ -365,33 +411,42 @@ __device__ inline int tier_of(int mode, int i, int n, int K, const uint32_t* row
 }
 
 // ---------------------------------------------------------------------------
-// k_active_list: sorted positions of the sites whose neighbour list is
-// recomputed this iteration (frozen sites keep theirs, main.cu:678).  The
-// append is aggregated per block (one atomic per block, not per warp: the
-// per-warp atomics on one counter serialised the kernel), which keeps each
-// block's active sites together and in sorted order.
+// k_site_count: the grid cell of every site of an iterating segment and its
+// rank within the cell (the counting half of the counting sort), and the list
+// of the sites whose neighbour list is recomputed this iteration (frozen
+// sites keep theirs, main.cu:678), in internal order.  Consecutive sites
+// mostly share their cell, so a warp adds to a cell once for all its sites
+// in it; the list is appended once per block (per-warp atomics on one counter
+// serialise).
 // ---------------------------------------------------------------------------
-constexpr int kActiveListThreads = 256;
+constexpr int kCountThreads = 256;
 
 template <class T>
-__global__ void __launch_bounds__(kActiveListThreads) k_active_list(EngineArgs<T> a) {
-  __shared__ int warp_base[kActiveListThreads / 32];
+__global__ void __launch_bounds__(kCountThreads) k_site_count(EngineArgs<T> a, int parity, int* __restrict__ cell_count,
+                                                              int2* __restrict__ cellrank) {
+  __shared__ int warp_base[kCountThreads / 32];
   __shared__ int block_base;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n_grid = __ldg(a.cell_start + a.total_cells);
-  bool act = false;
-  if (t < n_grid) {
-    const int g = (int)a.sorted[t].id;
-    const SegDev& sd = a.segs[__ldg(a.site_seg + g)];
-    act = !(sd.mode != 0 && a.frozen[g]);
-  }
-  const unsigned m = __ballot_sync(0xffffffffu, act);
+  const int g = blockIdx.x * kCountThreads + threadIdx.x;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int s = active_seg(a, g);
+  int cell = -1;
+  bool act = false;
+  if (s >= 0) {
+    cell = grid_cell(a.geom[s], ldp(a.S[parity], g));
+    act = !(a.segs[s].mode != 0 && a.frozen[g]);
+  }
+  const unsigned peers = __match_any_sync(0xffffffffu, cell);
+  const int leader = __ffs(peers) - 1;
+  int base = 0;
+  if (cell >= 0 && lane == leader) base = atomicAdd(cell_count + cell, __popc(peers));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (g < a.n_sites) cellrank[g] = make_int2(cell, base + __popc(peers & ((1u << lane) - 1u)));
+  const unsigned m = __ballot_sync(0xffffffffu, act);
   if (lane == 0) warp_base[wid] = __popc(m);
   __syncthreads();
   if (threadIdx.x == 0) {
     int sum = 0;
-    for (int w = 0; w < kActiveListThreads / 32; ++w) {
+    for (int w = 0; w < kCountThreads / 32; ++w) {
       const int c = warp_base[w];
       warp_base[w] = sum;
       sum += c;
@@ -399,7 +454,17 @@ __global__ void __launch_bounds__(kActiveListThreads) k_active_list(EngineArgs<T
     block_base = sum ? atomicAdd(a.act_count, sum) : 0;
   }
   __syncthreads();
-  if (act) a.act[block_base + warp_base[wid] + __popc(m & ((1u << lane) - 1u))] = t;
+  if (act) a.act[block_base + warp_base[wid] + __popc(m & ((1u << lane) - 1u))] = g;
+}
+
+// the scattering half: the cell-ordered copy of the positions
+template <class T>
+__global__ void k_site_scatter(EngineArgs<T> a, int parity, const int2* __restrict__ cellrank, Pt4<T>* __restrict__ sorted) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= a.n_sites) return;
+  const int2 cr = cellrank[g];
+  if (cr.x < 0) return;
+  sorted[__ldg(a.cell_start + cr.x) + cr.y] = a.S[parity][g];
 }
 
 // ---------------------------------------------------------------------------
@@ -413,13 +478,12 @@ __global__ void __launch_bounds__(kActiveListThreads) k_active_list(EngineArgs<T
 // the first kernel to read a.nnv.
 // ---------------------------------------------------------------------------
 template <class T>
-__global__ void k_frame_vertex(EngineArgs<T> a) {
+__global__ void k_frame_vertex(EngineArgs<T> a, int parity) {
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= __ldg(a.act_count)) return;
-  const Pt4<T> me = a.sorted[a.act[w]];
-  const int g = (int)me.id;
+  const int g = a.act[w];
   const MeshDev& md = a.meshes[a.segs[__ldg(a.site_seg + g)].mesh];
-  const V3<T> q{me.x, me.y, me.z};
+  const V3<T> q = ldp(a.S[parity], g);
   auto all = [](uint32_t) { return true; };
   TopK<T, 1> nv;
   const int old = a.nnv[g];
@@ -439,9 +503,7 @@ __global__ void k_frame_vertex(EngineArgs<T> a) {
 // ---------------------------------------------------------------------------
 // Site KNN (k_knn_verify + k_knn_search): exact K nearest other sites
 // within the site's segment (the reference's K+1 nearest with self dropped,
-// site_knn.cuh:79-103), one warp per site; lane j holds the j-th neighbour,
-// so the list row is read (for the freeze test's equality) and written
-// coalesced.  Sets same[g] (new list == stored list) and kth[g].
+// site_knn.cuh:79-103).  Sets same[g] (new list == stored list) and kth[g].
 // ---------------------------------------------------------------------------
 // Candidate lists (MM > 0): besides its K neighbours, a site keeps the MM
 // nearest other sites of its last full search (ids and the MM-th squared
@@ -460,43 +522,25 @@ __global__ void k_frame_vertex(EngineArgs<T> a) {
 // segment's first iteration) the full search runs for MM neighbours and
 // refreshes the list.  Margins of 1e-4 cover the rounding of the distances
 // and of the accumulated motion; a NaN motion fails every test.
-// The K-list of site g: lane j holds entry j (its key); writes the list
-// (local indices; only entries that changed), the K-th squared distance
-// (the next search's bound) and the `same` flag (list unchanged).
-template <class T, int KK>
-__device__ __forceinline__ void knn_store(const EngineArgs<T>& a, int g, const SegDev& sd,
-                                          typename KeyOps<T>::Key key, int lane) {
-  using O = KeyOps<T>;
-  const auto kth = shfl_key(key, KK - 1);
-  if (lane == 0) a.kth[g] = O::is_empty(kth) ? -1.f : (float)O::dist(kth);
-  const uint32_t gid = O::idx(key);
-  const uint32_t out = gid == 0xffffffffu ? 0xffffffffu : gid - (uint32_t)sd.site_base;
-  uint32_t* row = a.knn + (size_t)g * KK;
-  bool diff = false;
-  if (lane < KK) {
-    diff = row[lane] != out;
-    if (diff) row[lane] = out;
-  }
-  const unsigned changed = __ballot_sync(0xffffffffu, diff);
-  if (lane == 0) a.same[g] = changed ? 0 : 1;
-}
 
-// Full search of the site at sorted position t (one warp): the K nearest
-// (MM = 0), or the MM nearest, which refresh its candidate list and whose
-// first K are the K-list.  seg receives the site's segment.  With candidate
-// lists the search is first tried as one radius query (warp_radius_knn,
-// scratch buf of 64 keys): within bound tb when the check left one (the
-// largest re-keyed distance of the site's complete old list, so at least MM
-// sites lie within it), else within a squared distance expected to hold
-// about (MM + 64) / 2 sites; when the count falls outside [MM, 64] the ring
-// search runs instead.  Both return the MM smallest (distance, index) keys.
+// Full search of site g (one warp): the K nearest (MM = 0), or the MM
+// nearest, which refresh its candidate list and whose first K are the
+// K-list.  seg receives the site's segment.  With candidate lists the search
+// is first tried as one radius query (warp_radius_knn, scratch buf of 64
+// keys): within bound tb when the check left one (the largest re-keyed
+// distance of the site's complete old list, so at least MM sites lie within
+// it), else within a squared distance expected to hold about (MM + 64) / 2
+// sites; when the count falls outside [MM, 64] the ring search runs instead.
+// Both return the MM smallest (distance, caller index) keys; the list is
+// stored as internal indices.
 template <class T, int KK, int MM>
-__device__ __forceinline__ void knn_search_site(const EngineArgs<T>& a, int t, float tb, int lane, int& seg,
+__device__ __forceinline__ void knn_search_site(const EngineArgs<T>& a, int parity, int g, float tb, int lane, int& seg,
                                                 typename KeyOps<T>::Key* buf) {
   using O = KeyOps<T>;
   using Key = typename O::Key;
-  const Pt4<T> me = a.sorted[t];
-  const int g = (int)me.id;
+  constexpr int LEN = MM > 0 ? MM : KK;  // entries stored
+  constexpr int R = (LEN + 31) / 32;
+  const Pt4<T> me = a.S[parity][g];
   const int s = __ldg(a.site_seg + g);
   seg = s;
   const SegDev& sd = a.segs[s];
@@ -506,12 +550,11 @@ __device__ __forceinline__ void knn_search_site(const EngineArgs<T>& a, int t, f
   // the same K points), and the K-th distance equals the (K+1)-th with self.
   const V3<T> q{me.x, me.y, me.z};
   const float kp = a.kth[g];
-  const uint32_t self = (uint32_t)g;
+  const uint32_t self = me.id;
   auto not_self = [self](uint32_t id) { return id != self; };
-  Key key;
+  Key mk[2] = {O::empty(), O::empty()};
   if constexpr (MM > 0) {
     static_assert(MM <= 64, "at most 64 candidates");
-    Key mk[2];
     const float rho = a.cand_rho[g];
     const GridGeom G = a.geom[s];
     // kth holds the site's last K-th squared distance (K sites within it);
@@ -534,15 +577,11 @@ __device__ __forceinline__ void knn_search_site(const EngineArgs<T>& a, int t, f
         mk[1] = O::empty();
       }
     }
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-      if (32 * r + lane < MM) a.cand[(size_t)g * MM + 32 * r + lane] = O::idx(mk[r]);
     const Key mth = shfl_key(mk[(MM - 1) / 32], (MM - 1) % 32);
     if (lane == 0) {
       a.cand_rho[g] = O::is_empty(mth) ? __int_as_float(0x7f800000) : __fsqrt_rd(f32_rd(O::dist(mth)));
       a.cand_D[g] = 0.f;
     }
-    key = mk[0];
   } else {
     (void)tb; (void)buf;
     // candidates beyond 1.1x the last K-th squared distance are skipped; sites
@@ -551,128 +590,229 @@ __device__ __forceinline__ void knn_search_site(const EngineArgs<T>& a, int t, f
     const T thr0 = kp >= 0.f ? (T)kp * (T)1.1 : (T)sd.kth_est;
     Key kl[1];
     warp_knn<T, T, KK>(a.geom[s], a.cell_start, a.sorted, q, thr0, lane, not_self, kl);
-    key = kl[0];
+    mk[0] = kl[0];
   }
-  knn_store<T, KK>(a, g, sd, key, lane);
+  const Key kth = shfl_key(mk[0], KK - 1);
+  uint32_t* col = a.list + g;
+  bool diff = false;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int e = 32 * r + lane;
+    if (e < LEN) {
+      const uint32_t id = O::idx(mk[r]);
+      const uint32_t v = id == 0xffffffffu ? id : __ldg(a.internal_of + id);
+      if (e < KK) diff = diff || col[e * a.stride] != v;
+      col[e * a.stride] = v;
+    }
+  }
+  const unsigned changed = __ballot_sync(0xffffffffu, diff);
+  if (lane == 0) {
+    a.kth[g] = O::is_empty(kth) ? -1.f : (float)O::dist(kth);
+    a.same[g] = changed ? 0 : 1;
+  }
 }
 
-// Candidate-list check of active site w by a half warp (16 lanes, one site
-// each half, three list entries per lane: element e = 3 hl + r), so a warp
-// checks two sites at once.  The motion bound D grows by the largest last
-// motion M in the 8 coarse blocks nearest the site's old position (lanes
-// hl < 8 read one block each), which hold every site that started the step
-// within B/2 of it, plus the site's own motion; the step condition asks
-// that the segment's largest motion plus the site's own stay below
-// B/2 - rho (B/2 shrunk by 1e-3 for the rounding of cell coordinates), so a
-// site that started the step outside those blocks ends it beyond rho.  The list is re-keyed at the current positions and its
-// KK smallest selected in order (half_select3); it is accepted when the
-// KK-th is closer than rho - D.  `valid`: this half has a site.  Every lane
-// runs every warp-wide step; true when the half's K-list came from the list
-// (and is stored: row entries that changed, kth, same, the list's new
-// order, D).  bound: for a site whose complete list was re-keyed, the
-// largest re-keyed squared distance rounded up (its MM list sites are MM
-// other sites, so the MM nearest lie within it); else -1.
-template <class T, int KK, int MM>
-__device__ __forceinline__ bool knn_verify_half(const EngineArgs<T>& a, int parity, int w, bool valid, int lane,
-                                                int& seg, float& bound) {
-  static_assert(KK <= 32 && MM > KK && MM <= 48, "candidate list of KK < MM <= 48 entries");
-  using O = KeyOps<T>;
-  using Key = typename O::Key;
-  const int hl = lane & 15, half = lane >> 4;
-  const unsigned hmask = 0xffffu << (16 * half);
-  int g = -1, s = -1;
-  float rho = -1.f;
-  V3<T> q{0, 0, 0};
-  if (valid) {
-    const Pt4<T> me = a.sorted[a.act[w]];
-    g = (int)me.id;
-    s = __ldg(a.site_seg + g);
-    rho = a.cand_rho[g];
-    q = {me.x, me.y, me.z};
+// A thread's K (distance, internal index) keys in shared memory: entry t of
+// thread c at column c, so that a warp's accesses are conflict-free.
+template <class T, int KK, int BS> struct KeyColumns {
+  T d[KK][BS];
+  uint32_t i[KK][BS];
+  __device__ __forceinline__ void get(int t, int c, T& dd, uint32_t& id) const { dd = d[t][c]; id = i[t][c]; }
+  __device__ __forceinline__ void put(int t, int c, T dd, uint32_t id) { d[t][c] = dd; i[t][c] = id; }
+};
+template <int KK, int BS> struct KeyColumns<float, KK, BS> {
+  uint2 k[KK][BS];
+  __device__ __forceinline__ void get(int t, int c, float& dd, uint32_t& id) const {
+    const uint2 v = k[t][c];
+    dd = __uint_as_float(v.x); id = v.y;
   }
-  seg = s;
-  const bool have = valid && rho >= 0.f;
-  bool ok = have;
-  // motion bound: lanes hl and hl + 16 < 27 read blocks
-  unsigned mbits = 0u;
-  float D = 0.f, lim = 0.f;
-  if (ok) {
+  __device__ __forceinline__ void put(int t, int c, float dd, uint32_t id) { k[t][c] = make_uint2(__float_as_uint(dd), id); }
+};
+
+// Candidate-list check of active site g, one thread.  The motion bound D
+// grows by the largest last motion M in the 8 coarse blocks nearest the
+// site's old position, which hold every site that started the step within
+// B/2 of it, plus the site's own motion; the step condition asks that the
+// segment's largest motion plus the site's own stay below B/2 - rho (B/2
+// shrunk by 1e-3 for the rounding of cell coordinates), so a site that
+// started the step outside those blocks ends it beyond rho.  The list is
+// re-keyed at the current positions and its KK smallest kept in order by
+// insertion (the head of the list is the order of the last iteration, so most
+// entries go straight to the end); an entry pushed out of the first KK takes
+// the place of the one that pushed it.  Equal distances compare the caller's
+// indices.  The list is accepted when the KK-th is closer than rho - D.  True
+// when the K-list came from the list (and is stored: the entries that
+// changed, kth, same, D).  bound: for a site whose complete list was
+// re-keyed, the largest re-keyed squared distance rounded up (its MM list
+// sites are MM other sites, so the MM nearest lie within it); else -1.  A
+// rejected list is rewritten by the full search.
+template <class T, int KK, int MM, int BS>
+__device__ __forceinline__ bool knn_verify_site(const EngineArgs<T>& a, int parity, int g, int s,
+                                                KeyColumns<T, KK, BS>& L, float& bound) {
+  static_assert(MM > KK && MM % 4 == 0, "four entries per step");
+  constexpr uint32_t kNone = 0xffffffffu;
+  bound = -1.f;
+  const float rho = a.cand_rho[g];
+  if (!(rho >= 0.f)) return false;
+  const Pt4<T>* __restrict__ S = a.S[parity];
+  const int c = threadIdx.x;
+  uint32_t* col = a.list + g;
+  uint32_t id[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) id[j] = col[j * a.stride];
+  const V3<T> q = ldp(S, g);
+  float D, lim;
+  bool ok;
+  {
     const SegDev& sd = a.segs[s];
-    const GridGeom G = a.geom[s];
+    const GridGeom& G = a.geom[s];
     // the 2 x 2 x 2 blocks nearest the old position: per axis the block of
     // its cell and the neighbour on the side of the nearer block face, which
     // reach at least kBlockCells / 2 cells beyond the cell on either side
-    const V3<T> po = ld3(a.S[parity ^ 1], g);
+    const V3<T> po = ldp(a.S[parity ^ 1], g);
     const int c0[3] = {grid_coord(G, po.x, 0), grid_coord(G, po.y, 1), grid_coord(G, po.z, 2)};
-    int b0[3];
+    int b0[3], nb[3];
 #pragma unroll
-    for (int ax = 0; ax < 3; ++ax) b0[ax] = c0[ax] / kBlockCells - (c0[ax] % kBlockCells < kBlockCells / 2 ? 1 : 0);
-    const int dx = block_dim(G, 0), dy = block_dim(G, 1), dz = block_dim(G, 2);
-    if (hl < 8) {
-      const int x = b0[0] + (hl & 1), y = b0[1] + ((hl >> 1) & 1), z = b0[2] + (hl >> 2);
-      if (x >= 0 && x < dx && y >= 0 && y < dy && z >= 0 && z < dz) {
-        const unsigned long long v = a.blockmax[G.cell_base + (z * dy + y) * dx + x];
-        if ((unsigned)(v >> 32) == (unsigned)(sd.iter - 1)) mbits = (unsigned)v;
+    for (int ax = 0; ax < 3; ++ax) {
+      b0[ax] = c0[ax] / kBlockCells - (c0[ax] % kBlockCells < kBlockCells / 2 ? 1 : 0);
+      nb[ax] = block_dim(G, ax);
+    }
+    const unsigned stamp = (unsigned)(sd.iter - 1);
+    unsigned mbits = 0u;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int x = b0[0] + (k & 1), y = b0[1] + ((k >> 1) & 1), z = b0[2] + (k >> 2);
+      if (x >= 0 && x < nb[0] && y >= 0 && y < nb[1] && z >= 0 && z < nb[2]) {
+        const unsigned long long v = a.blockmax[G.cell_base + (z * nb[1] + y) * nb[0] + x];
+        if ((unsigned)(v >> 32) == stamp) mbits = max(mbits, (unsigned)v);
       }
     }
-    mbits = __reduce_max_sync(hmask, mbits);
     // this site's own motion (also inside M, but usually far below it)
-    const float mu = __fsqrt_rn(f32_ru(dist2(q, ld3(a.S[parity ^ 1], g)))) * 1.000001f;
+    const float mu = __fsqrt_rn(f32_ru(dist2(q, po))) * 1.000001f;
     D = __fadd_ru(a.cand_D[g], __fadd_ru(__uint_as_float(mbits), mu));
     const bool step_ok = __fadd_ru(sd.step_motion, mu) * 1.0001f < (0.4995f * (float)kBlockCells * G.h - rho) * 0.9999f;
     lim = rho * 0.9999f - D * 1.0001f;
     ok = isinf(rho) || (step_ok && lim > 0.f);
   }
-  // re-key and select (both halves take part in every pass)
-  Key k[3];
+  auto less = [&](T da, uint32_t ia, T db, uint32_t ib) {
+    if (da != db) return da < db;
+    return S[ia].id < S[ib].id;
+  };
+  T dmax = (T)0, dk = (T)0;  // largest distance; the last kept key
+  uint32_t ik = kNone;
+  int cnt = 0, nv = 0, lo = KK;  // kept keys, list entries, first position that changed
+  bool finite = true;
+#pragma unroll 1
+  for (int e0 = 0; e0 < MM; e0 += 4) {
+    uint32_t cur[4];
+    V3<T> p[4];
 #pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    const int e = 3 * hl + r;
-    k[r] = O::empty();
-    if (have && e < MM) {
-      const uint32_t id = __ldg(a.cand + (size_t)g * MM + e);
-      if (id != 0xffffffffu) k[r] = O::make(dist2(ld3(a.S[parity], (long)id), q), id);
+    for (int j = 0; j < 4; ++j) {
+      cur[j] = id[j];
+      p[j] = cur[j] != kNone ? ldp(S, cur[j]) : q;
+      if (e0 + 4 < MM) id[j] = col[(e0 + 4 + j) * a.stride];
     }
-  }
-  bool moved;
-  half_select3<T, KK>(k, hl, half, moved);
-  constexpr int KL = (KK - 1) / 3, KR = (KK - 1) % 3;
-  const Key kth = shfl16_key(k[KR], KL);
-  {
-    T dm = (T)0;
-    int nv = 0;
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
-      if (!O::is_empty(k[r])) { const T d = O::dist(k[r]); dm = d > dm ? d : dm; ++nv; }
-#pragma unroll
-    for (int o = 8; o >= 1; o >>= 1) {
-      const T od = __shfl_xor_sync(0xffffffffu, dm, o, 16);
-      dm = od > dm ? od : dm;
-      nv += __shfl_xor_sync(0xffffffffu, nv, o, 16);
-    }
-    bound = have && nv == MM ? f32_ru(dm) : -1.f;
-  }
-  ok = ok && !O::is_empty(kth) && (isinf(rho) || f32_ru(O::dist(kth)) * 1.0003f < lim * lim);
-  // store (per half: entries e < KK of this lane, the flags by lane hl 0)
-  bool diff = false;
-  if (ok) {
-    const uint32_t base = (uint32_t)a.segs[s].site_base;
-    uint32_t* row = a.knn + (size_t)g * KK;
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      const int e = 3 * hl + r;
-      if (moved && e < MM) a.cand[(size_t)g * MM + e] = O::idx(k[r]);
-      if (e < KK) {
-        const uint32_t gid = O::idx(k[r]);
-        const uint32_t out = gid == 0xffffffffu ? 0xffffffffu : gid - base;
-        if (row[e] != out) { row[e] = out; diff = true; }
+    for (int j = 0; j < 4; ++j) {
+      if (cur[j] == kNone) continue;
+      const T d = dist2(p[j], q);
+      ++nv;
+      finite = finite && d < (T)INFINITY;
+      dmax = d > dmax ? d : dmax;
+      if (!ok) continue;
+      const bool below = cnt > 0 && less(d, cur[j], dk, ik);
+      if (!below) {
+        if (cnt < KK) { L.put(cnt++, c, d, cur[j]); dk = d; ik = cur[j]; }
+        continue;
       }
+      const bool full = cnt == KK;
+      if (full) col[(e0 + j) * a.stride] = ik; else ++cnt;
+      int t = cnt - 1;
+      while (t > 0) {
+        T dt;
+        uint32_t it;
+        L.get(t - 1, c, dt, it);
+        if (!less(d, cur[j], dt, it)) break;
+        L.put(t, c, dt, it);
+        --t;
+      }
+      L.put(t, c, d, cur[j]);
+      lo = min(lo, t);
+      if (full) L.get(KK - 1, c, dk, ik);
     }
-    if (hl == 0) { a.cand_D[g] = D; a.kth[g] = (float)O::dist(kth); }
   }
-  const unsigned changed = __ballot_sync(0xffffffffu, diff) & hmask;
-  if (ok && hl == 0) a.same[g] = changed ? 0 : 1;
+  bound = nv == MM && finite ? f32_ru(dmax) : -1.f;
+  ok = ok && cnt == KK && finite && (isinf(rho) || f32_ru(dk) * 1.0003f < lim * lim);
+  if (ok) {
+    for (int t = lo; t < KK; ++t) {
+      T dt;
+      uint32_t it;
+      L.get(t, c, dt, it);
+      col[t * a.stride] = it;
+    }
+    a.cand_D[g] = D;
+    a.kth[g] = (float)dk;
+    a.same[g] = lo == KK ? 1 : 0;
+  }
   return ok;
+}
+
+// k_knn_verify: the check of every active site, one thread per site; the
+// sites it leaves are appended to a.srch once per block, the lists it proved
+// are added to their segment's statistics (word 6 of the iteration's slot).
+// Bound by instruction issue and the latency of the gathers.  Measured on 300k
+// sites, K = 24, after 10 iterations: 75 us at 116 warp instructions per site;
+// a half warp per site with the keys in registers (odd-even passes over
+// shuffles, 12-byte positions in the caller's order) took 167 us and 358.
+// 64 threads: 12 KB of keys (K = 24), 16 blocks on an SM.
+constexpr int kVerifyThreads = 64;
+
+template <class T, int KK, int MM>
+__global__ void __launch_bounds__(kVerifyThreads, sizeof(T) == 8 ? 8 : 16) k_knn_verify(EngineArgs<T> a, int parity) {
+  constexpr int BS = kVerifyThreads;
+  __shared__ KeyColumns<T, KK, BS> L;
+  __shared__ int warp_base[BS / 32], block_base, st_seg, st_n;
+  const int n = __ldg(a.act_count);
+  if (blockIdx.x * BS >= n) return;
+  if (threadIdx.x == 0) { st_seg = -1; st_n = 0; }
+  const int w = blockIdx.x * BS + threadIdx.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int g = -1, s = -1;
+  float bound = -1.f;
+  bool ok = false;
+  if (w < n) {
+    g = a.act[w];
+    s = __ldg(a.site_seg + g);
+    ok = knn_verify_site<T, KK, MM, BS>(a, parity, g, s, L, bound);
+  }
+  const bool need = g >= 0 && !ok;
+  const unsigned m = __ballot_sync(0xffffffffu, need);
+  if (lane == 0) warp_base[wid] = __popc(m);
+  __syncthreads();
+  const int key = ok ? s : -1;
+  const unsigned peers = __match_any_sync(0xffffffffu, key);
+  if (key >= 0 && lane == __ffs(peers) - 1) {
+    const int owner = atomicCAS(&st_seg, -1, key);
+    int* word = a.stats + ((size_t)key * kStatsRing + (a.segs[key].iter % kStatsRing)) * kStatsWords + 6;
+    if (owner == -1 || owner == key) atomicAdd(&st_n, __popc(peers)); else atomicAdd(word, __popc(peers));
+  }
+  if (threadIdx.x == 0) {
+    int sum = 0;
+    for (int k = 0; k < BS / 32; ++k) {
+      const int cw = warp_base[k];
+      warp_base[k] = sum;
+      sum += cw;
+    }
+    block_base = sum ? atomicAdd(a.srch, sum) : 0;
+  }
+  __syncthreads();
+  if (need) {
+    const int slot = block_base + warp_base[wid] + __popc(m & ((1u << lane) - 1u));
+    a.srch[1 + slot] = g;
+    a.srch_thr[slot] = bound;
+  }
+  if (threadIdx.x == 0 && st_seg >= 0)
+    atomicAdd(a.stats + ((size_t)st_seg * kStatsRing + (a.segs[st_seg].iter % kStatsRing)) * kStatsWords + 6, st_n);
 }
 
 // Per-warp running count of one statistics word for the segment it is on:
@@ -680,7 +820,6 @@ __device__ __forceinline__ bool knn_verify_half(const EngineArgs<T>& a, int pari
 template <class T>
 struct SegCounter {
   int cur = -1, n = 0;
-  // `lane` 0 adds for the whole warp (or half warp: pass its lane within the half)
   __device__ __forceinline__ void add(const EngineArgs<T>& a, int seg, int word, int lane) {
     if (seg != cur) { flush(a, word, lane); cur = seg; n = 0; }
     ++n;
@@ -691,55 +830,14 @@ struct SegCounter {
   }
 };
 
-// Site KNN, two persistent kernels, each launched with the warps its launch
-// bounds keep resident on every SM (so no block waits for a second wave):
-// k_knn_verify's warp i takes active positions i, i + nw, i + 2 nw, ...,
-// takes each site's K-list from its candidate list where the motion bound
-// proves it exact, and appends the other sites to its own part of a.srch
-// (no atomics: every verify warp owns a.srch_cap slots); k_knn_search's warp
-// j searches, in full, the sites of verify warps j, j + nws, ...  Without
-// candidate lists (MM = 0) only k_knn_search runs, over every active site.
-// The reused lists and the full searches are added to the segments'
-// statistics (words 6 and 7 of the iteration's slot).
-constexpr int kKnnVerifyWarpsPerSM = 48;
+// k_knn_search: full searches, persistent with the warps its launch bounds
+// keep resident on every SM (so no block waits for a second wave), one warp
+// per site: the sites the check left (a.srch), or without candidate lists
+// (MM = 0) every active site.  Counted in word 7 of the statistics.
 constexpr int kKnnSearchWarpsPerSM = 32;
 
 template <class T, int KK, int MM, int BS>
-__global__ void __launch_bounds__(BS, kKnnVerifyWarpsPerSM * 32 / BS) k_knn_verify(EngineArgs<T> a, int parity) {
-  const int lane = threadIdx.x & 31;
-  const int wi = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
-  const int nw = (int)((gridDim.x * (unsigned)blockDim.x) >> 5);
-  const int n = __ldg(a.act_count);
-  int* mine = a.srch + (size_t)wi * a.srch_cap;
-  float* mine_thr = a.srch_thr + (size_t)wi * a.srch_cap;
-  int cnt = 0;
-  SegCounter<T> reused;  // per half, kept by lanes 0 and 16
-  const int hl = lane & 15, half = lane >> 4;
-  // two sites per warp: the halves take positions 2i + half, 2i + half + 2 nw, ...
-  for (int w0 = 2 * wi; w0 < n; w0 += 2 * nw) {
-    const int w = w0 + half;
-    int seg;
-    float bound;
-    const bool ok = knn_verify_half<T, KK, MM>(a, parity, w, w < n, lane, seg, bound);
-    const bool need = w < n && !ok;
-    if (ok) reused.add(a, seg, 6, hl);
-    // the warp's list: half 0's site first, then half 1's
-    const unsigned b = __ballot_sync(0xffffffffu, need && hl == 0);
-    if (need && hl == 0) {
-      const int slot = cnt + (half ? (int)(b & 1u) : 0);
-      mine[slot] = a.act[w];
-      mine_thr[slot] = bound;
-    }
-    cnt += __popc(b);
-  }
-  reused.flush(a, 6, hl);
-  if (lane == 0) a.srch_n[wi] = cnt;
-}
-
-template <class T, int KK, int MM, int BS>
-__global__ void __launch_bounds__(BS, kKnnSearchWarpsPerSM * 32 / BS) k_knn_search(EngineArgs<T> a, int parity,
-                                                                                   int n_lists) {
-  (void)parity;
+__global__ void __launch_bounds__(BS, kKnnSearchWarpsPerSM * 32 / BS) k_knn_search(EngineArgs<T> a, int parity) {
   const int lane = threadIdx.x & 31;
   const int wi = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
   const int nw = (int)((gridDim.x * (unsigned)blockDim.x) >> 5);
@@ -747,21 +845,17 @@ __global__ void __launch_bounds__(BS, kKnnSearchWarpsPerSM * 32 / BS) k_knn_sear
   if constexpr (MM > 0) {
     __shared__ typename KeyOps<T>::Key buf[BS / 32][64];  // per warp: the radius query's keys
     auto* mybuf = buf[threadIdx.x >> 5];
-    for (int l = wi; l < n_lists; l += nw) {
-      const int* list = a.srch + (size_t)l * a.srch_cap;
-      const float* thr = a.srch_thr + (size_t)l * a.srch_cap;
-      const int n = a.srch_n[l];
-      for (int k = 0; k < n; ++k) {
-        int seg;
-        knn_search_site<T, KK, MM>(a, list[k], thr[k], lane, seg, mybuf);
-        searched.add(a, seg, 7, lane);
-      }
+    const int n = a.srch[0];
+    for (int k = wi; k < n; k += nw) {
+      int seg;
+      knn_search_site<T, KK, MM>(a, parity, a.srch[1 + k], a.srch_thr[k], lane, seg, mybuf);
+      searched.add(a, seg, 7, lane);
     }
   } else {
     const int n = __ldg(a.act_count);
     for (int w = wi; w < n; w += nw) {
       int seg;
-      knn_search_site<T, KK, MM>(a, a.act[w], -1.f, lane, seg, nullptr);
+      knn_search_site<T, KK, MM>(a, parity, a.act[w], -1.f, lane, seg, nullptr);
       searched.add(a, seg, 7, lane);
     }
   }
@@ -788,25 +882,24 @@ __device__ __forceinline__ bool site_clip(const EngineArgs<typename PT<PROF>::T>
   const int s = __ldg(a.site_seg + g);
   const SegDev& sd = a.segs[s];
   const MeshDev& md = a.meshes[sd.mesh];
-  const T* __restrict__ S = a.S[parity];
+  const ListNeighbours<T> nb{a.S[parity], a.list + g, a.stride};
   const bool fz = sd.mode != 0 && a.frozen[g];
-  const V3<T> si = ld3(S, g);
+  const V3<T> si = ldp(a.S[parity], g);
   // frame from the nearest vertex normal (frozen sites: their kept vertex
   // list; with the BVH projection, which keeps no vertex list, their kept
   // frame vertex); FRAME 1: from the PCA normal of the neighbour list,
   // started from that vertex normal
-  const int nn = (fz && a.proj_mode == 0) ? a.knnv[(size_t)g * kKProj] : a.nnv[g];
+  const int nn = (fz && a.proj_mode == 0) ? a.knnv[g] : a.nnv[g];
   Frame<T> fr;
   if (nn < 0) {
     fr = {{(T)1, (T)0, (T)0}, {(T)0, (T)1, (T)0}};
   } else {
     V3<T> n0{(T)__ldg(md.N + 3 * nn), (T)__ldg(md.N + 3 * nn + 1), (T)__ldg(md.N + 3 * nn + 2)};
-    if (FRAME == 1) n0 = pca_normal(S, sd.site_base, sd.n_sites, a.knn + (size_t)g * a.K, a.K, si, n0);
+    if (FRAME == 1) n0 = pca_normal<T>(nb, a.K, si, n0);
     fr = frame_from_normal(n0);
   }
   PolyRef<PP> cur = A, nxt = B;
-  const int np = clip_cell<PROF>(S, sd.site_base, sd.n_sites, si, a.knn + (size_t)g * a.K, a.K, fr, md.R, cur, nxt,
-                                 cap, !fz);
+  const int np = clip_cell<PROF>(nb, si, a.K, fr, md.R, cur, nxt, cap, !fz);
   if (np < 0) return false;
   const V2<PP> c2 = poly_centroid<PP>(cur, np, PROF == PROF_MIXED);
   V3<T> cent;
@@ -828,10 +921,8 @@ __global__ void __launch_bounds__(BLOCK, (sizeof(typename PT<PROF>::PP) == 8 ? k
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V2<PP>* sm = reinterpret_cast<V2<PP>*>(smem_raw);
   PolyRef<PP> A{sm + threadIdx.x, BLOCK}, B{sm + CAP * BLOCK + threadIdx.x, BLOCK};
-  const int t = blockIdx.x * BLOCK + threadIdx.x;
-  const int n_grid = __ldg(a.cell_start + a.total_cells);
-  if (t < n_grid) {
-    const int g = (int)a.sorted[t].id;
+  const int g = blockIdx.x * BLOCK + threadIdx.x;
+  if (active_seg(a, g) >= 0) {
     if (!site_clip<PROF, FRAME>(a, parity, g, A, B, CAP)) {
       const int k = atomicAdd(a.ovf, 1);
       a.ovf[1 + k] = g;
@@ -858,11 +949,9 @@ __device__ __forceinline__ void site_finish(const EngineArgs<typename PT<PROF>::
   const int s = __ldg(a.site_seg + g);
   const SegDev& sd = a.segs[s];
   const MeshDev& md = a.meshes[sd.mesh];
-  const int K = a.K;
-  const uint32_t* row = a.knn + (size_t)g * K;
-  const int i = g - sd.site_base;
   const bool fz = sd.mode != 0 && a.frozen[g];
-  const V3<T> si = ld3(a.S[parity], g);
+  const Pt4<T> me = a.S[parity][g];
+  const V3<T> si{me.x, me.y, me.z};
   const V3<T> cent = ld3((const T*)a.cent, g);
 
   // projection
@@ -877,18 +966,18 @@ __device__ __forceinline__ void site_finish(const EngineArgs<typename PT<PROF>::
   } else {
     sn = project_onering_rec<T, double>(cent, md.ring, md.nV, md.vf_off, knnv, kKProj);
   }
-  st3(a.S[parity ^ 1], g, sn);
+  a.S[parity ^ 1][g] = Pt4<T>{sn.x, sn.y, sn.z, me.id};
 
   // tiers on the segment's first iteration (modes 1/2)
   const int it = sd.iter;
   if (it == 0 && sd.mode != 0) {
-    const int base = sd.site_base;
     auto normal = [&](int j, float out[3]) {
-      int v = a.nnv[base + j];
+      int v = a.nnv[j];
       if (v < 0) { out[0] = out[1] = out[2] = 0.f; return; }
       out[0] = __ldg(md.N + 3 * v); out[1] = __ldg(md.N + 3 * v + 1); out[2] = __ldg(md.N + 3 * v + 2);
     };
-    a.tier[g] = (uint8_t)tier_of(sd.mode, i, sd.n_sites, K, row, normal);
+    auto row = [&](int t) { return (int)a.list[t * a.stride + g]; };
+    a.tier[g] = (uint8_t)tier_of(sd.mode, g, a.K, row, normal);
   }
 
   // freeze test + apply
@@ -936,17 +1025,14 @@ constexpr int kVertexDeferred = -2;
 template <int PROF, int BS>
 __global__ void __launch_bounds__(BS, PROF == PROF_FP64 ? 1 : 1536 / BS) k_site_vsearch(EngineArgs<typename PT<PROF>::T> a, int parity) {
   using T = typename PT<PROF>::T;
-  (void)parity;
-  const int t = blockIdx.x * BS + threadIdx.x;
-  const int n_grid = __ldg(a.cell_start + a.total_cells);
-  if (t >= n_grid) return;
-  const int g = (int)a.sorted[t].id;
-  const int s = __ldg(a.site_seg + g);
+  const int g = blockIdx.x * BS + threadIdx.x;
+  const int s = active_seg(a, g);
+  if (s < 0) return;
   const SegDev& sd = a.segs[s];
   if (sd.mode != 0 && a.frozen[g]) return;  // frozen sites keep their vertices
   const MeshDev& md = a.meshes[sd.mesh];
-  int* kv = a.knnv + (size_t)g * kKProj;
-  const int skip = (sd.mode == 0 && sd.ex_quirk) ? g - sd.site_base : -1;
+  int* kv = a.knnv + g;
+  const int skip = (sd.mode == 0 && sd.ex_quirk) ? (int)a.S[parity][g].id - sd.site_base : -1;
   auto accept = [skip](uint32_t id) { return (int)id != skip; };
   const V3<T> c = ld3((const T*)a.cent, g);
   TopK<T, kKProj> top;
@@ -959,7 +1045,7 @@ __global__ void __launch_bounds__(BS, PROF == PROF_FP64 ? 1 : 1536 / BS) k_site_
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < kKProj; ++k) {
-      const int v = kv[k];
+      const int v = kv[k * a.stride];
       ok = ok && (unsigned)v < (unsigned)md.nV && v != skip;
       if (ok) {
         const V3<T> pv{(T)__ldg(md.V + 3 * v), (T)__ldg(md.V + 3 * v + 1), (T)__ldg(md.V + 3 * v + 2)};
@@ -982,7 +1068,7 @@ __global__ void __launch_bounds__(BS, PROF == PROF_FP64 ? 1 : 1536 / BS) k_site_
     return;
   }
 #pragma unroll
-  for (int k = 0; k < kKProj; ++k) kv[k] = (int)KeyOps<T>::idx(top.k[k]);
+  for (int k = 0; k < kKProj; ++k) kv[k * a.stride] = (int)KeyOps<T>::idx(top.k[k]);
 }
 
 // Everything after the centroid and (PROJ 0) the vertex search of
@@ -995,10 +1081,9 @@ __device__ __forceinline__ bool site_proj(const EngineArgs<typename PT<PROF>::T>
     site_finish<PROF, 1>(a, parity, g, none, o);
     return true;
   }
-  const int* kv = a.knnv + (size_t)g * kKProj;
   int knnv[kKProj];
 #pragma unroll
-  for (int k = 0; k < kKProj; ++k) knnv[k] = kv[k];
+  for (int k = 0; k < kKProj; ++k) knnv[k] = a.knnv[k * a.stride + g];
   if (knnv[0] == kVertexDeferred) return false;
   site_finish<PROF, 0>(a, parity, g, knnv, o);
   return true;
@@ -1079,7 +1164,7 @@ __device__ __forceinline__ void motion_to_block(const EngineArgs<T>& a, int pari
   unsigned bits = 0u, stamp = 0u;
   if (g >= 0 && o.seg >= 0) {
     int bx, by, bz;
-    blk = motion_block(a.geom[o.seg], ld3(a.S[parity], g), bx, by, bz);
+    blk = motion_block(a.geom[o.seg], ldp(a.S[parity], g), bx, by, bz);
     bits = __float_as_uint(sqrtf(o.disp2));
     stamp = (unsigned)a.segs[o.seg].iter;
   }
@@ -1097,14 +1182,9 @@ __global__ void __launch_bounds__(BS, PROJ == 0 ? 768 / BS : 1) k_site_proj(Engi
   __shared__ StatsStage stage;
   stats_stage_init(stage);
   __syncthreads();
-  const int t = blockIdx.x * BS + threadIdx.x;
-  const int n_grid = __ldg(a.cell_start + a.total_cells);
+  const int g = blockIdx.x * BS + threadIdx.x;
   SiteOut o{-1, 0, 0, 0, 0, 0.f};
-  int g = -1;
-  if (t < n_grid) {
-    g = (int)a.sorted[t].id;
-    site_proj<PROF, PROJ>(a, parity, g, o);
-  }
+  if (active_seg(a, g) >= 0) site_proj<PROF, PROJ>(a, parity, g, o);
   if (a.blockmax) motion_to_block(a, parity, g, o);
   stats_flush(a.stats, a.segs, o, stage);
   __syncthreads();
@@ -1116,7 +1196,7 @@ __global__ void __launch_bounds__(BS, PROJ == 0 ? 768 / BS : 1) k_site_proj(Engi
 // no longer gridded or iterated: active = 2), reset the overflow, deferred
 // and active-site counts for the next iteration.
 __device__ __forceinline__ void seg_advance(SegDev* segs, int* active, int nseg, int* stats, int* ovf, int* far,
-                                            int* act_count) {
+                                            int* act_count, int* srch) {
   for (int s = threadIdx.x; s < nseg; s += blockDim.x) {
     if (active[s] != 1) continue;
     int it = segs[s].iter;
@@ -1133,7 +1213,10 @@ __device__ __forceinline__ void seg_advance(SegDev* segs, int* active, int nseg,
     const int cap = segs[s].stop_iters;
     if ((lim >= 0.f && d2 <= lim) || (cap > 0 && nx >= cap)) active[s] = 2;
   }
-  if (threadIdx.x == 0) { ovf[0] = 0; far[0] = 0; *act_count = 0; }
+  if (threadIdx.x == 0) {
+    ovf[0] = 0; far[0] = 0; *act_count = 0;
+    if (srch) srch[0] = 0;
+  }
 }
 
 // Deferred sites (a.far): one block per site finds the 5 nearest mesh
@@ -1155,7 +1238,7 @@ __global__ void __launch_bounds__(128) k_site_far(EngineArgs<typename PT<PROF>::
     const int s = __ldg(a.site_seg + g);
     const SegDev& sd = a.segs[s];
     const MeshDev& md = a.meshes[sd.mesh];
-    const int skip = (sd.mode == 0 && sd.ex_quirk) ? g - sd.site_base : -1;
+    const int skip = (sd.mode == 0 && sd.ex_quirk) ? (int)a.S[parity][g].id - sd.site_base : -1;
     const V3<T> q = ld3((const T*)a.cent, g);
     TopK<T, kKProj> top;
     for (int v = threadIdx.x; v < md.nV; v += 128) {
@@ -1171,15 +1254,17 @@ __global__ void __launch_bounds__(128) k_site_far(EngineArgs<typename PT<PROF>::
       TopK<T, kKProj> all;
       for (int j = 0; j < 128 * kKProj; ++j) all.insert(keys[j]);
       int knnv[kKProj];
-      int* kv = a.knnv + (size_t)g * kKProj;
 #pragma unroll
-      for (int j = 0; j < kKProj; ++j) { knnv[j] = (int)KeyOps<T>::idx(all.k[j]); kv[j] = knnv[j]; }
+      for (int j = 0; j < kKProj; ++j) {
+        knnv[j] = (int)KeyOps<T>::idx(all.k[j]);
+        a.knnv[j * a.stride + g] = knnv[j];
+      }
       SiteOut o{-1, 0, 0, 0, 0, 0.f};
       site_finish<PROF, 0>(a, parity, g, knnv, o);
       stats_atomic(a.stats, a.segs, o);
       if (a.blockmax) {
         int bx, by, bz;
-        const int blk = motion_block(a.geom[o.seg], ld3(a.S[parity], g), bx, by, bz);
+        const int blk = motion_block(a.geom[o.seg], ldp(a.S[parity], g), bx, by, bz);
         atomicMax(a.blockmax + blk, ((unsigned long long)(unsigned)a.segs[o.seg].iter << 32) |
                                         __float_as_uint(sqrtf(o.disp2)));
       }
@@ -1193,7 +1278,7 @@ __global__ void __launch_bounds__(128) k_site_far(EngineArgs<typename PT<PROF>::
   __syncthreads();
   if (!last) return;
   __threadfence();
-  seg_advance(segs, active, nseg, a.stats, a.ovf, a.far, a.act_count);
+  seg_advance(segs, active, nseg, a.stats, a.ovf, a.far, a.act_count, a.srch);
   if (threadIdx.x == 0) *ticket = 0u;
 }
 

@@ -84,11 +84,33 @@ __global__ void __launch_bounds__(128) k_hausdorff(const float* __restrict__ Vc,
 // ---------------------------------------------------------------------------
 constexpr int kFaceMaxPoly = 256;   // MAX_POLY (main.cu:393)
 
+// Neighbour lists of k_face_keys: get(i, t) is entry t of site i's list (an
+// index into the sites, or out of range), label(i) the index that a site has
+// in the faces.
+struct FaceRows {  // row-major lists
+  const uint32_t* knn;
+  int K;
+  __device__ __forceinline__ int get(int i, int t) const { return (int)knn[(size_t)i * K + t]; }
+  __device__ __forceinline__ int label(int i) const { return i; }
+};
+struct FaceColumns {  // an engine segment's lists (from its first site on)
+  const uint32_t* list;
+  const int* labels;
+  size_t stride;
+  uint32_t base;
+  __device__ __forceinline__ int get(int i, int t) const {
+    const uint32_t j = list[t * stride + i];
+    return j == 0xffffffffu ? -1 : (int)(j - base);
+  }
+  __device__ __forceinline__ int label(int i) const { return labels[i]; }
+};
+
 // Labelled clip (near_project.cuh:201-244) + active-bisector pairs
 // (near_project.cuh:318-351) + key emission (buildmesh.cuh:170-201) per site.
 // Buffers: per thread 2 x kFaceMaxPoly float2 + labels in local memory.
+template <class NB>
 __global__ void __launch_bounds__(64) k_face_keys(const float* __restrict__ S, const float* __restrict__ U,
-                                                  const float* __restrict__ Vv, const uint32_t* __restrict__ knn,
+                                                  const float* __restrict__ Vv, NB nb,
                                                   int n, int K, float R2, float eps_clip, float tol_active,
                                                   unsigned long long* keys, int* key_count, int max_keys) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -101,9 +123,8 @@ __global__ void __launch_bounds__(64) k_face_keys(const float* __restrict__ S, c
   cp[0] = make_float2(-R2, -R2); cp[1] = make_float2(R2, -R2); cp[2] = make_float2(R2, R2); cp[3] = make_float2(-R2, R2);
   cl[0] = cl[1] = cl[2] = cl[3] = -1;
   const V3<float> si = ld3(S, i), ui = ld3(U, i), vi = ld3(Vv, i);
-  const uint32_t* nb = knn + (size_t)i * K;
   for (int t = 0; t < K; ++t) {
-    int j = (int)nb[t];
+    int j = nb.get(i, t);
     if ((unsigned)j >= (unsigned)n || j == i) continue;
     V3<float> d = sub3(ld3(S, j), si);
     float a = dot3(d, ui), b = dot3(d, vi), c = 0.5f * dot3(d, d);
@@ -140,7 +161,7 @@ __global__ void __launch_bounds__(64) k_face_keys(const float* __restrict__ S, c
     float b1 = 1e30f, b2 = 1e30f;
     int j1 = -1, j2 = -1;
     for (int t = 0; t < K; ++t) {
-      int j = (int)nb[t];
+      int j = nb.get(i, t);
       if ((unsigned)j >= (unsigned)n || j == i) continue;
       V3<float> d = sub3(ld3(S, j), si);
       float a = dot3(d, ui), b = dot3(d, vi), c = 0.5f * dot3(d, d);
@@ -149,7 +170,7 @@ __global__ void __launch_bounds__(64) k_face_keys(const float* __restrict__ S, c
       else if (s < b2) { b2 = s; j2 = j; }
     }
     if (!(j1 >= 0 && j2 >= 0 && j1 != j2 && b1 <= tol_active && b2 <= tol_active)) continue;
-    int x = i, y = j1, z = j2, tmp;
+    int x = nb.label(i), y = nb.label(j1), z = nb.label(j2), tmp;
     if (x > y) { tmp = x; x = y; y = tmp; }
     if (y > z) { tmp = y; y = z; z = tmp; }
     if (x > y) { tmp = x; x = y; y = tmp; }

@@ -26,6 +26,12 @@ struct GridGeom {
 // Cell-ordered copy of a point: coordinates plus the point's global index.
 template <class T> struct alignas(16) Pt4 { T x, y, z; uint32_t id; };
 
+// position of point i (one 16-byte load; FP64: two)
+template <class T> __device__ __forceinline__ V3<T> ldp(const Pt4<T>* __restrict__ P, uint32_t i) {
+  const Pt4<T> p = P[i];
+  return {p.x, p.y, p.z};
+}
+
 template <class T>
 __device__ __forceinline__ int grid_coord(const GridGeom& g, T v, int a) {
   float f = floorf(((float)v - g.lo[a]) * g.inv_h);
@@ -472,76 +478,6 @@ __device__ __forceinline__ bool warp_radius_knn(const GridGeom& g, const int* __
   __syncwarp();  // every lane has read buf before the next query writes it
   warp_bitonic64<T>(list, lane);
   return true;
-}
-
-// ---------------------------------------------------------------------------
-// Warp-wide selection of the KK smallest keys of short lists, in order,
-// one list per half warp (16 lanes) with three keys per lane (element
-// e = 3 hl + r, hl = lane within the half): odd-even transposition passes
-// until the first KK elements are in order and every later one is above the
-// KK-th (the order among the later ones does not matter).  A list that is
-// already nearly in order (a site's candidate list from an earlier
-// iteration, re-keyed at the sites' new positions) needs a pass or two; 64
-// passes order any list.  Every pass is an odd-even transposition of the
-// half's 48 elements; both
-// halves run the same passes (the shuffles are warp-wide), a half that is
-// in order only repeats no-op exchanges.  `moved` tells whether this half's
-// keys moved.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long shfl16_key(unsigned long long k, int src) {
-  return __shfl_sync(0xffffffffu, k, src, 16);
-}
-__device__ __forceinline__ DKey shfl16_key(DKey k, int src) {
-  return {__shfl_sync(0xffffffffu, k.d, src, 16), __shfl_sync(0xffffffffu, k.i, src, 16)};
-}
-__device__ __forceinline__ unsigned long long shfl16_down_key(unsigned long long k) {
-  return __shfl_down_sync(0xffffffffu, k, 1, 16);
-}
-__device__ __forceinline__ DKey shfl16_down_key(DKey k) {
-  return {__shfl_down_sync(0xffffffffu, k.d, 1, 16), __shfl_down_sync(0xffffffffu, k.i, 1, 16)};
-}
-__device__ __forceinline__ unsigned long long shfl16_up_key(unsigned long long k) {
-  return __shfl_up_sync(0xffffffffu, k, 1, 16);
-}
-__device__ __forceinline__ DKey shfl16_up_key(DKey k) {
-  return {__shfl_up_sync(0xffffffffu, k.d, 1, 16), __shfl_up_sync(0xffffffffu, k.i, 1, 16)};
-}
-
-template <class T, int KK>
-__device__ __forceinline__ void half_select3(typename KeyOps<T>::Key (&k)[3], int hl, int half, bool& moved) {
-  using O = KeyOps<T>;
-  constexpr int KL = (KK - 1) / 3, KR = (KK - 1) % 3;  // lane and register of element KK-1
-  const int e0 = 3 * hl;
-  moved = false;
-  for (int pass = 0; pass < 64; ++pass) {
-    const auto nx0 = shfl16_down_key(k[0]);
-    const auto kth = shfl16_key(k[KR], KL);
-    const bool kth_empty = O::is_empty(kth);
-    bool ok = true;
-    if (e0 + 1 <= KK - 1) ok = ok && O::less(k[0], k[1]);
-    if (e0 + 2 <= KK - 1) ok = ok && O::less(k[1], k[2]);
-    if (e0 + 3 <= KK - 1 && hl < 15) ok = ok && O::less(k[2], nx0);
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-      if (e0 + r >= KK) ok = ok && (kth_empty || O::less(kth, k[r]));
-    const unsigned b = __ballot_sync(0xffffffffu, ok);
-    if (b == 0xffffffffu) break;
-    if (((b >> (16 * half)) & 0xffffu) != 0xffffu) moved = true;
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      const auto n0 = shfl16_down_key(k[0]);
-      const auto p2 = shfl16_up_key(k[2]);
-      if ((hl & 1) == p) {
-        const auto lo = O::kmin(k[0], k[1]), hi = O::kmax(k[0], k[1]);
-        k[0] = lo; k[1] = hi;
-        if (hl < 15) k[2] = O::kmin(k[2], n0);
-      } else {
-        const auto lo = O::kmin(k[1], k[2]), hi = O::kmax(k[1], k[2]);
-        k[1] = lo; k[2] = hi;
-        if (hl > 0) k[0] = O::kmax(k[0], p2);
-      }
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------

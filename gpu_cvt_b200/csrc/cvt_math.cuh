@@ -82,15 +82,14 @@ template <class T> __device__ __forceinline__ Frame<T> frame_from_normal(V3<T> n
 // --------------------------------------------------------------------------
 constexpr int kPcaSteps = 8;
 
-template <class T>
-__device__ __forceinline__ V3<T> pca_normal(const T* __restrict__ S, long site_base, int n_sites,
-                                            const uint32_t* __restrict__ row, int K, V3<T> si, V3<T> n0) {
+template <class T, class NB>
+__device__ __forceinline__ V3<T> pca_normal(const NB& nb, int K, V3<T> si, V3<T> n0) {
   T sx = 0, sy = 0, sz = 0, xx = 0, xy = 0, xz = 0, yy = 0, yz = 0, zz = 0;
   int m = 0;
   for (int t = 0; t < K; ++t) {
-    const uint32_t j = __ldg(row + t);
-    if (j >= (uint32_t)n_sites) continue;
-    const V3<T> d = sub3(ld3(S, site_base + (long)j), si);
+    const uint32_t j = nb.id(t);
+    if (!nb.valid(j)) continue;
+    const V3<T> d = sub3(nb.pos(j), si);
     sx = sx + d.x; sy = sy + d.y; sz = sz + d.z;
     xx = fmaT(d.x, d.x, xx); xy = fmaT(d.x, d.y, xy); xz = fmaT(d.x, d.z, xz);
     yy = fmaT(d.y, d.y, yy); yz = fmaT(d.y, d.z, yz); zz = fmaT(d.z, d.z, zz);

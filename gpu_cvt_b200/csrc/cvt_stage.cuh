@@ -189,7 +189,8 @@ __global__ void k_stage_frames_pca(const float* __restrict__ S, int n, const uin
   if (i >= n) return;
   int nn = knnV[(size_t)i * kproj];
   if (nn < 0) { st3(U, i, V3<float>{1, 0, 0}); st3(Vv, i, V3<float>{0, 1, 0}); return; }
-  const V3<float> nrm = pca_normal<float>(S, 0, n, knn + (size_t)i * K, K, ld3(S, i), ld3(N0, nn));
+  const V3<float> nrm = pca_normal<float>(RowNeighbours<float>{S, knn + (size_t)i * K, (uint32_t)n}, K, ld3(S, i),
+                                            ld3(N0, nn));
   Frame<float> fr = frame_from_normal(nrm);
   st3(U, i, fr.u);
   st3(Vv, i, fr.v);
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(BLOCK) k_stage_clip(const float* __restrict__ 
   V3<float> si = ld3(S, i);
   Frame<float> fr{ld3(U, i), ld3(Vv, i)};
   PolyRef<PP> cur = A, nxt = B;
-  int np = clip_cell<PROF>(S, 0, n, si, knn + (size_t)i * K, K, fr, R, cur, nxt, CAP, false);
+  int np = clip_cell<PROF>(RowNeighbours<float>{S, knn + (size_t)i * K, (uint32_t)n}, si, K, fr, R, cur, nxt, CAP, false);
   if (np < 0) {
     int k = atomicAdd(ovf, 1);
     ovf[1 + k] = i;
@@ -240,7 +241,8 @@ __global__ void __launch_bounds__(64) k_stage_clip_fallback(const float* __restr
     V3<float> si = ld3(S, i);
     Frame<float> fr{ld3(U, i), ld3(Vv, i)};
     PolyRef<PP> cur{buf[0], 1}, nxt{buf[1], 1};
-    int np = clip_cell<PROF>(S, 0, n, si, knn + (size_t)i * K, K, fr, R, cur, nxt, kFallbackCap, false);
+    int np = clip_cell<PROF>(RowNeighbours<float>{S, knn + (size_t)i * K, (uint32_t)n}, si, K, fr, R, cur, nxt, kFallbackCap,
+                             false);
     V2<PP> c2 = poly_centroid<PP>(cur, np, PROF == PROF_MIXED);
     V3<float> c;
     if (!(finiteT(c2.x) && finiteT(c2.y))) c = {NAN, NAN, NAN};
@@ -335,7 +337,11 @@ __global__ void k_stage_tiers(int mode, int n, int K, const float* __restrict__ 
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   auto normal = [&](int j, float out[3]) { out[0] = sn[3 * j]; out[1] = sn[3 * j + 1]; out[2] = sn[3 * j + 2]; };
-  tier[i] = (uint8_t)tier_of(mode, i, n, K, knn + (size_t)i * K, normal);
+  auto row = [&](int t) {
+    const int j = (int)knn[(size_t)i * K + t];
+    return j < n ? j : -1;
+  };
+  tier[i] = (uint8_t)tier_of(mode, i, K, row, normal);
 }
 
 }  // namespace cvt

@@ -1,0 +1,102 @@
+"""The engine stores a segment's sites in cell order and checks its neighbour
+lists with one thread per site; lists, ties and every result must be those of
+the caller's order, at block and warp edges, with exact distance ties (lattice
+sites, mirrored and repeated sites) and through removal and re-use of slots.
+The oracle works in the caller's order; everything is compared bit for bit."""
+import numpy as np
+import pytest
+
+from gpu_cvt_b200 import meshgen as mg
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def eng():
+    from gpu_cvt_b200 import engine
+    assert torch.cuda.is_available()
+    return engine
+
+
+def _run(eng, m, S0, k, mode, iters, profile, reuse):
+    mesh = eng.Mesh(m.V, m.F)
+    e = eng.Engine(eng.params(k=k, mode=mode, profile=profile, knn_reuse=reuse), 1, len(S0), eng.grid_cells(mesh, len(S0), k))
+    g = e.add(mesh, S0)
+    e.run(iters)
+    S = e.sites_f64(g) if profile == "fp64" else e.sites(g)
+    st = e.state(g)
+    reused = sum(e.stats(g, i)["knn_reused"] for i in range(iters))
+    e.close()
+    mesh.close()
+    return S, st, reused
+
+
+def _sites(kind):
+    if kind == "lattice":            # the reference's own start: the vertices, no noise, many equal distances
+        m = mg.torus(1.0, 0.3, 64, 32)
+        return m, m.V.copy()
+    if kind == "mirrored":           # mirrored exactly in every axis, shuffled
+        m = mg.icosphere(4)
+        S = mg.sample_sites(m.V, m.F, 120, seed=5)
+        S = np.concatenate([S * np.array(s, np.float32) for s in
+                            [(1, 1, 1), (-1, 1, 1), (1, -1, 1), (1, 1, -1), (-1, -1, 1), (1, -1, -1), (-1, 1, -1),
+                             (-1, -1, -1)]])
+        return m, np.ascontiguousarray(np.random.default_rng(0).permutation(S))
+    m = mg.icosphere(4)              # every site three times
+    S = mg.sample_sites(m.V, m.F, 230, seed=6)
+    return m, np.ascontiguousarray(np.random.default_rng(1).permutation(np.concatenate([S, S, S])))
+
+
+@pytest.mark.parametrize("kind", ["lattice", "mirrored", "repeated"])
+@pytest.mark.parametrize("k,mode,profile,reuse", [(24, 1, "mixed", True), (8, 0, "ref", True), (32, 2, "ref", True),
+                                                  (20, 1, "ref", False)])
+def test_equal_distances_keep_the_callers_order(eng, oracle, kind, k, mode, profile, reuse):
+    m, S0 = _sites(kind)
+    iters = 10
+    S, st, reused = _run(eng, m, S0, k, mode, iters, profile, reuse)
+    r = oracle.lloyd_run(m.V, m.F, S0, k, mode, iters, profile=oracle.PROFILES[profile])
+    assert np.array_equal(st["knn"], r["knn"])
+    assert np.array_equal(st["frozen"], r["frozen"])
+    assert np.array_equal(S, r["S"])
+    if reuse and kind == "lattice":
+        assert reused > 0            # the tied lists went through the check
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 63, 64, 65, 129, 257])
+@pytest.mark.parametrize("profile", ["mixed", "fp64"])
+def test_block_edges(eng, oracle, n, profile):
+    """Fewer sites than neighbours, one warp, one block and one more."""
+    m = mg.icosphere(3)
+    S0 = mg.sample_sites(m.V, m.F, n, seed=n)
+    S, st, _ = _run(eng, m, S0, 16, 0, 4, profile, True)
+    r = oracle.lloyd_run(m.V, m.F, S0, 16, 0, 4, profile=oracle.PROFILES[profile])
+    if n > 16:
+        assert np.array_equal(st["knn"], r["knn"])
+    assert np.array_equal(S, r["S"], equal_nan=True)
+
+
+def test_slots_used_again(eng, oracle):
+    """Segments of other sizes placed in slots that removed ones left, at both
+    buffer parities: each equals its own run."""
+    m = mg.torus(1.0, 0.3, 60, 30, noise_sigma=0.002, seed=1)
+    mesh = eng.Mesh(m.V, m.F)
+    sizes = [700, 1300, 450]
+    S = [mg.sample_sites(m.V, m.F, n, seed=n) for n in sizes]
+    cells = sum(eng.grid_cells(mesh, n, 12) for n in sizes)
+    e = eng.Engine(eng.params(k=12, mode=1, profile="ref"), 3, sum(sizes), cells)
+    a, b = e.add(mesh, S[0]), e.add(mesh, S[1])
+    e.run(3)
+    e.remove(a)
+    c = e.add(mesh, S[2])
+    e.run(2)
+    e.remove(b)
+    d = e.add(mesh, S[1])
+    e.run(4)
+    for g, s, it in ((c, 2, 6), (d, 1, 4)):
+        r = oracle.lloyd_run(m.V, m.F, S[s], 12, 1, it)
+        assert np.array_equal(e.sites(g), r["S"])
+        assert np.array_equal(e.state(g)["knn"], r["knn"])
+    e.close()
+    mesh.close()
