@@ -1109,6 +1109,8 @@ struct cvt_engine {
   std::vector<int> seg_p0;  // global parity when the segment was placed
   RangeAlloc site_alloc, cell_alloc;
   int parity = 0;
+  // slots and cells that the iteration's launches cover (cover_segments)
+  int cov_sites = 0, cov_cells = 0;
   // device: every array below is a slice of one allocation
   void* arena = nullptr;
   size_t bytes = 0;
@@ -1275,6 +1277,8 @@ extern "C" cvt_status_t cvt_engine_create(const cvt_params_t* p, int max_segment
   e->seg_cells.assign(max_segments, 0);
   e->host_iters.assign(max_segments, 0);
   e->seg_p0.assign(max_segments, 0);
+  e->cov_sites = max_sites;
+  e->cov_cells = max_cells;
   e->site_alloc.init(max_sites);
   e->cell_alloc.init(max_cells);
   const size_t tsz = e->f64 ? sizeof(double) : sizeof(float);
@@ -1501,7 +1505,7 @@ template <class T> static EngineArgs<T> engine_args(cvt_engine* e) {
   a.frozen = e->d_frozen; a.streak = e->d_streak; a.tier = e->d_tier;
   a.cell_start = e->d_cell_start; a.sorted = (const Pt4<T>*)e->d_sorted;
   a.stats = e->d_stats; a.ovf = e->d_ovf; a.far = e->d_far; a.cent = (T*)e->d_cent; a.K = e->K;
-  a.n_sites = e->max_sites;
+  a.n_sites = e->cov_sites;
   a.proj_mode = e->p.proj_mode; a.bvh_ovf = reinterpret_cast<int*>(e->d_tickets + 2);
   a.cand_rho = e->d_cand_rho; a.cand_D = e->d_cand_D; a.srch = e->d_srch; a.srch_thr = e->d_srch_thr;
   a.blockmax = e->d_blockmax;
@@ -1607,7 +1611,7 @@ static cvt_status_t enqueue_iteration_t(cvt_engine* e, int parity, cudaStream_t 
     CK(cudaEventRecord(br.fork, st));
     CK(cudaStreamWaitEvent(br.side, br.fork, 0));
   }
-  L += launch_exclusive_scan(e->max_cells, e->d_cell_count, e->d_part, e->d_cell_start, gs, true, e->d_tickets);
+  L += launch_exclusive_scan(e->cov_cells, e->d_cell_count, e->d_part, e->d_cell_start, gs, true, e->d_tickets);
   k_site_scatter<T><<<cdiv(ns, 256), 256, 0, gs>>>(a, parity, e->d_cellrank, (Pt4<T>*)e->d_sorted);
   L++;
   CK(cudaEventRecord(br.grid, gs));
@@ -1660,6 +1664,37 @@ static cvt_status_t enqueue_iteration(cvt_engine* e, int parity, cudaStream_t st
 static_assert(2 * kCellCap * 128 * sizeof(V2<float>) <= 48 * 1024 && 2 * kCellCap * 64 * sizeof(V2<double>) <= 48 * 1024,
               "clip buffers exceed the default dynamic shared memory limit");
 
+// Fit the launches to the occupied part of the engine.  A serving engine has
+// room for millions of sites and cells (4 GiB: 15M and 62M) of which a request
+// mix fills a few per cent, and a scan of every empty cell plus a block for
+// every empty slot cost it more than the sites did (16 requests of 2k-200k
+// sites: 0.48 of 1.6 ms per iteration).  The first-fit allocators keep
+// segments at low addresses.  Power-of-two extents, shrunk only to a quarter,
+// so that arrivals and departures seldom change them; a change drops the
+// captured graphs, and the next capture updates a kept one (graph_exec_for).
+static cvt_status_t cover_segments(cvt_engine* e, cudaStream_t st) {
+  int ns = 1, nc = 2;
+  for (int k = 0; k < e->max_seg; ++k)
+    if (e->seg_mesh[k]) {
+      ns = std::max(ns, e->segs[k].site_base + e->segs[k].n_sites);
+      nc = std::max(nc, e->geom[k].cell_base + e->seg_cells[k]);
+    }
+  auto fit = [](int need, int cur, int cap) {
+    if (need <= cur && (long)need * 4 > cur) return cur;
+    long p = 1024;
+    while (p < need) p <<= 1;
+    return (int)std::min<long>(p, cap);
+  };
+  const int cs = fit(ns, e->cov_sites, e->max_sites), cc = fit(nc, e->cov_cells, e->max_cells);
+  if (cs == e->cov_sites && cc == e->cov_cells) return CVT_OK;
+  e->cov_sites = cs;
+  e->cov_cells = cc;
+  if (e->gexec[0] || e->gexec[1]) CK(cudaStreamSynchronize(st));  // no replay in flight
+  for (int k = 0; k < 2; ++k)
+    if (e->gexec[k]) { graph_cache_put(graph_key(e), e->gexec[k]); e->gexec[k] = nullptr; }
+  return CVT_OK;
+}
+
 extern "C" cvt_status_t cvt_engine_run(cvt_engine_t e, int iters, void* stream) {
   if (!e || iters < 0) return fail(CVT_ERR_INVALID, "cvt_engine_run: bad arguments");
   cudaStream_t st = S_(stream);
@@ -1669,6 +1704,8 @@ extern "C" cvt_status_t cvt_engine_run(cvt_engine_t e, int iters, void* stream) 
   if (iters > 0) CK(thread_streams(&ts));
   const Branch eager{ts ? ts->side : nullptr, e->ev_fork, e->ev_grid, e->ev_join};
   e->last_launches = 0;
+  s = cover_segments(e, st);
+  if (s != CVT_OK) return s;
   for (int it = 0; it < iters; ++it) {
     const int par = e->parity;
     const bool capture = e->p.use_graph && !e->gexec[par];
@@ -1711,6 +1748,8 @@ extern "C" cvt_status_t cvt_engine_profile(cvt_engine_t e, int iters, float* ms,
   cvt_status_t s = CVT_OK;
   ThreadStreams* ts = nullptr;
   CK(thread_streams(&ts));
+  s = cover_segments(e, st);
+  if (s != CVT_OK) return s;
   cudaEvent_t ev[6];
   for (int k = 0; k < 6; ++k) CK(cudaEventCreate(&ev[k]));
   double acc[5] = {0, 0, 0, 0, 0};

@@ -100,3 +100,28 @@ def test_slots_used_again(eng, oracle):
         assert np.array_equal(e.state(g)["knn"], r["knn"])
     e.close()
     mesh.close()
+
+
+def test_launches_follow_the_occupied_slots(eng, oracle):
+    """A large engine whose launches cover only the occupied slots: segments
+    that arrive beyond the covered part, and departures that shrink it, leave
+    every result as it is alone (graph replays on both sides of a change)."""
+    m = mg.icosphere(4)
+    mesh = eng.Mesh(m.V, m.F)
+    e = eng.Engine(eng.params(k=12, mode=0, profile="ref"), 8, 2_000_000, 8_000_000)
+    S = {n: mg.sample_sites(m.V, m.F, n, seed=n) for n in (300, 1024, 5000, 70)}
+    done = {}
+    for n in (300, 1024, 5000):      # 300 -> 1324 -> 6324 slots
+        done[n] = [e.add(mesh, S[n]), 0]
+        e.run(5)
+        for v in done.values():
+            v[1] += 5
+    for n in (300, 1024, 5000):
+        assert np.array_equal(e.sites(done[n][0]), oracle.lloyd_run(m.V, m.F, S[n], 12, 0, done[n][1])["S"])
+    for n in (300, 1024, 5000):
+        e.remove(done[n][0])
+    g = e.add(mesh, S[70])           # back to the smallest extent
+    e.run(6)
+    assert np.array_equal(e.sites(g), oracle.lloyd_run(m.V, m.F, S[70], 12, 0, 6)["S"])
+    e.close()
+    mesh.close()
