@@ -366,12 +366,7 @@ static cvt_status_t clip_dispatch(const float* S, const float* U, const float* V
   int* ovf;
   CK(sc.get(&ovf, (size_t)n + 1));
   CK(cudaMemsetAsync(ovf, 0, sizeof(int), st));
-  const size_t smem = 2 * kClipCap * kClipBlock * sizeof(V2<float>);
-  static bool attr = false;
-  if (!attr) {
-    CK(cudaFuncSetAttribute(k_stage_clip<PROF, kClipBlock, kClipCap>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr = true;
-  }
+  const size_t smem = kClipCap * kClipBlock * sizeof(V2<float>);
   k_stage_clip<PROF, kClipBlock, kClipCap><<<cdiv(n, kClipBlock), kClipBlock, smem, st>>>(S, U, V, knn, n, K, R, cent, nverts, ovf);
   CKLAUNCH();
   k_stage_clip_fallback<PROF><<<sm_count(), 64, 0, st>>>(S, U, V, knn, n, K, R, cent, nverts, ovf);
@@ -452,7 +447,7 @@ struct cvt_mesh {
   GridGeom vg{};
   int* dvcell_start = nullptr;
   Pt4<float>* dvsorted = nullptr;
-  float4* dring = nullptr;    // one-ring records (kRingWords per CSR entry)
+  float4 *dring_head = nullptr, *dring_body = nullptr;  // one-ring records (1 + kRingBody words per CSR entry)
   float* dunref = nullptr;    // input vertices no face uses (Hausdorff probes only)
   int n_unref = 0;
   BVHNode* dnodes = nullptr;  // built on first use (Hausdorff)
@@ -465,7 +460,7 @@ struct cvt_mesh {
   MeshDev dev() const {
     MeshDev m;
     m.V = dV; m.F = dF; m.vf_off = doff; m.vf_faces = dfcs; m.N = dN;
-    m.vcell_start = dvcell_start; m.vsorted = dvsorted; m.ring = dring; m.vg = vg;
+    m.vcell_start = dvcell_start; m.vsorted = dvsorted; m.ring_head = dring_head; m.ring_body = dring_body; m.vg = vg;
     m.bvh = dnodes; m.bvh_tri = dtri;
     m.nV = nV; m.nF = nF; m.R = R;
     m.thr2 = ((0.01f * R) * 0.01f) * R;
@@ -739,7 +734,8 @@ static cvt_status_t mesh_create_on(const float* V, int nV, const int* F, int nF,
   ar.add(&m->doff, (size_t)nn + 1);
   ar.add(&m->dfcs, (size_t)n3);
   ar.add(&m->dN, 3 * (size_t)nn);
-  ar.add(&m->dring, (size_t)kRingWords * 3 * nF);
+  ar.add(&m->dring_head, (size_t)n3);
+  ar.add(&m->dring_body, (size_t)kRingBody * n3);
   ar.add(&m->dunref, 3 * (size_t)m->n_unref);
   // the vertex grid's cell array is sized after the area is known
   MCK(ar.commit(&m->arena));
@@ -786,7 +782,7 @@ static cvt_status_t mesh_create_on(const float* V, int nV, const int* F, int nF,
   k_stage_normals<<<cdiv(nn, 256), 256, 0, st>>>(m->dV, nn, m->dF, m->doff, m->dfcs, m->dN);
   LAUNCHED(1);
   MCK(cudaGetLastError());
-  k_build_ring_records<<<cdiv(n3, 256), 256, 0, st>>>(m->dV, m->dF, nF, m->dfcs, n3, m->dring);
+  k_build_ring_records<<<cdiv(n3, 256), 256, 0, st>>>(m->dV, m->dF, nF, m->dfcs, n3, m->dring_head, m->dring_body);
   LAUNCHED(1);
   MCK(cudaGetLastError());
   {
@@ -1548,7 +1544,7 @@ template <int PROF, int FRAME>
 static void launch_site_clip_f(const EngineArgs<typename PT<PROF>::T>& a, int parity, int ns, int bs, int nsm,
                                cudaStream_t st) {
   using PP = typename PT<PROF>::PP;
-  const size_t smem = 2 * kCellCap * (size_t)bs * sizeof(V2<PP>);
+  const size_t smem = kCellCap * (size_t)bs * sizeof(V2<PP>);
   if (sizeof(PP) == 8) {
     if (bs == 32) k_site_clip<PROF, 32, kCellCap, FRAME><<<cdiv(ns, 32), 32, smem, st>>>(a, parity);
     else k_site_clip<PROF, 64, kCellCap, FRAME><<<cdiv(ns, 64), 64, smem, st>>>(a, parity);
@@ -1658,10 +1654,10 @@ static cvt_status_t enqueue_iteration(cvt_engine* e, int parity, cudaStream_t st
   }
 }
 
-// k_site_clip's dynamic shared memory (two 16-vertex polygon buffers per
-// thread) is at most 32 KB per block for every launch shape, within the
-// default 48 KB limit, so no function attribute is needed.
-static_assert(2 * kCellCap * 128 * sizeof(V2<float>) <= 48 * 1024 && 2 * kCellCap * 64 * sizeof(V2<double>) <= 48 * 1024,
+// The clip kernels' dynamic shared memory (one polygon buffer per thread) is
+// within the default 48 KB limit, so no function attribute is needed.
+static_assert(kCellCap * 128 * sizeof(V2<float>) <= 48 * 1024 && kCellCap * 64 * sizeof(V2<double>) <= 48 * 1024 &&
+                  kClipCap * kClipBlock * sizeof(V2<float>) <= 48 * 1024,
               "clip buffers exceed the default dynamic shared memory limit");
 
 // Fit the launches to the occupied part of the engine.  A serving engine has

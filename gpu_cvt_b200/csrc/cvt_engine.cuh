@@ -60,10 +60,11 @@ constexpr int kKProj = 5;         // KPROJ (main.cu:394)
 // leaves the site to the ring search: ring 1's 27 cells.
 constexpr int kVertexBoxCells = 27;
 constexpr int kFallbackCap = 66;  // 64-vertex reference cap + room for the overshoot
-// threads per SM that k_site_clip's launch bounds ask to keep resident: it
-// caps registers near 80 (6 blocks of 128 with 32 KB of polygon buffers each
-// for FP32 polygons, 6 of 64 for FP64 ones) whatever the block size
-constexpr int kClipThreadsF = 768;
+// threads per SM that k_site_clip's launch bounds ask to keep resident,
+// whatever the block size (polygon buffers: 16 KB per block): 64 registers
+// for FP32 polygons (1024 threads; mixed, 300k sites: 57.7 us, 65.5 with 768
+// and 80 registers, 66.3 with 896)
+constexpr int kClipThreadsF = 1024;
 constexpr int kClipThreadsD = 384;
 
 struct MeshDev {
@@ -74,7 +75,8 @@ struct MeshDev {
   const float* N;
   const int* vcell_start;
   const Pt4<float>* vsorted;
-  const float4* ring;  // one-ring records, kRingWords per CSR entry (k_build_ring_records)
+  const float4* ring_head;  // one-ring records, one head and kRingBody body words per CSR entry
+  const float4* ring_body;  // (k_build_ring_records)
   const BVHNode* bvh;  // BVH over the faces (built before a segment that projects through it is placed)
   const int* bvh_tri;
   GridGeom vg;
@@ -256,8 +258,8 @@ template <class T> struct ListNeighbours {  // the engine's lists
   __device__ __forceinline__ V3<T> pos(uint32_t j) const { return ldp(S, j); }
 };
 
-// Clip the square [-R,R]^2 by the bisectors of the listed neighbours; returns
-// the vertex count (polygon in `cur` on return) or -1 on buffer overflow.
+// clip_cell in full generality: every clip copies the polygon from one buffer
+// to the other.  Run for the cells that clip_cell gives back.
 //
 // Security radius: a bisector whose half-plane contains the disk around the
 // site that holds the current polygon cannot cut it and is skipped
@@ -270,7 +272,7 @@ template <class T> struct ListNeighbours {  // the engine's lists
 // that would return their input unchanged: the result is the same bit for
 // bit as clipping by all K bisectors.
 template <int PROF, class NB>
-__device__ __forceinline__ int clip_cell(const NB& nb, V3<typename PT<PROF>::T> si, int K,
+__device__ __forceinline__ int clip_cell_full(const NB& nb, V3<typename PT<PROF>::T> si, int K,
                                          const Frame<typename PT<PROF>::T>& fr, float R,
                                          PolyRef<typename PT<PROF>::PP>& cur, PolyRef<typename PT<PROF>::PP>& nxt,
                                          int cap, bool row_sorted) {
@@ -315,6 +317,146 @@ __device__ __forceinline__ int clip_cell(const NB& nb, V3<typename PT<PROF>::T> 
     if (ovf) { n = -1; done = true; continue; }
     PolyRef<PP> tmp = cur; cur = nxt; nxt = tmp;
     if (n == 0) done = true;
+  }
+  return n;
+}
+
+// Clip the square [-R,R]^2 by the bisectors of the listed neighbours in one
+// buffer; returns the vertex count (polygon in P) or -1 when the cell has to
+// be redone by clip_cell_full: more than `cap` vertices, a clip whose outside
+// vertices are not one cyclic run, or a vertex that is not finite.  The
+// polygon is the one clip_cell_full computes, bit for bit.
+//
+// A clip first finds the outside vertices as a bit mask.  None: the polygon is
+// unchanged and nothing is written.  One run p..q (the only case for a convex
+// polygon): Sutherland-Hodgman keeps the others and puts one intersection
+// before and one after them, so two vertices are computed and the rest moves
+// by 2 - (run length) slots; the three orders below are those in which its
+// loop from vertex 0 emits them.  In the MIXED profile the mask is found in
+// FP32 where that decides the FP64 predicate: the FP32 value errs by less than
+// 9 u |d| r + 8 u c (u = 2^-24: difference, frame dots, half square and two
+// fma), and 2e-6 (|d| r + c) is left to the FP64 predicate itself; FP64
+// coefficients are only computed for those vertices and for real cuts.
+// Neighbours with |d|^2 > 4 r^2 (margin 2.5e-3) cannot cut whatever the frame
+// (its vectors have unit length to 1e-6): skipped, and on this iteration's
+// sorted list they end the loop (see clip_cell_full).
+//
+// Bound by issue (63 %) and latency; 24 of 32 threads active.  Clip kernel,
+// mixed, 300k sites, K = 24: 57 us and 117 warp instructions per site, against
+// 102 us and 187 with two buffers and every vertex clipped in FP64 (15 of 32
+// active, conversions 42 % of their pipe).
+template <int PROF, class NB>
+__device__ __forceinline__ int clip_cell(const NB& nb, V3<typename PT<PROF>::T> si, int K,
+                                         const Frame<typename PT<PROF>::T>& fr, float R,
+                                         const PolyRef<typename PT<PROF>::PP>& P, int cap, bool row_sorted) {
+  using T = typename PT<PROF>::T;
+  using Q = typename PT<PROF>::Q;
+  using PP = typename PT<PROF>::PP;
+  constexpr bool kFilter = PROF == PROF_MIXED;
+  const PP r = (PP)R;
+  P.set(0, {-r, -r}); P.set(1, {r, -r}); P.set(2, {r, r}); P.set(3, {-r, r});
+  int n = 4;
+  float r2 = 2.f * R * R * 1.0001f;
+  // the next neighbour's position is loaded while the current one clips
+  uint32_t jn = nb.id(0);
+  V3<T> sn = nb.valid(jn) ? nb.pos(jn) : si;
+  // every lane runs all K trips; see clip_cell_full
+  bool done = false;
+  for (int t = 0; t < K; ++t) {
+    if (done) continue;
+    const uint32_t j = jn;
+    const V3<T> sj = sn;
+    if (t + 1 < K) {
+      jn = nb.id(t + 1);
+      if (nb.valid(jn)) sn = nb.pos(jn);
+    }
+    if (!nb.valid(j)) continue;
+    const V3<T> d = sub3(sj, si);
+    const V3<float> df = cvt3<float>(d);
+    const float dd = dot3(df, df);
+    if (dd > 4.01f * r2 && dd > 2e-18f && dd < 1e30f) {
+      done = row_sorted;
+      continue;
+    }
+    // the half-plane a x + b y - c <= eps as the predicate computes it
+    const Q eps = (Q)1e-12;
+    Q a, b, c;
+    auto exact_plane = [&]() {
+      if (kFilter) {
+        V3<double> e{(double)sj.x - (double)si.x, (double)sj.y - (double)si.y, (double)sj.z - (double)si.z};
+        a = (Q)dot3(e, cvt3<double>(fr.u)); b = (Q)dot3(e, cvt3<double>(fr.v)); c = (Q)(0.5 * dot3(e, e));
+      } else {
+        a = (Q)dot3(d, fr.u); b = (Q)dot3(d, fr.v); c = (Q)((T)0.5 * dot3(d, d));
+      }
+    };
+    auto f = [&](V2<PP> v) -> Q { return fmaT(a, (Q)v.x, fmaT(b, (Q)v.y, -c)); };
+    unsigned out = 0u;
+    float rin = 0.f;
+    if (kFilter) {
+      const float af = (float)dot3(d, fr.u), bf = (float)dot3(d, fr.v), cf = 0.5f * dd;
+      float root;
+      asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"(dd * r2));
+      const float tol = 2e-6f * (root + cf) + 2e-12f;
+      unsigned unsure = 0u;
+      for (int i = 0; i < n; ++i) {
+        const V2<PP> v = P.get(i);
+        const float x = (float)v.x, y = (float)v.y;
+        const float g = fmaT(af, x, fmaT(bf, y, -cf));
+        if (!(g < -tol)) { if (g > tol) out |= 1u << i; else unsure |= 1u << i; }
+        else rin = fmaxf(rin, fmaT(y, y, x * x));
+      }
+      if (unsure) {
+        exact_plane();
+        while (unsure) {
+          const int i = __ffs(unsure) - 1;
+          unsure &= unsure - 1;
+          const V2<PP> v = P.get(i);
+          const float x = (float)v.x, y = (float)v.y;
+          if (f(v) <= eps) rin = fmaxf(rin, fmaT(y, y, x * x)); else out |= 1u << i;
+        }
+      }
+    } else {
+      exact_plane();
+      for (int i = 0; i < n; ++i) {
+        const V2<PP> v = P.get(i);
+        if (f(v) <= eps) rin = fmaxf(rin, f32_ru(fmaT(v.y, v.y, v.x * v.x))); else out |= 1u << i;
+      }
+    }
+    if (out == 0u) continue;
+    const unsigned all = 0xffffffffu >> (32 - n);
+    if (out == all) { n = 0; done = true; continue; }
+    const unsigned starts = out & ~((out << 1) | (out >> (n - 1)));  // outside, the vertex before it inside
+    const int len = __popc(out), p = __ffs(starts) - 1;
+    if ((starts & (starts - 1)) || n - len + 2 > cap) { n = -1; done = true; continue; }
+    const int q = p + len - 1 >= n ? p + len - 1 - n : p + len - 1;
+    const int ip = p == 0 ? n - 1 : p - 1, iq = q + 1 == n ? 0 : q + 1;
+    if (kFilter) exact_plane();
+    auto isect = [&](V2<PP> s, V2<PP> e) -> V2<PP> {
+      const Q fs = f(s), fe = f(e);
+      const Q u = divT(fs, (fs - fe) + (Q)1e-30);
+      return {(PP)fmaT(u, (Q)e.x - (Q)s.x, (Q)s.x), (PP)fmaT(u, (Q)e.y - (Q)s.y, (Q)s.y)};
+    };
+    const V2<PP> enter = isect(P.get(ip), P.get(p));  // before the run
+    const V2<PP> leave = isect(P.get(q), P.get(iq));  // after it
+    // kept vertices [lo, hi) move by `shift`
+    int lo, hi, shift, at_enter, at_leave;
+    if (p <= q && q + 1 < n) {  // v0 .. v(p-1), enter, leave, v(q+1) .. v(n-1)
+      lo = q + 1; hi = n; shift = 2 - len; at_enter = p; at_leave = p + 1;
+    } else {                    // leave, v(q+1) .. v(p-1), enter
+      lo = iq; hi = p; shift = 1 - iq; at_enter = n - len + 1; at_leave = 0;
+    }
+    if (shift > 0) {
+      for (int i = hi - 1; i >= lo; --i) P.set(i + shift, P.get(i));
+    } else if (shift < 0) {
+      for (int i = lo; i < hi; ++i) P.set(i + shift, P.get(i));
+    }
+    P.set(at_enter, enter);
+    P.set(at_leave, leave);
+    n += 2 - len;
+    auto rad2 = [&](V2<PP> v) { return f32_ru(fmaT(v.y, v.y, v.x * v.x)); };
+    const float re = rad2(enter), rl = rad2(leave);
+    r2 = fmaxf(rin, fmaxf(re, rl)) * 1.000001f;
+    if (!(re < INFINITY) || !(rl < INFINITY)) { n = -1; done = true; }
   }
   return n;
 }
@@ -871,9 +1013,10 @@ struct SiteOut {
   float disp2;
 };
 
-// Frame, clip and centroid of site g into a.cent; false when the polygon
-// outgrew the buffers (the site is then redone by k_clip_overflow).
-template <int PROF, int FRAME>
+// Frame, clip and centroid of site g into a.cent; false when clip_cell gave
+// the cell back (the site is then redone by k_clip_overflow: FULL, with a
+// second buffer B).
+template <int PROF, int FRAME, bool FULL>
 __device__ __forceinline__ bool site_clip(const EngineArgs<typename PT<PROF>::T>& a, int parity, int g,
                                           PolyRef<typename PT<PROF>::PP> A, PolyRef<typename PT<PROF>::PP> B,
                                           int cap) {
@@ -899,7 +1042,8 @@ __device__ __forceinline__ bool site_clip(const EngineArgs<typename PT<PROF>::T>
     fr = frame_from_normal(n0);
   }
   PolyRef<PP> cur = A, nxt = B;
-  const int np = clip_cell<PROF>(nb, si, a.K, fr, md.R, cur, nxt, cap, !fz);
+  const int np = FULL ? clip_cell_full<PROF>(nb, si, a.K, fr, md.R, cur, nxt, cap, !fz)
+                      : clip_cell<PROF>(nb, si, a.K, fr, md.R, A, cap, !fz);
   if (np < 0) return false;
   const V2<PP> c2 = poly_centroid<PP>(cur, np, PROF == PROF_MIXED);
   V3<T> cent;
@@ -920,10 +1064,10 @@ __global__ void __launch_bounds__(BLOCK, (sizeof(typename PT<PROF>::PP) == 8 ? k
   using PP = typename PT<PROF>::PP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V2<PP>* sm = reinterpret_cast<V2<PP>*>(smem_raw);
-  PolyRef<PP> A{sm + threadIdx.x, BLOCK}, B{sm + CAP * BLOCK + threadIdx.x, BLOCK};
+  const PolyRef<PP> A{sm + threadIdx.x, BLOCK};
   const int g = blockIdx.x * BLOCK + threadIdx.x;
   if (active_seg(a, g) >= 0) {
-    if (!site_clip<PROF, FRAME>(a, parity, g, A, B, CAP)) {
+    if (!site_clip<PROF, FRAME, false>(a, parity, g, A, A, CAP)) {
       const int k = atomicAdd(a.ovf, 1);
       a.ovf[1 + k] = g;
     }
@@ -936,16 +1080,17 @@ __global__ void __launch_bounds__(64) k_clip_overflow(EngineArgs<typename PT<PRO
   V2<PP> buf[2][kFallbackCap];
   const int n = *(volatile int*)a.ovf;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    site_clip<PROF, FRAME>(a, parity, a.ovf[1 + k], PolyRef<PP>{buf[0], 1}, PolyRef<PP>{buf[1], 1}, kFallbackCap);
+    site_clip<PROF, FRAME, true>(a, parity, a.ovf[1 + k], PolyRef<PP>{buf[0], 1}, PolyRef<PP>{buf[1], 1}, kFallbackCap);
 }
 
 // Projection, tiers and the freeze test of site g, given the centroid in
 // a.cent and (PROJ 0) its 5 nearest vertices knnv; PROJ 1 projects through
 // the mesh's BVH and ignores knnv.
-template <int PROF, int PROJ>
+template <int PROF, int PROJ, int BS>
 __device__ __forceinline__ void site_finish(const EngineArgs<typename PT<PROF>::T>& a, int parity, int g,
-                                            const int (&knnv)[kKProj], SiteOut& o) {
+                                            const int (&knnv)[kKProj], RingList<BS>& L, SiteOut& o) {
   using T = typename PT<PROF>::T;
+  using Q = typename PT<PROF>::Q;
   const int s = __ldg(a.site_seg + g);
   const SegDev& sd = a.segs[s];
   const MeshDev& md = a.meshes[sd.mesh];
@@ -959,12 +1104,9 @@ __device__ __forceinline__ void site_finish(const EngineArgs<typename PT<PROF>::
   if (PROF == PROF_MIXED && !finite3(cent)) {
     sn = si;
   } else if (PROJ == 1) {
-    using Q = typename PT<PROF>::Q;
     sn = project_bvh<T, Q>(cent, md.bvh, md.bvh_tri, md.V, md.F, (Q)bvh_bound2(cent, si), a.bvh_ovf);
-  } else if (PROF == PROF_REF) {
-    sn = project_onering_rec<T, float>(cent, md.ring, md.nV, md.vf_off, knnv, kKProj);
-  } else {
-    sn = project_onering_rec<T, double>(cent, md.ring, md.nV, md.vf_off, knnv, kKProj);
+  } else if (!project_onering_rec<T, Q, BS>(cent, md.ring_head, md.ring_body, md.nV, md.vf_off, knnv, L, sn)) {
+    sn = project_onering_plain<T, Q>(cent, md.V, md.nV, md.F, md.nF, md.vf_off, md.vf_faces, knnv, kKProj);
   }
   a.S[parity ^ 1][g] = Pt4<T>{sn.x, sn.y, sn.z, me.id};
 
@@ -1074,18 +1216,19 @@ __global__ void __launch_bounds__(BS, PROF == PROF_FP64 ? 1 : 1536 / BS) k_site_
 // Everything after the centroid and (PROJ 0) the vertex search of
 // k_site_vsearch; false when that search was deferred (the site is then
 // listed in a.far and finished by k_site_far).
-template <int PROF, int PROJ>
-__device__ __forceinline__ bool site_proj(const EngineArgs<typename PT<PROF>::T>& a, int parity, int g, SiteOut& o) {
+template <int PROF, int PROJ, int BS>
+__device__ __forceinline__ bool site_proj(const EngineArgs<typename PT<PROF>::T>& a, int parity, int g, RingList<BS>& L,
+                                          SiteOut& o) {
   if (PROJ == 1) {
     const int none[kKProj] = {-1, -1, -1, -1, -1};
-    site_finish<PROF, 1>(a, parity, g, none, o);
+    site_finish<PROF, 1>(a, parity, g, none, L, o);
     return true;
   }
   int knnv[kKProj];
 #pragma unroll
   for (int k = 0; k < kKProj; ++k) knnv[k] = a.knnv[k * a.stride + g];
   if (knnv[0] == kVertexDeferred) return false;
-  site_finish<PROF, 0>(a, parity, g, knnv, o);
+  site_finish<PROF, 0>(a, parity, g, knnv, L, o);
   return true;
 }
 
@@ -1174,17 +1317,18 @@ __device__ __forceinline__ void motion_to_block(const EngineArgs<T>& a, int pari
     atomicMax(a.blockmax + blk, ((unsigned long long)stamp << 32) | mb);
 }
 
-// One-ring projection: 24 resident warps per SM (80 registers), the
-// fastest budget of a register sweep (64 or 51: spills; 96 or 128: too few
-// warps).  The BVH projection keeps the compiler's choice.
+// One-ring projection: 24 resident warps per SM (80 registers); with 32 (64
+// registers, spills) it takes the same time.  The BVH projection keeps the
+// compiler's choice.
 template <int PROF, int BS, int PROJ>
 __global__ void __launch_bounds__(BS, PROJ == 0 ? 768 / BS : 1) k_site_proj(EngineArgs<typename PT<PROF>::T> a, int parity) {
   __shared__ StatsStage stage;
+  __shared__ RingList<PROJ == 0 ? BS : 1> rings;
   stats_stage_init(stage);
   __syncthreads();
   const int g = blockIdx.x * BS + threadIdx.x;
   SiteOut o{-1, 0, 0, 0, 0, 0.f};
-  if (active_seg(a, g) >= 0) site_proj<PROF, PROJ>(a, parity, g, o);
+  if (active_seg(a, g) >= 0) site_proj<PROF, PROJ>(a, parity, g, rings, o);
   if (a.blockmax) motion_to_block(a, parity, g, o);
   stats_flush(a.stats, a.segs, o, stage);
   __syncthreads();
@@ -1231,6 +1375,7 @@ __global__ void __launch_bounds__(128) k_site_far(EngineArgs<typename PT<PROF>::
   using T = typename PT<PROF>::T;
   using Key = typename KeyOps<T>::Key;
   __shared__ Key keys[128 * kKProj];
+  __shared__ RingList<1> rings;  // thread 0's
   __shared__ bool last;
   const int n = *(volatile int*)a.far;
   for (int k = blockIdx.x; k < n; k += gridDim.x) {
@@ -1260,7 +1405,7 @@ __global__ void __launch_bounds__(128) k_site_far(EngineArgs<typename PT<PROF>::
         a.knnv[j * a.stride + g] = knnv[j];
       }
       SiteOut o{-1, 0, 0, 0, 0, 0.f};
-      site_finish<PROF, 0>(a, parity, g, knnv, o);
+      site_finish<PROF, 0>(a, parity, g, knnv, rings, o);
       stats_atomic(a.stats, a.segs, o);
       if (a.blockmax) {
         int bx, by, bz;

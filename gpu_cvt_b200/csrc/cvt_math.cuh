@@ -250,24 +250,24 @@ __device__ __forceinline__ V3<T> project_onering(V3<T> c, const float* __restric
 }
 
 // One-ring records: for every vertex->face CSR entry (same order as the CSR),
-// the face's three corner positions and vertex ids and a bounding sphere in
-// four 16-byte words,
-//   r0 = {A.x, A.y, A.z, B.x}, r1 = {B.y, B.z, C.x, C.y}, r2 = {C.z, ia, ib, ic},
-//   r3 = {centre.x, centre.y, centre.z, radius}
-// (ids as int bits), so a projection reads one offset and then independent
-// 16-byte loads instead of the chain CSR entry -> face -> corners: r2 and r3
-// for every entry, r0 and r1 only for the faces that the shared-vertex and
-// sphere tests keep (2 % faster than loading all four up front).  The
-// sphere is centred on the float-rounded centroid; its radius is the largest
-// corner distance, computed in double and rounded up, so it holds the whole
+// a head and a body.  The head is the face's bounding sphere {centre, radius}
+// (16 bytes, a ring of six is 96 contiguous bytes); the body is the face's
+// three corner positions and vertex ids,
+//   r0 = {A.x, A.y, A.z, B.x}, r1 = {B.y, B.z, C.x, C.y}, r2 = {C.z, ia, ib, ic}
+// (ids as int bits).  A projection reads one offset and then the heads of the
+// ring, and the body only of the faces that the sphere test keeps (about a
+// third), instead of the chain CSR entry -> face -> corners.  The sphere is
+// centred on the float-rounded centroid; its radius is the largest corner
+// distance, computed in double and rounded up, so it holds the whole
 // triangle.  radius < 0 marks a face the projection never skips: an invalid
 // entry, or a triangle with a corner angle below ~5.7 degrees
 // (sin^2 < kPruneSin2), whose face-region formula is ill-conditioned.
-constexpr int kRingWords = 4;
+constexpr int kRingBody = 3;  // 16-byte words of a body
 constexpr double kPruneSin2 = 0.01;
 
 __global__ void k_build_ring_records(const float* __restrict__ V, const int* __restrict__ F, int nF,
-                                     const int* __restrict__ fcs, long n_entries, float4* __restrict__ rec) {
+                                     const int* __restrict__ fcs, long n_entries, float4* __restrict__ head,
+                                     float4* __restrict__ body) {
   const long ii = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (ii >= n_entries) return;
   const int fi = fcs[ii];
@@ -298,70 +298,160 @@ __global__ void k_build_ring_records(const float* __restrict__ V, const int* __r
     const float rad = __double2float_ru(sqrt(r2) * (1.0 + 1e-9));
     if (ok && isfinite(rad)) sph = make_float4(m[0], m[1], m[2], rad);
   }
-  rec[kRingWords * ii] = make_float4(a[0], a[1], a[2], b[0]);
-  rec[kRingWords * ii + 1] = make_float4(b[1], b[2], c[0], c[1]);
-  rec[kRingWords * ii + 2] = make_float4(c[2], __int_as_float(ia), __int_as_float(ib), __int_as_float(ic));
-  rec[kRingWords * ii + 3] = sph;
+  body[kRingBody * ii] = make_float4(a[0], a[1], a[2], b[0]);
+  body[kRingBody * ii + 1] = make_float4(b[1], b[2], c[0], c[1]);
+  body[kRingBody * ii + 2] = make_float4(c[2], __int_as_float(ia), __int_as_float(ib), __int_as_float(ic));
+  head[ii] = sph;
 }
 
-// project_onering over the one-ring records: the same faces in the same
-// order, the same arithmetic, so the same result bit for bit.
+// project_onering over the one-ring records, for the five nearest vertices:
+// the same result bit for bit, from the few faces that can hold it.
 //
-// A face whose bounding sphere lies so far from c that its computed d2 must
-// be >= the best so far cannot pass the strict '<' and is skipped, which
-// leaves the result unchanged.  The lower bound on the distance from c to
-// any point the closest-point code can return for the face,
-//   lb = |c - centre| - radius - 0.05 (|c - centre| + radius)
-//        - 1e-4 max|coordinate| - 1e-4 |c - centre|^2 / radius,
-// subtracts margins far above the rounding involved: the vertex and edge
-// results lie on the triangle up to the rounding of one fma per coordinate
-// (edge parameters are in [0, 1] under correct rounding); the face-region
-// result errs by about kappa u |AP|^2 / |edge| for kappa = 1/sin^2 <= 100
-// (the corner-angle flag), unit roundoff u <= 2^-24 and |AP| <= |c - centre|
-// + radius; |c - centre| is computed in FP32 from coordinates of magnitude
-// <= max|coordinate|; and the computed d2 is >= (1 - 5u) |p - c|^2.  A face is
-// skipped when lb > 0 and lb^2 > 1.001 best.
+// Whatever the closest-point code returns for a face lies at a distance from
+// c between lb and ub,
+//   lb = |c - centre| - radius - E,  ub = |c - centre| + E,
+//   E  = 0.05 (|c - centre| + radius) + 1e-4 max|coordinate|
+//        + 1e-4 |c - centre|^2 / radius
+// (the centre is the face's centroid up to rounding).  E is far above the
+// rounding involved: the vertex and edge results lie on the triangle up to
+// the rounding of one fma per coordinate (edge parameters are in [0, 1]
+// under correct rounding); the face-region result errs by about
+// kappa u |AP|^2 / |edge| for kappa = 1/sin^2 <= 100 (the corner-angle flag),
+// unit roundoff u <= 2^-24 and |AP| <= |c - centre| + radius; |c - centre| is
+// computed in FP32 from coordinates of magnitude <= max|coordinate|; and the
+// computed d2 is within 5u of |p - c|^2.  For |c - centre| <= 50 radius, with
+// max|coordinate| <= max|c| + |c - centre|, these become
+//   lb >= 0.9449 dc - 1.05 radius - 1e-4 max|c|
+//   ub <= 1.0552 dc + 0.05 radius + 1e-4 max|c|,
+// evaluated with 0.9438, 1.0501, 1.0563 and 0.0501 for the rounding of the
+// sums and of the approximate root (2^-22).  Flagged faces and far ones have
+// no bounds.
+//
+// The faces are taken in short loops, each over this thread's own list, since
+// the one loop over all ~30 ring entries that tests a face where it meets it
+// runs its test for a few lanes at nearly every entry of the warp:
+//   1. of the nearest vertex's ring, the face with the nearest centre is
+//      tested;
+//   2. the heads of all entries: those with lb above the distance found are
+//      dropped, the rest listed;
+//   3. of these, the faces that contain an earlier listed vertex are dropped
+//      (already met in that vertex's ring with the same inputs);
+//   4. the remaining faces (two to four) are tested.
+// The smallest squared distance wins, the first entry in the CSR's order on
+// ties, as in project_onering's strict '<'.  More than kRingList entries
+// listed: project_onering itself.  Bound by the latency of the gathers (the
+// warp waits on loads 9 of 16 cycles per instruction at 24 warps per SM).
+// Projection kernel on 300k sites and 500k faces, mixed: 114 us with one loop
+// over interleaved 64-byte records, 111 with heads apart, 105 so; an FP32
+// edge test before the FP64 one (109) and 32 warps (spills; 104) gain nothing.
+constexpr int kRingList = 32;
+template <int BS> struct RingList { int e[kRingList][BS]; };  // entries, per thread
+
 template <class T, class Q>
-__device__ __forceinline__ V3<T> project_onering_rec(V3<T> c, const float4* __restrict__ rec, int nV,
-                                                     const int* __restrict__ off, const int* knnv, int kproj) {
-  V3<Q> cq = cvt3<Q>(c), bp = cq;
-  Q best = (Q)1e30;
+__device__ __noinline__ V3<T> project_onering_plain(V3<T> c, const float* __restrict__ V, int nV,
+                                                    const int* __restrict__ F, int nF, const int* __restrict__ off,
+                                                    const int* __restrict__ fcs, const int* knnv, int kproj) {
+  return project_onering<T, Q>(c, V, nV, F, nF, off, fcs, knnv, kproj);
+}
+
+__device__ __forceinline__ float approx_root(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// false: more than kRingList faces are left (out is not set)
+template <class T, class Q, int BS, int NV>
+__device__ __forceinline__ bool project_onering_rec(V3<T> c, const float4* __restrict__ head,
+                                                    const float4* __restrict__ body, int nV,
+                                                    const int* __restrict__ off, const int (&knnv)[NV],
+                                                    RingList<BS>& L, V3<T>& out) {
+  const int col = threadIdx.x;
   const float qx = (float)c.x, qy = (float)c.y, qz = (float)c.z;
-  const float qm = fmaxf(fabsf(qx), fmaxf(fabsf(qy), fabsf(qz)));
-  for (int t = 0; t < kproj; ++t) {
-    int v = knnv[t];
-    if ((unsigned)v >= (unsigned)nV) continue;
-    int beg = __ldg(off + v), end = __ldg(off + v + 1);
-    for (int ii = beg; ii < end; ++ii) {
-      const float4* r = rec + kRingWords * (long)ii;
-      // ids and sphere first; the corner words only for faces that are tested
-      const float4 r2 = __ldg(r + 2), r3 = __ldg(r + 3);
-      const int ia = __float_as_int(r2.y), ib = __float_as_int(r2.z), ic = __float_as_int(r2.w);
-      if (ia < 0) continue;
-      bool seen = false;
-      for (int s = 0; s < t; ++s) {
-        const int w = knnv[s];
-        seen = seen || w == ia || w == ib || w == ic;
-      }
-      if (seen) continue;
-      if (r3.w >= 0.f) {
-        const float dx = qx - r3.x, dy = qy - r3.y, dz = qz - r3.z;
-        const float dc = __fsqrt_rn(fmaT(dz, dz, fmaT(dy, dy, dx * dx)));
-        const float mc = fmaxf(qm, fmaxf(fabsf(r3.x), fmaxf(fabsf(r3.y), fabsf(r3.z))));
-        const float lb = dc - r3.w - 0.05f * (dc + r3.w) - 1e-4f * mc - 1e-4f * divT(dc * dc, r3.w);
-        if (lb > 0.f && (double)lb * (double)lb > 1.001 * (double)best) continue;
-      }
-      const float4 r0 = __ldg(r), r1 = __ldg(r + 1);
-      V3<Q> A = {(Q)r0.x, (Q)r0.y, (Q)r0.z};
-      V3<Q> B = {(Q)r0.w, (Q)r1.x, (Q)r1.y};
-      V3<Q> C = {(Q)r1.z, (Q)r1.w, (Q)r2.x};
-      V3<Q> p = closest_point_tri(cq, A, B, C);
-      V3<Q> dd = sub3(p, cq);
-      Q d2 = dot3(dd, dd);
-      if (d2 < best) { best = d2; bp = p; }
+  const float slack = 1e-4f * fmaxf(fabsf(qx), fmaxf(fabsf(qy), fabsf(qz)));
+  int beg[NV], end[NV];
+#pragma unroll
+  for (int t = 0; t < NV; ++t) {
+    const bool valid = (unsigned)knnv[t] < (unsigned)nV;
+    beg[t] = valid ? __ldg(off + knnv[t]) : 0;
+    end[t] = valid ? __ldg(off + knnv[t] + 1) : 0;
+  }
+  const V3<Q> cq = cvt3<Q>(c);
+  V3<Q> bp = cq;
+  Q best = (Q)1e30;
+  int best_at = 0;
+  auto test = [&](int entry, int at) {
+    const float4* w = body + kRingBody * (long)entry;
+    const float4 r0 = __ldg(w), r1 = __ldg(w + 1), r2 = __ldg(w + 2);
+    if (__float_as_int(r2.y) < 0) return;  // an invalid entry
+    const V3<Q> A = {(Q)r0.x, (Q)r0.y, (Q)r0.z};
+    const V3<Q> B = {(Q)r0.w, (Q)r1.x, (Q)r1.y};
+    const V3<Q> C = {(Q)r1.z, (Q)r1.w, (Q)r2.x};
+    const V3<Q> p = closest_point_tri(cq, A, B, C);
+    const V3<Q> dd = sub3(p, cq);
+    const Q d2 = dot3(dd, dd);
+    if (d2 < best || (d2 == best && at < best_at)) { best = d2; bp = p; best_at = at; }
+  };
+  auto dist = [&](float4 h) {
+    const float dx = qx - h.x, dy = qy - h.y, dz = qz - h.z;
+    return approx_root(fmaT(dz, dz, fmaT(dy, dy, dx * dx)));
+  };
+  int first = -1;
+  {
+    float dmin = INFINITY;
+    for (int i = beg[0]; i < end[0]; ++i) {
+      const float dc = dist(__ldg(head + i));
+      if (dc < dmin) { dmin = dc; first = i; }
     }
   }
-  return cvt3<T>(bp);
+  float limit = INFINITY;
+  if (first >= 0) {
+    test(first, first - end[0]);
+    limit = approx_root((float)best) * 1.001f;
+  }
+  // entries that may hold a nearer point, in the CSR's order; for ties an
+  // entry's place is its list index, below 0 in the first ring
+  int cnt = 0;
+  int ends[NV];  // list length after ring t
+#pragma unroll
+  for (int t = 0; t < NV; ++t) {
+    for (int i0 = beg[t]; i0 < end[t]; i0 += 2) {
+      float4 h[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) h[k] = __ldg(head + min(i0 + k, end[t] - 1));
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float dc = dist(h[k]), r = h[k].w;
+        if (dc <= 50.f * r && fmaT(0.9438f, dc, -slack) - 1.0501f * r > limit) continue;
+        const int i = i0 + k;
+        if (i >= end[t] || i == first) continue;
+        if (cnt < kRingList) L.e[cnt][col] = i;
+        ++cnt;
+      }
+    }
+    ends[t] = cnt;
+  }
+  if (cnt > kRingList) return false;
+  int m = 0, m0 = 0;
+  for (int k = 0; k < cnt; ++k) {
+    const int e = L.e[k][col];
+    const float4 r2 = __ldg(body + kRingBody * (long)e + 2);
+    const int ia = __float_as_int(r2.y), ib = __float_as_int(r2.z), ic = __float_as_int(r2.w);
+    bool seen = ia < 0;
+#pragma unroll
+    for (int s = 0; s + 1 < NV; ++s) {
+      const int w = knnv[s];
+      seen = seen || (k >= ends[s] && (w == ia || w == ib || w == ic));
+    }
+    if (!seen) L.e[m++][col] = e;
+    if (k < ends[0]) m0 = m;
+  }
+  for (int k = 0; k < m; ++k) {
+    const int e = L.e[k][col];
+    test(e, k < m0 ? e - end[0] : k);
+  }
+  out = cvt3<T>(bp);
+  return true;
 }
 
 // --------------------------------------------------------------------------

@@ -205,13 +205,12 @@ __global__ void __launch_bounds__(BLOCK) k_stage_clip(const float* __restrict__ 
   using PP = typename PT<PROF>::PP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   V2<PP>* sm = reinterpret_cast<V2<PP>*>(smem_raw);
-  PolyRef<PP> A{sm + threadIdx.x, BLOCK}, B{sm + CAP * BLOCK + threadIdx.x, BLOCK};
+  const PolyRef<PP> cur{sm + threadIdx.x, BLOCK};
   const int i = blockIdx.x * BLOCK + threadIdx.x;
   if (i >= n) return;
   V3<float> si = ld3(S, i);
   Frame<float> fr{ld3(U, i), ld3(Vv, i)};
-  PolyRef<PP> cur = A, nxt = B;
-  int np = clip_cell<PROF>(RowNeighbours<float>{S, knn + (size_t)i * K, (uint32_t)n}, si, K, fr, R, cur, nxt, CAP, false);
+  int np = clip_cell<PROF>(RowNeighbours<float>{S, knn + (size_t)i * K, (uint32_t)n}, si, K, fr, R, cur, CAP, false);
   if (np < 0) {
     int k = atomicAdd(ovf, 1);
     ovf[1 + k] = i;
@@ -241,7 +240,7 @@ __global__ void __launch_bounds__(64) k_stage_clip_fallback(const float* __restr
     V3<float> si = ld3(S, i);
     Frame<float> fr{ld3(U, i), ld3(Vv, i)};
     PolyRef<PP> cur{buf[0], 1}, nxt{buf[1], 1};
-    int np = clip_cell<PROF>(RowNeighbours<float>{S, knn + (size_t)i * K, (uint32_t)n}, si, K, fr, R, cur, nxt, kFallbackCap,
+    int np = clip_cell_full<PROF>(RowNeighbours<float>{S, knn + (size_t)i * K, (uint32_t)n}, si, K, fr, R, cur, nxt, kFallbackCap,
                              false);
     V2<PP> c2 = poly_centroid<PP>(cur, np, PROF == PROF_MIXED);
     V3<float> c;

@@ -125,3 +125,32 @@ def test_launches_follow_the_occupied_slots(eng, oracle):
     assert np.array_equal(e.sites(g), oracle.lloyd_run(m.V, m.F, S[70], 12, 0, 6)["S"])
     e.close()
     mesh.close()
+
+
+@pytest.mark.parametrize("profile", ["ref", "mixed", "fp64"])
+def test_cells_beyond_the_buffer_and_long_rings(eng, oracle, profile):
+    """Cells with more than 16 vertices (a ring of 20 sites around one: redone
+    with the 64-vertex cap), square cells of lone sites, and a mesh whose pole
+    vertices have rings of 90 faces (more entries than the projection's list
+    holds)."""
+    nu, nv = 90, 24
+    th = np.pi * np.arange(1, nv) / nv
+    ph = 2 * np.pi * np.arange(nu) / nu
+    V = np.concatenate([[[0, 0, 1]], np.stack([np.sin(th)[:, None] * np.cos(ph), np.sin(th)[:, None] * np.sin(ph),
+                                              np.cos(th)[:, None] + 0 * ph], -1).reshape(-1, 3), [[0, 0, -1]]])
+    i, j = np.meshgrid(np.arange(nv - 2), np.arange(nu), indexing="ij")
+    a, b = 1 + i * nu + j, 1 + i * nu + (j + 1) % nu
+    ring = np.arange(nu)
+    F = np.concatenate([np.stack([0 * ring, 1 + ring, 1 + (ring + 1) % nu], 1),
+                        np.stack([a, a + nu, b], -1).reshape(-1, 3), np.stack([b, a + nu, b + nu], -1).reshape(-1, 3),
+                        np.stack([0 * ring + len(V) - 1, 1 + (nv - 2) * nu + (ring + 1) % nu, 1 + (nv - 2) * nu + ring], 1)])
+    m = mg.Mesh(np.ascontiguousarray(V, np.float32), np.ascontiguousarray(F, np.int32), "poles")
+    t = 2 * np.pi * np.arange(20) / 20
+    cap = np.concatenate([[[0, 0, 1]], np.stack([0.1 * np.cos(t), 0.1 * np.sin(t), np.sqrt(0.99) + 0 * t], 1)])
+    S0 = np.concatenate([cap, mg.sample_sites(m.V, m.F, 500, seed=2), [[0, 0, -1]]]).astype(np.float32)
+    S, st, _ = _run(eng, m, S0, 24, 0, 5, profile, True)
+    r = oracle.lloyd_run(m.V, m.F, S0, 24, 0, 5, profile=oracle.PROFILES[profile])
+    assert np.array_equal(S, r["S"])
+    one = oracle.lloyd_run(m.V, m.F, S0[:21], 24, 0, 2, profile=oracle.PROFILES[profile])  # the 20-gon, with the square around it
+    S, _, _ = _run(eng, m, S0[:21], 24, 0, 2, profile, True)
+    assert np.array_equal(S, one["S"], equal_nan=True)
