@@ -668,13 +668,13 @@ __global__ void k_frame_vertex(EngineArgs<T> a, int parity) {
 // Full search of site g (one warp): the K nearest (MM = 0), or the MM
 // nearest, which refresh its candidate list and whose first K are the
 // K-list.  seg receives the site's segment.  With candidate lists the search
-// is first tried as one radius query (warp_radius_knn, scratch buf of 64
-// keys): within bound tb when the check left one (the largest re-keyed
-// distance of the site's complete old list, so at least MM sites lie within
-// it), else within a squared distance expected to hold about (MM + 64) / 2
-// sites; when the count falls outside [MM, 64] the ring search runs instead.
-// Both return the MM smallest (distance, caller index) keys; the list is
-// stored as internal indices.
+// is first tried as one radius query (warp_radius_knn, scratch buf of
+// kRadiusKeys keys): within bound tb when the check left one (the largest
+// re-keyed distance of the site's complete old list, so at least MM sites lie
+// within it), else within a squared distance expected to hold 1.45 MM sites;
+// when that fails (too few or too many) the ring search runs instead.  Both
+// return the MM smallest (distance, caller index) keys; the list is stored as
+// internal indices.
 template <class T, int KK, int MM>
 __device__ __forceinline__ void knn_search_site(const EngineArgs<T>& a, int parity, int g, float tb, int lane, int& seg,
                                                 typename KeyOps<T>::Key* buf) {
@@ -696,12 +696,11 @@ __device__ __forceinline__ void knn_search_site(const EngineArgs<T>& a, int pari
   auto not_self = [self](uint32_t id) { return id != self; };
   Key mk[2] = {O::empty(), O::empty()};
   if constexpr (MM > 0) {
-    static_assert(MM <= 64, "at most 64 candidates");
     const float rho = a.cand_rho[g];
     const GridGeom G = a.geom[s];
     // kth holds the site's last K-th squared distance (K sites within it);
     // kth_est, from the segment's density, is expected to hold 2 (K + 1)
-    constexpr double kTarget = (MM + 64) / 2.0;
+    constexpr double kTarget = 1.45 * MM;
     const T thr_r = tb >= 0.f ? (T)tb
                     : kp >= 0.f ? (T)kp * (T)(kTarget / KK) : (T)sd.kth_est * (T)(kTarget / (2.0 * (KK + 1)));
     const float qm = fmaxf(fabsf((float)q.x), fmaxf(fabsf((float)q.y), fabsf((float)q.z)));
@@ -985,7 +984,7 @@ __global__ void __launch_bounds__(BS, kKnnSearchWarpsPerSM * 32 / BS) k_knn_sear
   const int nw = (int)((gridDim.x * (unsigned)blockDim.x) >> 5);
   SegCounter<T> searched;
   if constexpr (MM > 0) {
-    __shared__ typename KeyOps<T>::Key buf[BS / 32][64];  // per warp: the radius query's keys
+    __shared__ typename KeyOps<T>::Key buf[BS / 32][kRadiusKeys];  // per warp: the radius query's keys
     auto* mybuf = buf[threadIdx.x >> 5];
     const int n = a.srch[0];
     for (int k = wi; k < n; k += nw) {

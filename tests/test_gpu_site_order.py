@@ -154,3 +154,17 @@ def test_cells_beyond_the_buffer_and_long_rings(eng, oracle, profile):
     one = oracle.lloyd_run(m.V, m.F, S0[:21], 24, 0, 2, profile=oracle.PROFILES[profile])  # the 20-gon, with the square around it
     S, _, _ = _run(eng, m, S0[:21], 24, 0, 2, profile, True)
     assert np.array_equal(S, one["S"], equal_nan=True)
+
+
+@pytest.mark.parametrize("n,k,profile", [(1500, 32, "mixed"), (9000, 32, "ref"), (9000, 8, "mixed"), (9000, 24, "fp64")])
+def test_uneven_density_searches(eng, oracle, n, k, profile):
+    """Full searches whose radius holds far more or fewer sites than expected:
+    nine tenths of the sites packed into a small cap."""
+    m = mg.icosphere(5)
+    S = mg.sample_sites(m.V, m.F, 60 * n, seed=n)
+    cap = S[S[:, 2] > 0.97][: n - n // 10]
+    S0 = np.random.default_rng(3).permutation(np.concatenate([cap, S[: n - len(cap)]]))
+    S, st, _ = _run(eng, m, S0, k, 0, 3, profile, True)
+    r = oracle.lloyd_run(m.V, m.F, S0, k, 0, 3, profile=oracle.PROFILES[profile])
+    assert np.array_equal(st["knn"], r["knn"])
+    assert np.array_equal(S, r["S"])
