@@ -140,6 +140,9 @@ static int sm_count() {
   return n > 0 ? n : 148;
 }
 
+// blocks of a grid-stride kernel over n items: at most four per SM
+static int wave_blocks(long n, int threads) { return std::min(cdiv(n, threads), 4 * sm_count()); }
+
 // Streams a host thread runs engine iterations on besides the caller's: the
 // second branch of an eagerly launched iteration, and the origin and second
 // branch of a graph capture.  One set per thread and device, because a
@@ -218,7 +221,7 @@ static cvt_status_t build_point_grid(Scratch& sc, const float* P, int n, float p
     CK(sc.get(&bb, 6));
     k_bbox_init<<<1, 32, 0, st>>>(bb);
     CKLAUNCH();
-    if (n > 0) { k_bbox<<<cdiv(n, 256), 256, 0, st>>>(n, P, bb); CKLAUNCH(); }
+    if (n > 0) { k_bbox<<<wave_blocks(n, kBboxThreads), kBboxThreads, 0, st>>>(n, P, bb); CKLAUNCH(); }
     k_grid_geom<<<1, 32, 0, st>>>(bb, n, per_cell, cap, pg.geom);
     CKLAUNCH();
   }
@@ -452,6 +455,8 @@ struct cvt_mesh {
   int n_unref = 0;
   BVHNode* dnodes = nullptr;  // built on first use (Hausdorff)
   int* dtri = nullptr;
+  float4* dbvh = nullptr;     // the tree as the traversals read it: pairs, then triangles
+  BvhView bvh{};
   int nnodes = 0;
   void* arena = nullptr;      // V, F, CSR, normals, ring records, unreferenced vertices
   void* arena_grid = nullptr; // vertex grid (sized once the area is known)
@@ -461,7 +466,7 @@ struct cvt_mesh {
     MeshDev m;
     m.V = dV; m.F = dF; m.vf_off = doff; m.vf_faces = dfcs; m.N = dN;
     m.vcell_start = dvcell_start; m.vsorted = dvsorted; m.ring_head = dring_head; m.ring_body = dring_body; m.vg = vg;
-    m.bvh = dnodes; m.bvh_tri = dtri;
+    m.bvh = bvh;
     m.nV = nV; m.nF = nF; m.R = R;
     m.thr2 = ((0.01f * R) * 0.01f) * R;
     return m;
@@ -488,7 +493,7 @@ struct Arena {
 static void mesh_free(cvt_mesh* m) {
   if (!m) return;
   dev_free_sync(m->arena); dev_free_sync(m->arena_grid); dev_free_sync(m->dcdf); dev_free_sync(m->dnodes);
-  dev_free_sync(m->dtri);
+  dev_free_sync(m->dtri); dev_free_sync(m->dbvh);
   delete m;
 }
 
@@ -501,8 +506,10 @@ static int bvh_subtree_nodes(int n, int leaf, std::vector<std::pair<int, int>>& 
   return c;
 }
 
-// BVH of the mesh (evaluate.cuh:114-201, leaf 8), built on the device level
-// by level (cvt_ingest.cuh) the first time a Hausdorff distance needs it.
+// BVH of the mesh (evaluate.cuh:114-201, leaf 8), built on the device the
+// first time something needs it (cvt_ingest.cuh): the upper levels one after
+// another over all triangles, each segment of at most kSubTris triangles then
+// by one block.
 static cvt_status_t mesh_ensure_bvh(cvt_mesh* m) {
   std::lock_guard<std::mutex> lk(m->lazy_mu);
   if (m->dnodes) return CVT_OK;
@@ -513,27 +520,58 @@ static cvt_status_t mesh_ensure_bvh(cvt_mesh* m) {
   const int n_nodes = bvh_subtree_nodes(nF, leaf, memo);
   BVHNode* dn = nullptr;
   int* dt = nullptr;
-  cudaError_t e = dev_alloc_sync(reinterpret_cast<void**>(&dn), sizeof(BVHNode) * (size_t)n_nodes);
-  if (e == cudaSuccess) e = dev_alloc_sync(reinterpret_cast<void**>(&dt), sizeof(int) * (size_t)nF);
+  float4* db = nullptr;
+  const size_t bvh_words = 4 * (size_t)n_nodes + 3 * (size_t)nF;
+  cudaError_t e = dev_alloc(reinterpret_cast<void**>(&dn), sizeof(BVHNode) * (size_t)n_nodes, st);
+  if (e == cudaSuccess) e = dev_alloc(reinterpret_cast<void**>(&dt), sizeof(int) * (size_t)nF, st);
+  if (e == cudaSuccess) e = dev_alloc(reinterpret_cast<void**>(&db), sizeof(float4) * bvh_words, st);
   auto bail = [&](cudaError_t err) {
-    dev_free_sync(dn); dev_free_sync(dt);
+    dev_free_sync(dn); dev_free_sync(dt); dev_free_sync(db);
     return fail(err == cudaErrorMemoryAllocation ? CVT_ERR_OOM : CVT_ERR_CUDA,
                 std::string("mesh BVH: ") + cudaGetErrorString(err));
   };
   if (e != cudaSuccess) return bail(e);
+  // segments of the upper levels, one level after another; the last level's
+  // go to k_bvh_subtree
+  std::vector<BvhSeg> table{{0, nF, 0, -1, -1}};
+  std::vector<std::pair<int, int>> levels{{0, 1}};  // first segment, segments
+  while (true) {
+    const auto [first, nseg] = levels.back();
+    bool split = false;
+    for (int k = first; k < first + nseg; ++k) split = split || table[k].count > kSubTris;
+    if (!split) break;
+    for (int k = first; k < first + nseg; ++k) {
+      BvhSeg& g = table[k];
+      if (g.count <= leaf) continue;
+      g.left = g.node + 1;
+      g.right = g.node + 1 + bvh_subtree_nodes(g.count / 2, leaf, memo);
+    }
+    const int at = (int)table.size();
+    for (int k = first; k < first + nseg; ++k) {
+      const BvhSeg g = table[k];
+      table.push_back({g.start, g.count / 2, g.left, -1, -1});
+      table.push_back({g.start + g.count / 2, g.count - g.count / 2, g.right, -1, -1});
+    }
+    levels.push_back({at, (int)table.size() - at});
+  }
+  // (segments of one level differ by at most one triangle, so all split)
+  int sub[kSubTris + 1];
+  for (int k = 0; k <= kSubTris; ++k) sub[k] = k <= leaf ? 1 : 1 + sub[k / 2] + sub[k - k / 2];
+  BVHNode root;
   {
     Scratch sc(st);
     float* tinfo;
-    int *ids2, *acc, *axis;
+    int *ids2, *acc, *axis, *dsub;
     unsigned long long *keys, *keys2;
     BvhSeg* dseg;
-    // a split segment has more than `leaf` triangles, so both halves hold at
-    // least leaf/2: the frontier never has more than nF/(leaf/2) + 1 segments
-    const size_t max_seg = (size_t)nF / (leaf / 2) + 2;
+    const size_t max_seg = (size_t)levels.back().second;
     if ((e = sc.get(&tinfo, 9 * (size_t)nF)) != cudaSuccess || (e = sc.get(&ids2, (size_t)nF)) != cudaSuccess ||
         (e = sc.get(&keys, (size_t)nF)) != cudaSuccess || (e = sc.get(&keys2, (size_t)nF)) != cudaSuccess ||
         (e = sc.get(&acc, 12 * max_seg)) != cudaSuccess || (e = sc.get(&axis, max_seg)) != cudaSuccess ||
-        (e = sc.get(&dseg, max_seg)) != cudaSuccess)
+        (e = sc.get(&dseg, table.size())) != cudaSuccess || (e = sc.get(&dsub, kSubTris + 1)) != cudaSuccess)
+      return bail(e);
+    if ((e = cudaMemcpyAsync(dseg, table.data(), sizeof(BvhSeg) * table.size(), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(dsub, sub, sizeof(sub), cudaMemcpyHostToDevice, st)) != cudaSuccess)
       return bail(e);
     k_tri_info<<<cdiv(nF, 256), 256, 0, st>>>(m->dV, m->dF, nF, tinfo);
     k_iota<<<cdiv(nF, 256), 256, 0, st>>>(dt, nF);
@@ -543,53 +581,43 @@ static cvt_status_t mesh_ensure_bvh(cvt_mesh* m) {
       return bail(e);
     void* tmp;
     if ((e = sc.get(reinterpret_cast<char**>(&tmp), tb)) != cudaSuccess) return bail(e);
-    std::vector<BvhSeg> segs{{0, nF, 0, -1, -1}};
     int* cur = dt;
     int* alt = ids2;
-    while (true) {
-      bool split = false;
-      for (auto& g : segs)
-        if (g.node >= 0 && g.count > leaf) {
-          g.left = g.node + 1;
-          g.right = g.node + 1 + bvh_subtree_nodes(g.count / 2, leaf, memo);
-          split = true;
-        }
-      const int nseg = (int)segs.size();
-      if ((e = cudaMemcpyAsync(dseg, segs.data(), sizeof(BvhSeg) * nseg, cudaMemcpyHostToDevice, st)) != cudaSuccess)
-        return bail(e);
+    for (size_t l = 0; l + 1 < levels.size(); ++l) {
+      const BvhSeg* seg = dseg + levels[l].first;
+      const int nseg = levels[l].second;
       k_seg_acc_init<<<cdiv(nseg, 256), 256, 0, st>>>(nseg, acc);
-      k_seg_reduce<<<cdiv(nF, 256), 256, 0, st>>>(cur, nF, dseg, nseg, tinfo, acc);
-      k_seg_emit<<<cdiv(nseg, 256), 256, 0, st>>>(dseg, nseg, acc, leaf, dn, axis);
-      LAUNCHED(3);
-      if (!split) break;
-      k_seg_keys<<<cdiv(nF, 256), 256, 0, st>>>(cur, nF, dseg, nseg, axis, tinfo, keys);
-      LAUNCHED(1);
-      int sbits = 1;
+      k_seg_reduce<<<cdiv(nF, 256), 256, 0, st>>>(cur, nF, seg, nseg, tinfo, acc);
+      k_seg_emit<<<cdiv(nseg, 256), 256, 0, st>>>(seg, nseg, acc, leaf, dn, axis);
+      k_seg_keys<<<cdiv(nF, 256), 256, 0, st>>>(cur, nF, seg, nseg, axis, tinfo, keys);
+      LAUNCHED(4);
+      int sbits = 0;
       while (sbits < 31 && (1LL << sbits) < (long long)nseg) ++sbits;
       if ((e = cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, cur, alt, nF, 0, 32 + sbits, st)) != cudaSuccess)
         return bail(e);
       std::swap(cur, alt);
-      std::vector<BvhSeg> next;
-      next.reserve(2 * segs.size());
-      for (const auto& g : segs) {
-        if (g.node >= 0 && g.count > leaf) {
-          next.push_back({g.start, g.count / 2, g.left, -1, -1});
-          next.push_back({g.start + g.count / 2, g.count - g.count / 2, g.right, -1, -1});
-        } else {
-          next.push_back({g.start, g.count, -1, -1, -1});
-        }
-      }
-      // (a pageable upload has left the host buffer when cudaMemcpyAsync
-      // returns; the device copy is reused in stream order)
-      segs.swap(next);
     }
+    if ((e = cudaFuncSetAttribute(k_bvh_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SubTree))) != cudaSuccess)
+      return bail(e);
+    k_bvh_subtree<<<levels.back().second, kSubThreads, sizeof(SubTree), st>>>(cur, dseg + levels.back().first, tinfo, dsub, leaf, dn);
+    LAUNCHED(1);
     if (cur != dt && (e = cudaMemcpyAsync(dt, cur, sizeof(int) * (size_t)nF, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
       return bail(e);
-    if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(st)) != cudaSuccess) return bail(e);
+    k_bvh_pack<<<cdiv(n_nodes, 128), 128, 0, st>>>(dn, n_nodes, dt, m->dV, m->dF, db, db + 4 * (size_t)n_nodes);
+    LAUNCHED(1);
+    if ((e = cudaGetLastError()) != cudaSuccess ||
+        (e = cudaMemcpyAsync(&root, dn, sizeof(BVHNode), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(st)) != cudaSuccess)
+      return bail(e);
   }
   m->nnodes = n_nodes;
   m->dtri = dt;
-  m->bytes += sizeof(BVHNode) * (size_t)n_nodes + sizeof(int) * (size_t)nF;
+  m->dbvh = db;
+  m->bvh.pair = db;
+  m->bvh.tris = db + 4 * (size_t)n_nodes;
+  for (int a = 0; a < 3; ++a) { m->bvh.bmin[a] = root.bmin[a]; m->bvh.bmax[a] = root.bmax[a]; }
+  m->bvh.root = root.triCount > 0 ? ~0 : 0;
+  m->bytes += sizeof(BVHNode) * (size_t)n_nodes + sizeof(int) * (size_t)nF + sizeof(float4) * bvh_words;
   m->dnodes = dn;
   return CVT_OK;
 }
@@ -697,7 +725,7 @@ static cvt_status_t mesh_create_on(const float* V, int nV, const int* F, int nF,
   MCK(cudaMemsetAsync(info, 0, sizeof(int), st));
   k_ingest_bounds_init<<<1, 32, 0, st>>>(info + 1);
   k_ingest_mark<<<cdiv(n3, 256), 256, 0, st>>>(rF, n3, nV, used, info);
-  k_ingest_bounds<<<cdiv(nV, 256), 256, 0, st>>>(rV, nV, used, info + 1, info);
+  k_ingest_bounds<<<wave_blocks(nV, 256), 256, 0, st>>>(rV, nV, used, info + 1, info);
   LAUNCHED(3);
   MCK(cudaGetLastError());
   {
@@ -846,7 +874,7 @@ extern "C" cvt_status_t cvt_hausdorff_to_mesh(cvt_mesh_t ref, const float* Vc, i
   CK(sc.get(&ovf, 1));
   CK(cudaMemsetAsync(bits, 0, sizeof(unsigned), st));
   CK(cudaMemsetAsync(ovf, 0, sizeof(int), st));
-  k_hausdorff<<<cdiv(nP, 128), 128, 0, st>>>(Vc, nVc, Fc, nP, ref->dnodes, ref->dtri, ref->dV, ref->dF, bits, ovf);
+  k_hausdorff<<<cdiv(nP, 128), 128, 0, st>>>(Vc, nVc, Fc, nP, ref->bvh, bits, ovf);
   CKLAUNCH();
   unsigned hb = 0;
   int ho = 0;
@@ -891,9 +919,9 @@ extern "C" cvt_status_t cvt_project_bvh(cvt_mesh_t m, const float* cent, int n, 
   CK(sc.get(&ovf, 1));
   CK(cudaMemsetAsync(ovf, 0, sizeof(int), st));
   if (profile == CVT_PROFILE_REF)
-    k_stage_project_bvh<PROF_REF><<<cdiv(n, 128), 128, 0, st>>>(cent, n, m->dnodes, m->dtri, m->dV, m->dF, Sold, Snew, ovf);
+    k_stage_project_bvh<PROF_REF><<<cdiv(n, 128), 128, 0, st>>>(cent, n, m->bvh, Sold, Snew, ovf);
   else
-    k_stage_project_bvh<PROF_MIXED><<<cdiv(n, 128), 128, 0, st>>>(cent, n, m->dnodes, m->dtri, m->dV, m->dF, Sold, Snew, ovf);
+    k_stage_project_bvh<PROF_MIXED><<<cdiv(n, 128), 128, 0, st>>>(cent, n, m->bvh, Sold, Snew, ovf);
   CKLAUNCH();
   int h_ovf = 0;
   CK(cudaMemcpyAsync(&h_ovf, ovf, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -920,12 +948,11 @@ extern "C" cvt_status_t cvt_hausdorff_meshes(cvt_mesh_t a, cvt_mesh_t b, float* 
   // three edge midpoints) against the BVH of `to`, max into *dst
   auto side = [&](const cvt_mesh* from, const cvt_mesh* to, unsigned* dst) -> cudaError_t {
     const long nP = (long)from->nV + 4L * from->nF;
-    k_hausdorff<<<cdiv(nP, 128), 128, 0, st>>>(from->dV, from->nV, from->dF, nP, to->dnodes, to->dtri, to->dV,
-                                               to->dF, dst, ovf);
+    k_hausdorff<<<cdiv(nP, 128), 128, 0, st>>>(from->dV, from->nV, from->dF, nP, to->bvh, dst, ovf);
     LAUNCHED(1);
     if (from->n_unref) {
       k_hausdorff<<<cdiv(from->n_unref, 128), 128, 0, st>>>(from->dunref, from->n_unref, nullptr, from->n_unref,
-                                                             to->dnodes, to->dtri, to->dV, to->dF, dst, ovf);
+                                                             to->bvh, dst, ovf);
       LAUNCHED(1);
     }
     return cudaGetLastError();
@@ -2076,8 +2103,9 @@ static cvt_status_t extract_faces(const float* S, const float* U, const float* V
   *n_faces = 0;
   if (n == 0) return CVT_OK;
   Scratch sc(st);
-  int* cnt;
+  int *cnt, *over;
   CK(sc.get(&cnt, 1));
+  CK(sc.get(&over, (size_t)n + 1));
   int cap = std::max(16 * n, 1024);
   unsigned long long* keys = nullptr;
   int nk = 0;
@@ -2085,7 +2113,10 @@ static cvt_status_t extract_faces(const float* S, const float* U, const float* V
     Scratch ks(st);
     CK(ks.get(&keys, (size_t)cap));
     CK(cudaMemsetAsync(cnt, 0, sizeof(int), st));
-    k_face_keys<<<cdiv(n, 64), 64, 0, st>>>(S, U, V, nb, n, K, R2, 1e-8f, 1e-7f, keys, cnt, cap);
+    CK(cudaMemsetAsync(over, 0, sizeof(int), st));
+    k_face_keys<<<cdiv(n, kFaceThreads), kFaceThreads, 0, st>>>(S, U, V, nb, n, K, R2, 1e-8f, 1e-7f, keys, cnt, cap, over);
+    CKLAUNCH();
+    k_face_keys_over<<<sm_count(), 64, 0, st>>>(S, U, V, nb, n, K, R2, 1e-8f, 1e-7f, keys, cnt, cap, over);
     CKLAUNCH();
     CK(cudaMemcpyAsync(&nk, cnt, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -2152,7 +2183,7 @@ extern "C" cvt_status_t cvt_quality(const float* V, const int* F, int nF, float*
   CK(sc.get(&mins, 2));
   CK(cudaMemsetAsync(acc, 0, 4 * sizeof(double), st));
   CK(cudaMemsetAsync(mins, 0x7f, 2 * sizeof(unsigned), st));
-  k_quality<<<cdiv(nF, 256), 256, 0, st>>>(V, F, nF, acc, mins);
+  k_quality<<<wave_blocks(nF, kQualityThreads), kQualityThreads, 0, st>>>(V, F, nF, acc, mins);
   CKLAUNCH();
   double h[4];
   unsigned m[2];
@@ -2242,7 +2273,7 @@ static cvt_status_t engine_eval_impl(cvt_engine_t e, int s, cvt_eval_t* out, int
   CK(sc.get(&bb, 6));
   k_bbox_init<<<1, 32, 0, st>>>(bb);
   CKLAUNCH();
-  k_bbox<<<cdiv(n, 256), 256, 0, st>>>(n, Sf, bb);
+  k_bbox<<<wave_blocks(n, kBboxThreads), kBboxThreads, 0, st>>>(n, Sf, bb);
   CKLAUNCH();
   int hb[6];
   CK(cudaMemcpyAsync(hb, bb, sizeof(hb), cudaMemcpyDeviceToHost, st));

@@ -77,8 +77,7 @@ struct MeshDev {
   const Pt4<float>* vsorted;
   const float4* ring_head;  // one-ring records, one head and kRingBody body words per CSR entry
   const float4* ring_body;  // (k_build_ring_records)
-  const BVHNode* bvh;  // BVH over the faces (built before a segment that projects through it is placed)
-  const int* bvh_tri;
+  BvhView bvh;  // over the faces (built before a segment that projects through it is placed)
   GridGeom vg;
   int nV, nF;
   float R;     // clip square half-size: longest input bbox edge (main.cu:421)
@@ -1103,7 +1102,7 @@ __device__ __forceinline__ void site_finish(const EngineArgs<typename PT<PROF>::
   if (PROF == PROF_MIXED && !finite3(cent)) {
     sn = si;
   } else if (PROJ == 1) {
-    sn = project_bvh<T, Q>(cent, md.bvh, md.bvh_tri, md.V, md.F, (Q)bvh_bound2(cent, si), a.bvh_ovf);
+    sn = project_bvh<T, Q>(cent, md.bvh, (Q)bvh_bound2(cent, si), a.bvh_ovf);
   } else if (!project_onering_rec<T, Q, BS>(cent, md.ring_head, md.ring_body, md.nV, md.vf_off, knnv, L, sn)) {
     sn = project_onering_plain<T, Q>(cent, md.V, md.nV, md.F, md.nF, md.vf_off, md.vf_faces, knnv, kKProj);
   }

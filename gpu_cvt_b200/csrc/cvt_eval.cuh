@@ -13,40 +13,26 @@ namespace cvt {
 // triangles, otherwise the centroid-sorted list split at its middle, nodes in
 // pre-order, evaluate.cuh:114-201); it is built on the device, cvt_ingest.cuh.
 
-// Per-probe closest squared distance to the BVH surface.  Near-first
-// traversal: of two children the nearer box is visited first, which only
-// changes the order, not the minimum (stack: kBvhStack, cvt_math.cuh).
-
-__device__ __forceinline__ float bvh_closest_d2(V3<float> p, const BVHNode* __restrict__ nodes,
-                                                const int* __restrict__ tri, const float* __restrict__ V,
-                                                const int* __restrict__ F, int* overflow) {
+// Closest squared distance of p to the surface (the traversal order only
+// changes the order, not the minimum), or any value <= floor2() once it is
+// known not to be above that (floor2 is looked at once per leaf).
+template <class Floor>
+__device__ __forceinline__ float bvh_closest_d2(V3<float> p, const BvhView& bvh, int* overflow, Floor floor2) {
   float best = 1e30f;
-  int stack[kBvhStack];
-  int sp = 0;
-  stack[sp++] = 0;
-  while (sp) {
-    const BVHNode nd = nodes[stack[--sp]];
-    if (aabb_d2(p, nd.bmin, nd.bmax) >= best) continue;
-    if (nd.triCount > 0) {
-      for (int k = 0; k < nd.triCount; ++k) {
-        int t = __ldg(tri + nd.triStart + k);
-        V3<float> a = ld3(V, __ldg(F + 3 * t)), b = ld3(V, __ldg(F + 3 * t + 1)), c = ld3(V, __ldg(F + 3 * t + 2));
-        float d2 = point_tri_d2(p, a, b, c);
-        if (d2 < best) best = d2;
-      }
-    } else {
-      const BVHNode L = nodes[nd.left], R = nodes[nd.right];
-      float dl = aabb_d2(p, L.bmin, L.bmax), dr = aabb_d2(p, R.bmin, R.bmax);
-      if (sp + 2 > kBvhStack) { atomicAdd(overflow, 1); continue; }
-      if (dl < dr) {
-        if (dr < best) stack[sp++] = nd.right;
-        if (dl < best) stack[sp++] = nd.left;
-      } else {
-        if (dl < best) stack[sp++] = nd.left;
-        if (dr < best) stack[sp++] = nd.right;
+  bvh_walk(bvh, p, overflow, [&]() { return best; }, [&](int t) {
+    const float fl = floor2();
+    for (bool last = false; !last; ++t) {
+      const float4* w = bvh.tris + 3 * (size_t)t;
+      const float4 r0 = __ldg(w), r1 = __ldg(w + 1), r2 = __ldg(w + 2);
+      last = __float_as_int(r2.y) != 0;
+      const float d2 = point_tri_d2(p, {r0.x, r0.y, r0.z}, {r0.w, r1.x, r1.y}, {r1.z, r1.w, r2.x});
+      if (d2 < best) {
+        best = d2;
+        if (best <= fl) return false;
       }
     }
-  }
+    return true;
+  });
   return best;
 }
 
@@ -67,23 +53,24 @@ __device__ __forceinline__ V3<float> probe_point(const float* __restrict__ V, in
 // max over probes of the closest squared distance, reduced in-kernel:
 // warp max, then one atomicMax on the float bits (non-negative floats
 // order as unsigned ints) -- replaces the CUB max of evaluate.cuh:335-343.
+// A probe whose closest distance so far is not above the maximum of the
+// probes already done cannot raise it and stops there, which ends most of
+// them at their first leaf; the maximum is the same.
 __global__ void __launch_bounds__(128) k_hausdorff(const float* __restrict__ Vc, int nVc, const int* __restrict__ Fc,
-                                                   long nP, const BVHNode* __restrict__ nodes, const int* __restrict__ tri,
-                                                   const float* __restrict__ Vr, const int* __restrict__ Fr,
-                                                   unsigned* out_bits, int* overflow) {
+                                                   long nP, BvhView bvh, unsigned* out_bits, int* overflow) {
   long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   float d = 0.f;
-  if (k < nP) d = bvh_closest_d2(probe_point(Vc, nVc, Fc, k), nodes, tri, Vr, Fr, overflow);
+  if (k < nP)
+    d = bvh_closest_d2(probe_point(Vc, nVc, Fc, k), bvh, overflow,
+                       [&]() { return __uint_as_float(*(volatile unsigned*)out_bits); });
   unsigned b = __float_as_uint(d);
   b = __reduce_max_sync(0xffffffffu, b);
-  if ((threadIdx.x & 31) == 0) atomicMax(out_bits, b);
+  if ((threadIdx.x & 31) == 0 && b > *(volatile unsigned*)out_bits) atomicMax(out_bits, b);
 }
 
 // ---------------------------------------------------------------------------
 // dual-triangle extraction
 // ---------------------------------------------------------------------------
-constexpr int kFaceMaxPoly = 256;   // MAX_POLY (main.cu:393)
-
 // Neighbour lists of k_face_keys: get(i, t) is entry t of site i's list (an
 // index into the sites, or out of range), label(i) the index that a site has
 // in the faces.
@@ -107,77 +94,167 @@ struct FaceColumns {  // an engine segment's lists (from its first site on)
 
 // Labelled clip (near_project.cuh:201-244) + active-bisector pairs
 // (near_project.cuh:318-351) + key emission (buildmesh.cuh:170-201) per site.
-// Buffers: per thread 2 x kFaceMaxPoly float2 + labels in local memory.
+
+__device__ __forceinline__ void face_emit(int x, int y, int z, unsigned long long* keys, int* key_count, int max_keys) {
+  int tmp;
+  if (x > y) { tmp = x; x = y; y = tmp; }
+  if (y > z) { tmp = y; y = z; z = tmp; }
+  if (x > y) { tmp = x; x = y; y = tmp; }
+  const int pos = atomicAdd(key_count, 1);
+  if (pos < max_keys)
+    keys[pos] = (unsigned long long)(uint32_t)x | ((unsigned long long)(uint32_t)y << 21) |
+                ((unsigned long long)(uint32_t)z << 42);
+}
+
+// One site per thread, the polygon in shared memory (kFaceCap vertices), cut
+// in place by outside masks as clip_cell does; sites that need more vertices
+// or whose outside vertices are not one run go to `over` (k_face_keys_over).
+// The clip's labels only name the edges, which the faces do not use: a face
+// joins the site and the two listed neighbours whose bisectors pass nearest a
+// vertex, both within tol_active; neighbours beyond it cannot be among them,
+// so one pass over the neighbours finds both for every vertex.  100k sites,
+// K = 24: 148 us with 256-vertex buffers in local memory and all neighbours'
+// bisectors recomputed for every vertex, now 110.
+constexpr int kFaceThreads = 64;
+constexpr int kFaceCap = 16;
+
 template <class NB>
-__global__ void __launch_bounds__(64) k_face_keys(const float* __restrict__ S, const float* __restrict__ U,
-                                                  const float* __restrict__ Vv, NB nb,
-                                                  int n, int K, float R2, float eps_clip, float tol_active,
-                                                  unsigned long long* keys, int* key_count, int max_keys) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kFaceThreads) k_face_keys(const float* __restrict__ S, const float* __restrict__ U,
+                                                            const float* __restrict__ Vv, NB nb, int n, int K, float R2,
+                                                            float eps_clip, float tol_active, unsigned long long* keys,
+                                                            int* key_count, int max_keys, int* __restrict__ over) {
+  __shared__ float2 P[kFaceCap][kFaceThreads];
+  __shared__ float2 near_d[kFaceCap][kFaceThreads];  // the two smallest |f| within tol_active
+  __shared__ int2 near_j[kFaceCap][kFaceThreads];
+  const int c = threadIdx.x, i = blockIdx.x * kFaceThreads + threadIdx.x;
   if (i >= n) return;
-  float2 bufA[kFaceMaxPoly], bufB[kFaceMaxPoly];
-  int labA[kFaceMaxPoly], labB[kFaceMaxPoly];
-  float2* cp = bufA; float2* np = bufB;
-  int* cl = labA; int* nl = labB;
-  int na = 4;
-  cp[0] = make_float2(-R2, -R2); cp[1] = make_float2(R2, -R2); cp[2] = make_float2(R2, R2); cp[3] = make_float2(-R2, R2);
-  cl[0] = cl[1] = cl[2] = cl[3] = -1;
   const V3<float> si = ld3(S, i), ui = ld3(U, i), vi = ld3(Vv, i);
+  P[0][c] = make_float2(-R2, -R2); P[1][c] = make_float2(R2, -R2); P[2][c] = make_float2(R2, R2); P[3][c] = make_float2(-R2, R2);
+  int na = 4;
+  float r2 = 2.f * R2 * R2 * 1.0001f;
   for (int t = 0; t < K; ++t) {
-    int j = nb.get(i, t);
+    if (na <= 0) continue;
+    const int j = nb.get(i, t);
     if ((unsigned)j >= (unsigned)n || j == i) continue;
-    V3<float> d = sub3(ld3(S, j), si);
-    float a = dot3(d, ui), b = dot3(d, vi), c = 0.5f * dot3(d, d);
-    int m = 0;
-    if (na > 0) {
+    const V3<float> d = sub3(ld3(S, j), si);
+    const float dd = dot3(d, d);
+    if (dd > 4.01f * r2 && dd > 2e-18f && dd < 1e30f) continue;  // cannot cut (clip_cell)
+    const float a = dot3(d, ui), b = dot3(d, vi), cc = 0.5f * dd;
+    auto f = [&](float2 p) { return fmaT(a, p.x, fmaT(b, p.y, -cc)); };
+    unsigned out = 0u;
+    float rin = 0.f;
+    for (int k = 0; k < na; ++k) {
+      const float2 p = P[k][c];
+      if (f(p) <= eps_clip) rin = fmaxf(rin, fmaT(p.y, p.y, p.x * p.x)); else out |= 1u << k;
+    }
+    if (out == 0u) continue;
+    const unsigned all = 0xffffffffu >> (32 - na);
+    if (out == all) { na = 0; continue; }
+    const unsigned starts = out & ~((out << 1) | (out >> (na - 1)));
+    const int len = __popc(out), p0 = __ffs(starts) - 1;
+    if ((starts & (starts - 1)) || na - len + 2 > kFaceCap) { na = -1; continue; }
+    const int q = p0 + len - 1 >= na ? p0 + len - 1 - na : p0 + len - 1;
+    const int ip = p0 == 0 ? na - 1 : p0 - 1, iq = q + 1 == na ? 0 : q + 1;
+    auto isect = [&](float2 s, float2 e) {
+      const float fs = f(s), fe = f(e);
+      const float tt = divT(fs, (fs - fe) + 1e-30f);
+      return make_float2(fmaT(tt, e.x - s.x, s.x), fmaT(tt, e.y - s.y, s.y));
+    };
+    const float2 enter = isect(P[ip][c], P[p0][c]), leave = isect(P[q][c], P[iq][c]);
+    int lo, hi, shift, at_enter, at_leave;
+    if (p0 <= q && q + 1 < na) { lo = q + 1; hi = na; shift = 2 - len; at_enter = p0; at_leave = p0 + 1; }
+    else { lo = iq; hi = p0; shift = 1 - iq; at_enter = na - len + 1; at_leave = 0; }
+    if (shift > 0) { for (int k = hi - 1; k >= lo; --k) P[k + shift][c] = P[k][c]; }
+    else if (shift < 0) { for (int k = lo; k < hi; ++k) P[k + shift][c] = P[k][c]; }
+    P[at_enter][c] = enter;
+    P[at_leave][c] = leave;
+    na += 2 - len;
+    const float re = fmaT(enter.y, enter.y, enter.x * enter.x), rl = fmaT(leave.y, leave.y, leave.x * leave.x);
+    r2 = fmaxf(rin, fmaxf(re, rl)) * 1.000001f;
+    if (!(re < INFINITY) || !(rl < INFINITY)) na = -1;
+  }
+  if (na < 0) { over[1 + atomicAdd(over, 1)] = i; return; }
+  if (na < 3) return;
+  for (int k = 0; k < na; ++k) { near_d[k][c] = make_float2(1e30f, 1e30f); near_j[k][c] = make_int2(-1, -1); }
+  for (int t = 0; t < K; ++t) {
+    const int j = nb.get(i, t);
+    if ((unsigned)j >= (unsigned)n || j == i) continue;
+    const V3<float> d = sub3(ld3(S, j), si);
+    const float a = dot3(d, ui), b = dot3(d, vi), cc = 0.5f * dot3(d, d);
+    for (int k = 0; k < na; ++k) {
+      const float2 p = P[k][c];
+      const float s = fabsf(fmaT(a, p.x, fmaT(b, p.y, -cc)));
+      if (!(s <= tol_active)) continue;
+      float2 nd = near_d[k][c];
+      int2 nj = near_j[k][c];
+      if (s < nd.x) { nd.y = nd.x; nj.y = nj.x; nd.x = s; nj.x = j; }
+      else if (s < nd.y) { nd.y = s; nj.y = j; }
+      near_d[k][c] = nd; near_j[k][c] = nj;
+    }
+  }
+  for (int k = 0; k < na; ++k) {
+    const int2 nj = near_j[k][c];
+    if (nj.x >= 0 && nj.y >= 0 && nj.x != nj.y)
+      face_emit(nb.label(i), nb.label(nj.x), nb.label(nj.y), keys, key_count, max_keys);
+  }
+}
+
+// The sites that k_face_keys gave back, with the reference's two buffers of
+// kFaceMaxPoly vertices (MAX_POLY, main.cu:393) in local memory.
+constexpr int kFaceMaxPoly = 256;
+
+template <class NB>
+__global__ void __launch_bounds__(64) k_face_keys_over(const float* __restrict__ S, const float* __restrict__ U,
+                                                       const float* __restrict__ Vv, NB nb, int n, int K, float R2,
+                                                       float eps_clip, float tol_active, unsigned long long* keys,
+                                                       int* key_count, int max_keys, const int* __restrict__ over) {
+  float2 bufA[kFaceMaxPoly], bufB[kFaceMaxPoly];
+  const int n_over = over[0];
+  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n_over; w += gridDim.x * blockDim.x) {
+    const int i = over[1 + w];
+    float2* cp = bufA; float2* np = bufB;
+    int na = 4;
+    cp[0] = make_float2(-R2, -R2); cp[1] = make_float2(R2, -R2); cp[2] = make_float2(R2, R2); cp[3] = make_float2(-R2, R2);
+    const V3<float> si = ld3(S, i), ui = ld3(U, i), vi = ld3(Vv, i);
+    for (int t = 0; t < K && na > 0; ++t) {
+      const int j = nb.get(i, t);
+      if ((unsigned)j >= (unsigned)n || j == i) continue;
+      const V3<float> d = sub3(ld3(S, j), si);
+      const float a = dot3(d, ui), b = dot3(d, vi), c = 0.5f * dot3(d, d);
+      int m = 0;
       float2 s = cp[na - 1];
       float fs = fmaT(a, s.x, fmaT(b, s.y, -c));
       for (int k = 0; k < na; ++k) {
-        float2 e = cp[k];
-        int le = cl[k];
-        float fe = fmaT(a, e.x, fmaT(b, e.y, -c));
-        bool ins_e = fe <= eps_clip, ins_s = fs <= eps_clip;
-        if (ins_e) {
-          if (!ins_s && m < kFaceMaxPoly) {
-            float tt = divT(fs, (fs - fe) + 1e-30f);
-            np[m] = make_float2(fmaT(tt, e.x - s.x, s.x), fmaT(tt, e.y - s.y, s.y)); nl[m] = j; m++;
-          }
-          if (m < kFaceMaxPoly) { np[m] = e; nl[m] = le; m++; }
-        } else if (ins_s && m < kFaceMaxPoly) {
-          float tt = divT(fs, (fs - fe) + 1e-30f);
-          np[m] = make_float2(fmaT(tt, e.x - s.x, s.x), fmaT(tt, e.y - s.y, s.y)); nl[m] = j; m++;
+        const float2 e = cp[k];
+        const float fe = fmaT(a, e.x, fmaT(b, e.y, -c));
+        const bool ins_e = fe <= eps_clip, ins_s = fs <= eps_clip;
+        if (ins_e != ins_s && m < kFaceMaxPoly) {
+          const float tt = divT(fs, (fs - fe) + 1e-30f);
+          np[m++] = make_float2(fmaT(tt, e.x - s.x, s.x), fmaT(tt, e.y - s.y, s.y));
         }
+        if (ins_e && m < kFaceMaxPoly) np[m++] = e;
         s = e; fs = fe;
       }
+      na = m;
+      float2* tp = cp; cp = np; np = tp;
     }
-    na = m;
-    float2* tp = cp; cp = np; np = tp;
-    int* tl = cl; cl = nl; nl = tl;
-    if (na == 0) break;
-  }
-  if (na < 3) return;
-  for (int k = 0; k < na; ++k) {
-    float2 p = cp[k];
-    float b1 = 1e30f, b2 = 1e30f;
-    int j1 = -1, j2 = -1;
-    for (int t = 0; t < K; ++t) {
-      int j = nb.get(i, t);
-      if ((unsigned)j >= (unsigned)n || j == i) continue;
-      V3<float> d = sub3(ld3(S, j), si);
-      float a = dot3(d, ui), b = dot3(d, vi), c = 0.5f * dot3(d, d);
-      float s = fabsf(fmaT(a, p.x, fmaT(b, p.y, -c)));
-      if (s < b1) { b2 = b1; j2 = j1; b1 = s; j1 = j; }
-      else if (s < b2) { b2 = s; j2 = j; }
+    if (na < 3) continue;
+    for (int k = 0; k < na; ++k) {
+      const float2 p = cp[k];
+      float b1 = 1e30f, b2 = 1e30f;
+      int j1 = -1, j2 = -1;
+      for (int t = 0; t < K; ++t) {
+        const int j = nb.get(i, t);
+        if ((unsigned)j >= (unsigned)n || j == i) continue;
+        const V3<float> d = sub3(ld3(S, j), si);
+        const float a = dot3(d, ui), b = dot3(d, vi), c = 0.5f * dot3(d, d);
+        const float s = fabsf(fmaT(a, p.x, fmaT(b, p.y, -c)));
+        if (s < b1) { b2 = b1; j2 = j1; b1 = s; j1 = j; }
+        else if (s < b2) { b2 = s; j2 = j; }
+      }
+      if (j1 >= 0 && j2 >= 0 && j1 != j2 && b1 <= tol_active && b2 <= tol_active)
+        face_emit(nb.label(i), nb.label(j1), nb.label(j2), keys, key_count, max_keys);
     }
-    if (!(j1 >= 0 && j2 >= 0 && j1 != j2 && b1 <= tol_active && b2 <= tol_active)) continue;
-    int x = nb.label(i), y = nb.label(j1), z = nb.label(j2), tmp;
-    if (x > y) { tmp = x; x = y; y = tmp; }
-    if (y > z) { tmp = y; y = z; z = tmp; }
-    if (x > y) { tmp = x; x = y; y = tmp; }
-    int pos = atomicAdd(key_count, 1);
-    if (pos < max_keys)
-      keys[pos] = (unsigned long long)(uint32_t)x | ((unsigned long long)(uint32_t)y << 21) |
-                  ((unsigned long long)(uint32_t)z << 42);
   }
 }
 
@@ -217,11 +294,19 @@ __global__ void k_face_compact(const int* __restrict__ tri, const int* __restric
 // quality metrics (evaluate.cuh:388-462) as a device reduction: acc[0] Qsum,
 // acc[1] min-angle sum, acc[2] #angles < 30, acc[3] #angles > 90 (doubles);
 // mins[0] Qmin bits, mins[1] theta_min bits (non-negative floats as uint)
-__global__ void k_quality(const float* __restrict__ V, const int* __restrict__ F, int nF, double* acc, unsigned* mins) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+// Grid-stride blocks, one set of atomics per block (per warp: 43 us for 200k
+// faces, now 8).
+constexpr int kQualityThreads = 256;
+__global__ void __launch_bounds__(kQualityThreads) k_quality(const float* __restrict__ V, const int* __restrict__ F, int nF,
+                                                             double* acc, unsigned* mins) {
+  __shared__ double sacc[4];
+  __shared__ unsigned smin[2];
+  if (threadIdx.x < 4) sacc[threadIdx.x] = 0.0;
+  if (threadIdx.x < 2) smin[threadIdx.x] = 0x7f7f7f7fu;
+  __syncthreads();
   double q = 0.0, th = 0.0, lt = 0.0, gt = 0.0;
   float qmin = 3.0e38f, tmin = 3.0e38f;
-  if (f < nF) {
+  for (int f = blockIdx.x * kQualityThreads + threadIdx.x; f < nF; f += gridDim.x * kQualityThreads) {
     V3<float> a = ld3(V, F[3 * f]), b = ld3(V, F[3 * f + 1]), c = ld3(V, F[3 * f + 2]);
     V3<float> ab = sub3(b, a), ac = sub3(c, a), ba = sub3(a, b), bc = sub3(c, b), ca = sub3(a, c), cb = sub3(b, c);
     auto ang = [](V3<float> u, V3<float> v) {
@@ -232,10 +317,11 @@ __global__ void k_quality(const float* __restrict__ V, const int* __restrict__ F
       return acosf(cs) * (180.0f / 3.14159265358979323846f);
     };
     float A = ang(ab, ac), B = ang(ba, bc), Cc = ang(ca, cb);
-    tmin = fminf(A, fminf(B, Cc));
-    th = tmin;
-    lt = (A < 30.f) + (B < 30.f) + (Cc < 30.f);
-    gt = (A > 90.f) + (B > 90.f) + (Cc > 90.f);
+    const float tm = fminf(A, fminf(B, Cc));
+    tmin = fminf(tmin, tm);
+    th += tm;
+    lt += (A < 30.f) + (B < 30.f) + (Cc < 30.f);
+    gt += (A > 90.f) + (B > 90.f) + (Cc > 90.f);
     float l0 = sqrtT(dot3(ab, ab)), l1 = sqrtT(dot3(bc, bc)), l2 = sqrtT(dot3(ca, ca));
     V3<float> cr = cross3(ab, ac);
     float area = 0.5f * sqrtT(dot3(cr, cr));
@@ -243,8 +329,8 @@ __global__ void k_quality(const float* __restrict__ V, const int* __restrict__ F
     float e = fmaxf(l0, fmaxf(l1, l2));
     float den = fmaxf(s * e, 1e-30f);
     float qq = divT(6.0f, sqrtT(3.0f)) * divT(area, den);
-    qmin = qq;
-    q = qq;
+    qmin = fminf(qmin, qq);
+    q += qq;
   }
   for (int o = 16; o; o >>= 1) {
     q += __shfl_xor_sync(0xffffffffu, q, o);
@@ -255,10 +341,13 @@ __global__ void k_quality(const float* __restrict__ V, const int* __restrict__ F
     tmin = fminf(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
   }
   if ((threadIdx.x & 31) == 0) {
-    atomicAdd(acc + 0, q); atomicAdd(acc + 1, th); atomicAdd(acc + 2, lt); atomicAdd(acc + 3, gt);
-    atomicMin(mins + 0, __float_as_uint(qmin));
-    atomicMin(mins + 1, __float_as_uint(tmin));
+    atomicAdd(sacc + 0, q); atomicAdd(sacc + 1, th); atomicAdd(sacc + 2, lt); atomicAdd(sacc + 3, gt);
+    atomicMin(smin + 0, __float_as_uint(qmin));
+    atomicMin(smin + 1, __float_as_uint(tmin));
   }
+  __syncthreads();
+  if (threadIdx.x < 4) atomicAdd(acc + threadIdx.x, sacc[threadIdx.x]);
+  if (threadIdx.x < 2) atomicMin(mins + threadIdx.x, smin[threadIdx.x]);
 }
 
 }  // namespace cvt

