@@ -198,6 +198,7 @@ struct PointGrid {
   int* part = nullptr;
   int2* cellrank = nullptr;
   Pt4<float>* sorted = nullptr;
+  int* rest = nullptr;  // stage searches: [0] = count, queries left to k_stage_knn_warp
   int total_cells = 0;  // scan length (spatial capacity + NaN bucket)
 };
 
@@ -253,7 +254,7 @@ template <int KK>
 static void launch_knn_query(const PointGrid& pg, const float* Q, int nQ, const uint8_t* frozen, int kk, int ex,
                              uint32_t* knn, float* dist, cudaStream_t st) {
   k_stage_knn_query<KK><<<cdiv(nQ, 128), 128, 0, st>>>(pg.geom, pg.cell_start, pg.sorted, Q, nQ, frozen, kk, ex, knn,
-                                                       dist);
+                                                       dist, pg.rest);
 }
 
 #define KK_DISPATCH(kk, FN, ...)                                 \
@@ -268,6 +269,68 @@ static void launch_knn_query(const PointGrid& pg, const float* Q, int nQ, const 
     else FN<64>(__VA_ARGS__);                                    \
   } while (0)
 
+// one warp per query: all n of them, or those listed in rest
+static void launch_knn_warp(const PointGrid& pg, const float* Q, int n, const int* rest, const uint8_t* frozen, int kk,
+                            int ex, uint32_t* knn, float* dist, cudaStream_t st) {
+  const int blocks = std::min(cdiv(n, 4), 8 * sm_count());
+  if (kk <= 32)
+    k_stage_knn_warp<1><<<blocks, 128, 0, st>>>(pg.geom, pg.cell_start, pg.sorted, Q, n, rest, frozen, kk, ex, knn, dist);
+  else
+    k_stage_knn_warp<2><<<blocks, 128, 0, st>>>(pg.geom, pg.cell_start, pg.sorted, Q, n, rest, frozen, kk, ex, knn, dist);
+}
+
+// Which search: one warp per query for up to kWarpPoints points or kWarpQueries
+// queries; more points with 10 to 40 neighbours each go in groups of 32, the
+// rest one thread each with its list in registers.  Measured, warp against the
+// other (us): 2k points, K = 21: 13, 67 (thread); 30k, K = 25: 73, 129
+// (group); 100k: about 240, 169 (group; thread 178); 1M, K = 33: group 1424,
+// thread 2174.  5 nearest of 250k vertices for 2k queries: 14, 135 (thread);
+// 30k: 60, 94; 60k: 112, 93.
+constexpr int kWarpPoints = 60000;
+constexpr int kWarpQueries = 50000;
+
+// the points' own neighbours; pg.rest[0] is zero
+static cvt_status_t launch_knn_sites(const PointGrid& pg, int n, const uint8_t* frozen, int kk, uint32_t* knn, float* dist,
+                                     cudaStream_t st) {
+  if (n < kWarpPoints) {
+    launch_knn_warp(pg, nullptr, n, nullptr, frozen, kk, 0, knn, dist, st);
+    CKLAUNCH();
+    return CVT_OK;
+  }
+  if (kk < 10 || kk > 40) {
+    if (kk <= 1) launch_knn_points<1>(pg, n, frozen, kk, knn, dist, st);
+    else if (kk <= 5) launch_knn_points<5>(pg, n, frozen, kk, knn, dist, st);
+    else if (kk <= 9) launch_knn_points<9>(pg, n, frozen, kk, knn, dist, st);
+    else launch_knn_points<64>(pg, n, frozen, kk, knn, dist, st);
+    CKLAUNCH();
+    return CVT_OK;
+  }
+  k_stage_knn_group<<<std::min(cdiv(n, 32), 20 * sm_count()), 32, 0, st>>>(pg.geom, pg.cell_start, pg.sorted, n, frozen, kk,
+                                                                          knn, dist, pg.rest);
+  CKLAUNCH();
+  launch_knn_warp(pg, nullptr, n, pg.rest, frozen, kk, 0, knn, dist, st);
+  CKLAUNCH();
+  return CVT_OK;
+}
+
+// the neighbours of nQ query points among n points
+static cvt_status_t launch_knn_queries(Scratch& sc, PointGrid& pg, const float* Q, int nQ, const uint8_t* frozen, int kk,
+                                       int ex, uint32_t* knn, float* dist) {
+  cudaStream_t st = sc.st;
+  if (nQ < kWarpQueries) {
+    launch_knn_warp(pg, Q, nQ, nullptr, frozen, kk, ex, knn, dist, st);
+    CKLAUNCH();
+    return CVT_OK;
+  }
+  CK(sc.get(&pg.rest, (size_t)nQ + 1));
+  CK(cudaMemsetAsync(pg.rest, 0, sizeof(int), st));
+  KK_DISPATCH(kk, launch_knn_query, pg, Q, nQ, frozen, kk, ex, knn, dist, st);
+  CKLAUNCH();
+  launch_knn_warp(pg, Q, nQ, pg.rest, frozen, kk, ex, knn, dist, st);
+  CKLAUNCH();
+  return CVT_OK;
+}
+
 extern "C" cvt_status_t cvt_knn_sites(const float* pts, int n, int kk, const uint8_t* frozen, uint32_t* knn,
                                       float* dist, void* stream) {
   if (n < 0 || kk < 1 || kk > 64 || (n > 0 && (!pts || !knn))) return fail(CVT_ERR_INVALID, "cvt_knn_sites: bad arguments");
@@ -277,9 +340,9 @@ extern "C" cvt_status_t cvt_knn_sites(const float* pts, int n, int kk, const uin
   PointGrid pg;
   cvt_status_t s = build_point_grid(sc, pts, n, 0.2f * kk, nullptr, pg);
   if (s != CVT_OK) return s;
-  KK_DISPATCH(kk, launch_knn_points, pg, n, frozen, kk, knn, dist, st);
-  CKLAUNCH();
-  return CVT_OK;
+  CK(sc.get(&pg.rest, (size_t)n + 1));
+  CK(cudaMemsetAsync(pg.rest, 0, sizeof(int), st));
+  return launch_knn_sites(pg, n, frozen, kk, knn, dist, st);
 }
 
 extern "C" cvt_status_t cvt_knn_query_to_points(const float* cand, int n_cand, const float* query, int n_query, int kk,
@@ -292,9 +355,7 @@ extern "C" cvt_status_t cvt_knn_query_to_points(const float* cand, int n_cand, c
   PointGrid pg;
   cvt_status_t s = build_point_grid(sc, cand, n_cand, 0.2f * kk + 1.f, nullptr, pg);
   if (s != CVT_OK) return s;
-  KK_DISPATCH(kk, launch_knn_query, pg, query, n_query, frozen, kk, 0, knn, dist, st);
-  CKLAUNCH();
-  return CVT_OK;
+  return launch_knn_queries(sc, pg, query, n_query, frozen, kk, 0, knn, dist);
 }
 
 extern "C" cvt_status_t cvt_knn_vertices(const float* V, int nV, const float* Q, int nQ, int k, int exclude_self,
@@ -308,10 +369,7 @@ extern "C" cvt_status_t cvt_knn_vertices(const float* V, int nV, const float* Q,
   cvt_status_t s = build_point_grid(sc, V, nV, 0.2f * k + 1.f, nullptr, pg);
   if (s != CVT_OK) return s;
   // int output: the uint32 sentinel 0xFFFFFFFF reads as -1
-  KK_DISPATCH(k, launch_knn_query, pg, Q, nQ, frozen, k, exclude_self ? 1 : 0, reinterpret_cast<uint32_t*>(out),
-              (float*)nullptr, st);
-  CKLAUNCH();
-  return CVT_OK;
+  return launch_knn_queries(sc, pg, Q, nQ, frozen, k, exclude_self ? 1 : 0, reinterpret_cast<uint32_t*>(out), nullptr);
 }
 
 extern "C" cvt_status_t cvt_knn_drop_self(const uint32_t* in, int n, int kin, int kout, uint32_t* out, void* stream) {

@@ -10,12 +10,12 @@
 // (or fail with out-of-memory halfway through) is not acceptable.  This
 // variant keeps every temporary of the search (bounding box, grid geometry,
 // cell counts and starts, scan partials, per-point cell ranks, the
-// cell-ordered point copy) in one fixed array compiled into the library.
+// cell-ordered point copy, the list of left-over queries) in one fixed array compiled into the library.
 //
 // Limits and rules:
 //   * at most CVT_NOALLOC_MAX_POINTS points per call (larger calls return
 //     CVT_ERR_CAPACITY and do nothing);
-//   * the array (~5 MB) is held by every GPU that loads the library, until
+//   * the array (~5.5 MB) is held by every GPU that loads the library, until
 //     the process exits;
 //   * all calls share that one array: calls whose work overlaps on the GPU
 //     (different streams, or different host threads without ordering) race
@@ -42,7 +42,8 @@ constexpr size_t kOffStart = up256(kOffCount + (size_t)(kCap + 1) * sizeof(int))
 constexpr size_t kOffPart = up256(kOffStart + (size_t)(kCap + 2) * sizeof(int));
 constexpr size_t kOffRank = up256(kOffPart + kScanParts * sizeof(int));
 constexpr size_t kOffSorted = up256(kOffRank + (size_t)kMaxPoints * sizeof(int2));
-constexpr size_t kBytes = up256(kOffSorted + (size_t)kMaxPoints * sizeof(Pt4<float>));
+constexpr size_t kOffRest = up256(kOffSorted + (size_t)kMaxPoints * sizeof(Pt4<float>));
+constexpr size_t kBytes = up256(kOffRest + (size_t)(kMaxPoints + 1) * sizeof(int));
 
 }  // namespace noalloc
 
@@ -92,6 +93,7 @@ extern "C" cvt_status_t cvt_knn_sites_noalloc(const float* pts, int n, int kk, c
   pg.part = reinterpret_cast<int*>(b + noalloc::kOffPart);
   pg.cellrank = reinterpret_cast<int2*>(b + noalloc::kOffRank);
   pg.sorted = reinterpret_cast<Pt4<float>*>(b + noalloc::kOffSorted);
+  pg.rest = reinterpret_cast<int*>(b + noalloc::kOffRest);
   const int cap = std::max(64, 2 * n);
   pg.total_cells = cap + 1;
   // the array keeps the previous call's contents: the bounding box and the
@@ -103,6 +105,7 @@ extern "C" cvt_status_t cvt_knn_sites_noalloc(const float* pts, int n, int kk, c
   k_grid_geom<<<1, 32, 0, st>>>(bb, n, 0.2f * kk, cap, pg.geom);
   CKLAUNCH();
   CK(cudaMemsetAsync(pg.cell_count, 0, sizeof(int) * pg.total_cells, st));
+  CK(cudaMemsetAsync(pg.rest, 0, sizeof(int), st));
   k_grid_count<float><<<cdiv(n, 256), 256, 0, st>>>(n, pts, SegGrid{pg.geom, nullptr, nullptr}, pg.cell_count, pg.cellrank);
   CKLAUNCH();
   launch_exclusive_scan(pg.total_cells, pg.cell_count, pg.part, pg.cell_start, st);
@@ -110,7 +113,5 @@ extern "C" cvt_status_t cvt_knn_sites_noalloc(const float* pts, int n, int kk, c
   CK(cudaGetLastError());
   k_grid_scatter<float><<<cdiv(n, 256), 256, 0, st>>>(n, pts, pg.cellrank, pg.cell_start, pg.sorted);
   CKLAUNCH();
-  KK_DISPATCH(kk, launch_knn_points, pg, n, frozen, kk, knn, dist, st);
-  CKLAUNCH();
-  return CVT_OK;
+  return launch_knn_sites(pg, n, frozen, kk, knn, dist, st);
 }

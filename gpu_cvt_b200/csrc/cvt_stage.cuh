@@ -3,6 +3,7 @@
 // device routines of the fused engine.
 #pragma once
 #include "cvt_engine.cuh"
+#include "cvt_knn.cuh"
 
 namespace cvt {
 
@@ -104,24 +105,131 @@ __global__ void __launch_bounds__(128) k_stage_knn_points(const GridGeom* geom, 
   }
 }
 
-// queries are separate points; out_int != 0 writes int (-1 for missing)
+// queries are separate points; out_int != 0 writes int (-1 for missing).  A
+// query that has not ended after kQueryRings rings is far from the points (a
+// centroid of an unbounded cell: its thread would walk the whole grid, several
+// milliseconds) and is left to k_stage_knn_warp: rest[0] = count, then queries.
+constexpr int kQueryRings = 4;
 template <int KK>
 __global__ void __launch_bounds__(128) k_stage_knn_query(const GridGeom* geom, const int* __restrict__ cell_start,
                                                          const Pt4<float>* __restrict__ sorted, const float* __restrict__ Q,
                                                          int nQ, const uint8_t* frozen, int kk, int exclude_self,
-                                                         uint32_t* knn, float* dist) {
+                                                         uint32_t* knn, float* dist, int* __restrict__ rest) {
   const int qi = blockIdx.x * blockDim.x + threadIdx.x;
   if (qi >= nQ) return;
   if (frozen && frozen[qi]) return;
   TopK<float, KK> top;
   const GridGeom G = *geom;
   const int skip = exclude_self ? qi : -1;
-  grid_knn<float, float, KK>(G, cell_start, sorted, ld3(Q, qi), top, [skip](uint32_t id) { return (int)id != skip; });
+  if (!grid_knn<float, float, KK>(G, cell_start, sorted, ld3(Q, qi), top, [skip](uint32_t id) { return (int)id != skip; },
+                                  kQueryRings)) {
+    rest[1 + atomicAdd(rest, 1)] = qi;
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < KK; ++k) {
     if (k >= kk) break;
     knn[(size_t)qi * kk + k] = KeyOps<float>::idx(top.k[k]);
     if (dist) dist[(size_t)qi * kk + k] = KeyOps<float>::dist(top.k[k]);
+  }
+}
+
+// One warp per query (kk <= 32 R): the queries of `rest` ([0] = count), or with
+// rest == NULL all n.  Q == NULL: query w is the w-th of the cell-ordered
+// points.  Few queries (one thread each would leave most of the chip idle for
+// the length of one thread's search) and those that the other kernels leave.
+template <int R>
+__global__ void __launch_bounds__(128) k_stage_knn_warp(const GridGeom* geom, const int* __restrict__ cell_start,
+                                                        const Pt4<float>* __restrict__ sorted, const float* __restrict__ Q,
+                                                        int n, const int* __restrict__ rest, const uint8_t* frozen, int kk,
+                                                        int exclude_self, uint32_t* knn, float* dist) {
+  const int lane = threadIdx.x & 31;
+  const int nw = (int)((gridDim.x * 128u) >> 5);
+  const GridGeom G = *geom;
+  const int n_pts = __ldg(cell_start + G.cell_base + G.ncell);  // without the non-finite ones
+  const int count = rest ? rest[0] : n;
+  for (int w = (int)((blockIdx.x * 128u + threadIdx.x) >> 5); w < count; w += nw) {
+    const int i = rest ? rest[1 + w] : w;
+    V3<float> q;
+    int row = i, skip = -1;
+    if (Q) {
+      q = ld3(Q, i);
+      if (exclude_self) skip = i;
+    } else {
+      const Pt4<float> me = sorted[i];
+      q = {me.x, me.y, me.z};
+      row = (int)me.id;
+    }
+    if (frozen && frozen[row]) continue;
+    unsigned long long list[R];
+    warp_knn_k<float, float, R>(G, cell_start, sorted, n_pts, q, kk, lane, [skip](uint32_t id) { return (int)id != skip; },
+                                Q ? kQueryRings : 0, list);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int e = 32 * r + lane;
+      if (e < kk) {
+        knn[(size_t)row * kk + e] = KeyOps<float>::idx(list[r]);
+        if (dist) dist[(size_t)row * kk + e] = KeyOps<float>::dist(list[r]);
+      }
+    }
+  }
+}
+
+// Many points with 10 to 40 neighbours each: one warp per 32 consecutive
+// points of the cell order (group_knn), rows written by the whole warp.  The
+// radius is expected to hold 1.3 kk points at the density of the 27 cells
+// around the point (a surface crosses about eleven cells' worth of area
+// there).  Left to k_stage_knn_warp: points whose radius holds too few or more
+// than 64, and non-finite ones.
+__global__ void __launch_bounds__(32, 20) k_stage_knn_group(const GridGeom* geom, const int* __restrict__ cell_start,
+                                                        const Pt4<float>* __restrict__ sorted, int n, const uint8_t* frozen,
+                                                        int kk, uint32_t* __restrict__ knn, float* __restrict__ dist,
+                                                        int* __restrict__ rest) {
+  __shared__ GroupPlaces L;
+  const int lane = threadIdx.x;
+  const GridGeom G = *geom;
+  for (int t0 = blockIdx.x * 32; t0 < n; t0 += gridDim.x * 32) {
+    const int t = t0 + lane;
+    Pt4<float> me{};
+    bool in = t < n;
+    if (in) {
+      me = sorted[t];
+      if (frozen && frozen[me.id]) in = false;
+    }
+    const V3<float> q{me.x, me.y, me.z};
+    float thr = 0.f, rad = 0.f;
+    if (in && finite3(q)) {
+      const int c[3] = {grid_coord(G, q.x, 0), grid_coord(G, q.y, 1), grid_coord(G, q.z, 2)};
+      const int x0 = max(c[0] - 1, 0), x1 = min(c[0] + 1, G.dim[0] - 1);
+      int near = 0;
+      for (int z = max(c[2] - 1, 0); z <= min(c[2] + 1, G.dim[2] - 1); ++z)
+        for (int y = max(c[1] - 1, 0); y <= min(c[1] + 1, G.dim[1] - 1); ++y) {
+          const int row = G.cell_base + (z * G.dim[1] + y) * G.dim[0];
+          near += __ldg(cell_start + row + x1 + 1) - __ldg(cell_start + row + x0);
+        }
+      thr = (1.3f * 11.f / 3.14159265f) * (float)kk * G.h * G.h / (float)near;
+      rad = query_radius(G, q, thr);
+    }
+    const bool ok = group_knn<float, float>(G, 0, cell_start, sorted, in, q, thr, rad, 0xffffffffu, kk, L);
+    const unsigned left = __ballot_sync(0xffffffffu, in && !ok);
+    if (left) {
+      int base = 0;
+      if (lane == 0) base = atomicAdd(rest, __popc(left));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (in && !ok) rest[1 + base + __popc(left & ((1u << lane) - 1u))] = t;
+    }
+    for (unsigned rows = __ballot_sync(0xffffffffu, ok); rows; rows &= rows - 1) {
+      const int src = __ffs(rows) - 1;
+      const V3<float> qs{__shfl_sync(0xffffffffu, q.x, src), __shfl_sync(0xffffffffu, q.y, src),
+                         __shfl_sync(0xffffffffu, q.z, src)};
+      const size_t row = (size_t)__shfl_sync(0xffffffffu, me.id, src) * kk;
+      for (int e = lane; e < kk; e += 32) {
+        const Pt4<float> p = sorted[L.at[e][src]];
+        knn[row + e] = p.id;
+        if (dist) dist[row + e] = dist2(V3<float>{p.x, p.y, p.z}, qs);
+      }
+    }
+    __syncwarp();
   }
 }
 
