@@ -108,14 +108,30 @@ static cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t st) {
   return cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, st);
 }
 
+// Held while an iteration is captured and its graph instantiated or updated,
+// and around every device-wide wait and release of this library: with one
+// thread capturing and another waiting for the device, tearing an engine down
+// or ending (its streams go), the driver failed the capture or crashed (two
+// threads that create, run and destroy engines: within 150 rounds).
+static std::mutex g_capture_mu;
+
+static cudaError_t device_sync() {
+  std::lock_guard<std::mutex> lk(g_capture_mu);
+  return cudaDeviceSynchronize();
+}
+
 // long-lived objects: allocated and freed on the legacy stream, then waited for
 static cudaError_t dev_alloc_sync(void** p, size_t bytes) {
+  std::lock_guard<std::mutex> lk(g_capture_mu);
   cudaError_t e = dev_alloc(p, bytes, 0);
   if (e == cudaSuccess) e = cudaStreamSynchronize(0);
   return e;
 }
 static void dev_free_sync(void* p) {
-  if (p) { cudaFreeAsync(p, 0); cudaStreamSynchronize(0); }
+  if (!p) return;
+  std::lock_guard<std::mutex> lk(g_capture_mu);
+  cudaFreeAsync(p, 0);
+  cudaStreamSynchronize(0);
 }
 
 static void graph_cache_clear();
@@ -156,6 +172,7 @@ struct ThreadStreams {
 struct ThreadStreamSet {
   std::vector<ThreadStreams> dev;
   ~ThreadStreamSet() {
+    std::lock_guard<std::mutex> lk(g_capture_mu);
     for (ThreadStreams& t : dev)
       for (cudaStream_t s : {t.side, t.cap, t.cap_side})
         if (s) cudaStreamDestroy(s);
@@ -168,6 +185,8 @@ static cudaError_t thread_streams(ThreadStreams** out) {
   if (e != cudaSuccess) return e;
   if ((int)set.dev.size() <= d) set.dev.resize(d + 1);
   ThreadStreams& t = set.dev[d];
+  if (t.side && t.cap && t.cap_side) { *out = &t; return cudaSuccess; }
+  std::lock_guard<std::mutex> lk(g_capture_mu);
   for (cudaStream_t* s : {&t.side, &t.cap, &t.cap_side})
     if (!*s && (e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking)) != cudaSuccess) return e;
   *out = &t;
@@ -911,7 +930,7 @@ extern "C" cvt_status_t cvt_mesh_device_arrays(cvt_mesh_t m, const float** V, co
 
 extern "C" cvt_status_t cvt_mesh_destroy(cvt_mesh_t m) {
   if (!m) return CVT_OK;
-  cudaDeviceSynchronize();
+  device_sync();
   mesh_free(m);
   return CVT_OK;
 }
@@ -1305,10 +1324,13 @@ static cudaError_t graph_exec_for(const GraphKey& k, cudaGraph_t gr, cudaGraphEx
 
 static void engine_free(cvt_engine* e) {
   if (!e) return;
-  for (int k = 0; k < 2; ++k)
-    if (e->gexec[k]) graph_cache_put(graph_key(e), e->gexec[k]);
-  for (cudaEvent_t ev : {e->ev_fork, e->ev_grid, e->ev_join, e->ev_cfork, e->ev_cgrid, e->ev_cjoin})
-    if (ev) cudaEventDestroy(ev);
+  {
+    std::lock_guard<std::mutex> lk(g_capture_mu);
+    for (int k = 0; k < 2; ++k)
+      if (e->gexec[k]) graph_cache_put(graph_key(e), e->gexec[k]);
+    for (cudaEvent_t ev : {e->ev_fork, e->ev_grid, e->ev_join, e->ev_cfork, e->ev_cgrid, e->ev_cjoin})
+      if (ev) cudaEventDestroy(ev);
+  }
   dev_free_sync(e->arena);
   delete e;
 }
@@ -1418,7 +1440,7 @@ extern "C" cvt_status_t cvt_engine_create(const cvt_params_t* p, int max_segment
   ECK(cudaGetLastError());
   for (cudaEvent_t* ev : {&e->ev_fork, &e->ev_grid, &e->ev_join, &e->ev_cfork, &e->ev_cgrid, &e->ev_cjoin})
     ECK(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
-  ECK(cudaDeviceSynchronize());
+  ECK(device_sync());
 #undef ECK
   *out = e;
   return CVT_OK;
@@ -1426,7 +1448,7 @@ extern "C" cvt_status_t cvt_engine_create(const cvt_params_t* p, int max_segment
 
 extern "C" cvt_status_t cvt_engine_destroy(cvt_engine_t e) {
   if (!e) return CVT_OK;
-  cudaDeviceSynchronize();
+  device_sync();
   engine_free(e);
   return CVT_OK;
 }
@@ -1562,12 +1584,12 @@ static cvt_status_t place_all_segments(cvt_engine* e, const float* raw, int n, c
 
 extern "C" cvt_status_t cvt_engine_remove_segment(cvt_engine_t e, int s) {
   if (!e || s < 0 || s >= e->max_seg || !e->seg_mesh[s]) return fail(CVT_ERR_INVALID, "cvt_engine_remove_segment: bad segment");
-  CK(cudaDeviceSynchronize());
+  CK(device_sync());
   e->active[s] = 0;
   CK(cudaMemcpy(e->d_active + s, &e->active[s], sizeof(int), cudaMemcpyHostToDevice));
   k_fill_int<<<cdiv(e->segs[s].n_sites, 256), 256>>>(e->d_site_seg + e->segs[s].site_base, e->segs[s].n_sites, -1);
   CKLAUNCH();
-  CK(cudaDeviceSynchronize());
+  CK(device_sync());
   e->site_alloc.give(e->segs[s].site_base, e->segs[s].n_sites);
   e->cell_alloc.give(e->geom[s].cell_base, e->seg_cells[s]);
   e->seg_mesh[s] = nullptr;
@@ -1808,6 +1830,7 @@ extern "C" cvt_status_t cvt_engine_run(cvt_engine_t e, int iters, void* stream) 
     for (int k = 0; k < e->max_seg; ++k) if (e->active[k] == 1) e->host_iters[k]++;
     if (capture) {
       int ng = 0;
+      std::lock_guard<std::mutex> lk(g_capture_mu);
       CK(cudaStreamBeginCapture(ts->cap, cudaStreamCaptureModeThreadLocal));
       cvt_status_t q = enqueue_iteration(e, par, ts->cap, Branch{ts->cap_side, e->ev_cfork, e->ev_cgrid, e->ev_cjoin}, &ng);
       cudaGraph_t gr = nullptr;
