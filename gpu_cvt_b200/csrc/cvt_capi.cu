@@ -1269,11 +1269,11 @@ struct cvt_engine {
 // destroys them.
 struct GraphKey {
   int dev, profile, k, knn_block, clip_block, proj_block, proj_mode, frame_mode;
-  bool knn_reuse;
+  bool knn_reuse, few;
   bool operator==(const GraphKey& o) const {
     return dev == o.dev && profile == o.profile && k == o.k && knn_block == o.knn_block &&
            clip_block == o.clip_block && proj_block == o.proj_block && proj_mode == o.proj_mode &&
-           frame_mode == o.frame_mode && knn_reuse == o.knn_reuse;
+           frame_mode == o.frame_mode && knn_reuse == o.knn_reuse && few == o.few;
   }
 };
 constexpr size_t kGraphCacheMax = 16;
@@ -1282,7 +1282,7 @@ static std::vector<std::pair<GraphKey, cudaGraphExec_t>> g_graph_cache;
 
 static GraphKey graph_key(const cvt_engine* e) {
   return {e->dev, e->p.profile, e->K, e->p.knn_block, e->p.clip_block, e->p.proj_block, e->p.proj_mode,
-          e->p.frame_mode, e->p.knn_reuse != 0};
+          e->p.frame_mode, e->p.knn_reuse != 0, e->cov_sites <= kFewSites};
 }
 
 static cudaGraphExec_t graph_cache_take(const GraphKey& k) {
@@ -1738,11 +1738,17 @@ static cvt_status_t enqueue_iteration_t(cvt_engine* e, int parity, cudaStream_t 
   launch_site_clip<PROF>(a, parity, ns, e->p.clip_block, e->p.frame_mode, e->num_sms, st);
   L += 2;
   if (ev) CK(cudaEventRecord(ev[3], st));
-  if (e->p.proj_mode == CVT_PROJ_ONERING) {
-    k_site_vsearch<PROF, 128><<<cdiv(ns, 128), 128, 0, st>>>(a, parity);
+  if (e->p.proj_mode == CVT_PROJ_ONERING && ns <= kFewSites) {
+    k_site_vsearch_lanes<PROF><<<cdiv((long)ns * kVsearchLanes, 128), 128, 0, st>>>(a, parity);
+    k_site_proj_lanes<PROF><<<cdiv((long)ns * kProjLanes, 128), 128, 0, st>>>(a, parity);
     L++;
+  } else {
+    if (e->p.proj_mode == CVT_PROJ_ONERING) {
+      k_site_vsearch<PROF, 128><<<cdiv(ns, 128), 128, 0, st>>>(a, parity);
+      L++;
+    }
+    launch_site_proj<PROF>(a, parity, ns, e->p.proj_block, e->p.proj_mode, st);
   }
-  launch_site_proj<PROF>(a, parity, ns, e->p.proj_block, e->p.proj_mode, st);
   k_site_far<PROF><<<e->num_sms, 128, 0, st>>>(a, parity, e->d_segs, e->d_active, e->max_seg, e->d_tickets + 1);
   L += 2;
   if (ev) CK(cudaEventRecord(ev[4], st));
@@ -1790,11 +1796,11 @@ static cvt_status_t cover_segments(cvt_engine* e, cudaStream_t st) {
   };
   const int cs = fit(ns, e->cov_sites, e->max_sites), cc = fit(nc, e->cov_cells, e->max_cells);
   if (cs == e->cov_sites && cc == e->cov_cells) return CVT_OK;
-  e->cov_sites = cs;
-  e->cov_cells = cc;
   if (e->gexec[0] || e->gexec[1]) CK(cudaStreamSynchronize(st));  // no replay in flight
   for (int k = 0; k < 2; ++k)
     if (e->gexec[k]) { graph_cache_put(graph_key(e), e->gexec[k]); e->gexec[k] = nullptr; }
+  e->cov_sites = cs;
+  e->cov_cells = cc;
   return CVT_OK;
 }
 

@@ -1081,6 +1081,11 @@ __global__ void __launch_bounds__(64) k_clip_overflow(EngineArgs<typename PT<PRO
     site_clip<PROF, FRAME, true>(a, parity, a.ovf[1 + k], PolyRef<PP>{buf[0], 1}, PolyRef<PP>{buf[1], 1}, kFallbackCap);
 }
 
+// The new position sn of site g, tiers and the freeze test.
+template <int PROF>
+__device__ __forceinline__ void site_settle(const EngineArgs<typename PT<PROF>::T>& a, int parity, int g,
+                                            V3<typename PT<PROF>::T> sn, SiteOut& o);
+
 // Projection, tiers and the freeze test of site g, given the centroid in
 // a.cent and (PROJ 0) its 5 nearest vertices knnv; PROJ 1 projects through
 // the mesh's BVH and ignores knnv.
@@ -1092,9 +1097,7 @@ __device__ __forceinline__ void site_finish(const EngineArgs<typename PT<PROF>::
   const int s = __ldg(a.site_seg + g);
   const SegDev& sd = a.segs[s];
   const MeshDev& md = a.meshes[sd.mesh];
-  const bool fz = sd.mode != 0 && a.frozen[g];
-  const Pt4<T> me = a.S[parity][g];
-  const V3<T> si{me.x, me.y, me.z};
+  const V3<T> si = ldp(a.S[parity], g);
   const V3<T> cent = ld3((const T*)a.cent, g);
 
   // projection
@@ -1106,6 +1109,19 @@ __device__ __forceinline__ void site_finish(const EngineArgs<typename PT<PROF>::
   } else if (!project_onering_rec<T, Q, BS>(cent, md.ring_head, md.ring_body, md.nV, md.vf_off, knnv, L, sn)) {
     sn = project_onering_plain<T, Q>(cent, md.V, md.nV, md.F, md.nF, md.vf_off, md.vf_faces, knnv, kKProj);
   }
+  site_settle<PROF>(a, parity, g, sn, o);
+}
+
+template <int PROF>
+__device__ __forceinline__ void site_settle(const EngineArgs<typename PT<PROF>::T>& a, int parity, int g,
+                                            V3<typename PT<PROF>::T> sn, SiteOut& o) {
+  using T = typename PT<PROF>::T;
+  const int s = __ldg(a.site_seg + g);
+  const SegDev& sd = a.segs[s];
+  const MeshDev& md = a.meshes[sd.mesh];
+  const bool fz = sd.mode != 0 && a.frozen[g];
+  const Pt4<T> me = a.S[parity][g];
+  const V3<T> si{me.x, me.y, me.z};
   a.S[parity ^ 1][g] = Pt4<T>{sn.x, sn.y, sn.z, me.id};
 
   // tiers on the segment's first iteration (modes 1/2)
@@ -1209,6 +1225,111 @@ __global__ void __launch_bounds__(BS, PROF == PROF_FP64 ? 1 : 1536 / BS) k_site_
   }
 #pragma unroll
   for (int k = 0; k < kKProj; ++k) kv[k * a.stride] = (int)KeyOps<T>::idx(top.k[k]);
+}
+
+// Few sites (a.n_sites <= kFewSites): the vertex search and the projection with
+// 8 lanes per site each, which shorten a site's chain of loads where one
+// thread each would leave most of the chip idle.  The same results: the lanes'
+// candidates are merged by the keys that one thread compares.  Iteration of a
+// lone segment on a 40k-face torus, lanes against threads (us, ref, K = 20):
+// 2k sites 62, 94; 8k 66, 94; 16k 70, 94; 30k 83, 94; 60k (16 lanes) 126, 98.
+// 16 lanes for the projection: 60 at 2k, 75 at 16k; 4 for the search: 79 at 2k.
+constexpr int kFewSites = 32768;
+constexpr int kVsearchLanes = 8;
+constexpr int kProjLanes = 8;
+
+template <int PROF>
+__global__ void __launch_bounds__(128) k_site_vsearch_lanes(EngineArgs<typename PT<PROF>::T> a, int parity) {
+  using T = typename PT<PROF>::T;
+  using O = KeyOps<T>;
+  using Key = typename O::Key;
+  constexpr unsigned full = 0xffffffffu;
+  const int g = (int)(blockIdx.x * 128u + threadIdx.x) / kVsearchLanes;
+  const int sub = threadIdx.x & (kVsearchLanes - 1);
+  const int s = active_seg(a, g);
+  const bool in = s >= 0 && !(a.segs[s].mode != 0 && a.frozen[g]);  // frozen sites keep their vertices
+  const MeshDev& md = a.meshes[in ? a.segs[s].mesh : 0];
+  int skip = -1;
+  V3<T> c{0, 0, 0};
+  T thr = (T)0;
+  bool ok = false;
+  if (in) {
+    const SegDev& sd = a.segs[s];
+    skip = (sd.mode == 0 && sd.ex_quirk) ? (int)a.S[parity][g].id - sd.site_base : -1;
+    c = ld3((const T*)a.cent, g);
+    ok = true;
+    if (sub < kKProj) {
+      const int v = a.knnv[sub * a.stride + g];
+      ok = (unsigned)v < (unsigned)md.nV && v != skip;
+      if (ok) thr = dist2(V3<T>{(T)__ldg(md.V + 3 * v), (T)__ldg(md.V + 3 * v + 1), (T)__ldg(md.V + 3 * v + 2)}, c);
+    }
+  }
+  // the box of k_site_vsearch: within the largest of the five distances
+#pragma unroll
+  for (int o = kVsearchLanes / 2; o > 0; o >>= 1) {
+    const T x = __shfl_xor_sync(full, thr, o);
+    thr = x > thr ? x : thr;
+  }
+  const unsigned group = ((1u << kVsearchLanes) - 1u) << (threadIdx.x & 31 & ~(kVsearchLanes - 1));
+  bool box = (__ballot_sync(full, ok) & group) == group && finite3(c) && thr >= (T)0;
+  TopK<T, kKProj> top;
+  if (box) {
+    const GridGeom& G = md.vg;
+    const float qf[3] = {(float)c.x, (float)c.y, (float)c.z};
+    const float qm = fmaxf(fabsf(qf[0]), fmaxf(fabsf(qf[1]), fabsf(qf[2])));
+    const float rad = __fsqrt_ru(f32_ru(thr)) * 1.0001f + 1e-3f * G.h + 4e-7f * qm;
+    int lo[3], hi[3];
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+      lo[ax] = grid_coord(G, __fsub_rd(qf[ax], rad), ax);
+      hi[ax] = grid_coord(G, __fadd_ru(qf[ax], rad), ax);
+    }
+    const int ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1;
+    box = rad < INFINITY && (hi[0] - lo[0] + 1) * ny * nz <= kVertexBoxCells;
+    if (box)
+      for (int r = sub; r < ny * nz; r += kVsearchLanes) {
+        const int row = G.cell_base + ((lo[2] + r / ny) * G.dim[1] + lo[1] + r % ny) * G.dim[0];
+        const int e = __ldg(md.vcell_start + row + hi[0] + 1);
+        for (int k = __ldg(md.vcell_start + row + lo[0]); k < e; ++k) {
+          const Pt4<float> p = md.vsorted[k];
+          if ((int)p.id == skip) continue;
+          const T d = dist2(V3<T>{(T)p.x, (T)p.y, (T)p.z}, c);
+          if (d <= thr && d <= top.worst_d()) top.insert(O::make(d, p.id));
+        }
+      }
+  }
+  // the group's five smallest keys, smallest first; the lane that holds one
+  // moves on to its next
+  Key out[kKProj];
+#pragma unroll
+  for (int k = 0; k < kKProj; ++k) {
+    Key m = top.k[0];
+#pragma unroll
+    for (int o = kVsearchLanes / 2; o > 0; o >>= 1) m = O::kmin(m, shfl_xor_key(m, o));
+    out[k] = m;
+    if (!O::less(m, top.k[0])) {
+#pragma unroll
+      for (int j = 0; j + 1 < kKProj; ++j) top.k[j] = top.k[j + 1];
+      top.k[kKProj - 1] = O::empty();
+    }
+  }
+  if (!in) return;
+  if (!(box && !O::is_empty(out[kKProj - 1]))) {
+    if (sub != 0) return;
+    top = TopK<T, kKProj>();
+    if (!grid_knn<T, float, kKProj>(md.vg, md.vcell_start, md.vsorted, c, top,
+                                    [skip](uint32_t id) { return (int)id != skip; }, kVertexRingLimit)) {
+      a.far[1 + atomicAdd(a.far, 1)] = g;
+      a.knnv[g] = kVertexDeferred;
+      return;
+    }
+#pragma unroll
+    for (int k = 0; k < kKProj; ++k) a.knnv[k * a.stride + g] = (int)O::idx(top.k[k]);
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < kKProj; ++k)
+    if (sub == k) a.knnv[k * a.stride + g] = (int)O::idx(out[k]);
 }
 
 // Everything after the centroid and (PROJ 0) the vertex search of
@@ -1328,6 +1449,43 @@ __global__ void __launch_bounds__(BS, PROJ == 0 ? 768 / BS : 1) k_site_proj(Engi
   SiteOut o{-1, 0, 0, 0, 0, 0.f};
   if (active_seg(a, g) >= 0) site_proj<PROF, PROJ>(a, parity, g, rings, o);
   if (a.blockmax) motion_to_block(a, parity, g, o);
+  stats_flush(a.stats, a.segs, o, stage);
+  __syncthreads();
+  stats_stage_flush(a.stats, a.segs, stage);
+}
+
+// k_site_proj (one-ring) with kProjLanes lanes per site; the first lane of a
+// site does what follows its projection.
+template <int PROF>
+__global__ void __launch_bounds__(128) k_site_proj_lanes(EngineArgs<typename PT<PROF>::T> a, int parity) {
+  using T = typename PT<PROF>::T;
+  using Q = typename PT<PROF>::Q;
+  __shared__ StatsStage stage;
+  stats_stage_init(stage);
+  __syncthreads();
+  const int g = (int)(blockIdx.x * 128u + threadIdx.x) / kProjLanes;
+  const int s = active_seg(a, g);
+  const MeshDev& md = a.meshes[s >= 0 ? a.segs[s].mesh : 0];
+  int knnv[kKProj] = {-1, -1, -1, -1, -1};
+  V3<T> cent{0, 0, 0};
+  bool in = s >= 0;
+  if (in) {
+#pragma unroll
+    for (int k = 0; k < kKProj; ++k) knnv[k] = a.knnv[k * a.stride + g];
+    in = knnv[0] != kVertexDeferred;
+    cent = ld3((const T*)a.cent, g);
+    if (!in || (PROF == PROF_MIXED && !finite3(cent)))
+#pragma unroll
+      for (int k = 0; k < kKProj; ++k) knnv[k] = -1;
+  }
+  V3<T> sn = project_onering_lanes<T, Q, kProjLanes>(cent, md.ring_head, md.ring_body, md.nV, md.vf_off, knnv);
+  SiteOut o{-1, 0, 0, 0, 0, 0.f};
+  const bool lead = in && (threadIdx.x & (kProjLanes - 1)) == 0;
+  if (lead) {
+    if (PROF == PROF_MIXED && !finite3(cent)) sn = ldp(a.S[parity], g);
+    site_settle<PROF>(a, parity, g, sn, o);
+  }
+  if (a.blockmax) motion_to_block(a, parity, lead ? g : -1, o);
   stats_flush(a.stats, a.segs, o, stage);
   __syncthreads();
   stats_stage_flush(a.stats, a.segs, stage);

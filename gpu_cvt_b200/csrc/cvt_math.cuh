@@ -6,6 +6,7 @@
 // of each routine follows the reference kernels it replaces (cited below);
 // the reference's rsqrtf() becomes 1/sqrt (IEEE), a <=1-ulp difference.
 #pragma once
+#include <climits>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -452,6 +453,100 @@ __device__ __forceinline__ bool project_onering_rec(V3<T> c, const float4* __res
   }
   out = cvt3<T>(bp);
   return true;
+}
+
+// project_onering_rec by LANES lanes of a warp (all of the warp takes part):
+// the entries of the rings are dealt out to the lanes, each tests the faces
+// its entries keep, and the smallest (squared distance, place) of all wins.
+// c and knnv are the same in every lane of a group.
+template <class T, class Q, int LANES, int NV>
+__device__ __forceinline__ V3<T> project_onering_lanes(V3<T> c, const float4* __restrict__ head,
+                                                       const float4* __restrict__ body, int nV,
+                                                       const int* __restrict__ off, const int (&knnv)[NV]) {
+  constexpr unsigned full = 0xffffffffu;
+  const int sub = threadIdx.x & (LANES - 1);
+  const float qx = (float)c.x, qy = (float)c.y, qz = (float)c.z;
+  const float slack = 1e-4f * fmaxf(fabsf(qx), fmaxf(fabsf(qy), fabsf(qz)));
+  // entry i of the rings laid end to end is ring t's entry first[t] + i
+  int first[NV], end[NV];
+  int total = 0;
+#pragma unroll
+  for (int t = 0; t < NV; ++t) {
+    const bool valid = (unsigned)knnv[t] < (unsigned)nV;
+    const int b = valid ? __ldg(off + knnv[t]) : 0, e = valid ? __ldg(off + knnv[t] + 1) : 0;
+    first[t] = b - total;
+    total += e - b;
+    end[t] = total;
+  }
+  auto entry_of = [&](int i, int& t) {
+    int f = first[0];
+    t = 0;
+#pragma unroll
+    for (int k = 1; k < NV; ++k)
+      if (i >= end[k - 1]) { f = first[k]; t = k; }
+    return f + i;
+  };
+  auto dist = [&](float4 h) {
+    const float dx = qx - h.x, dy = qy - h.y, dz = qz - h.z;
+    return approx_root(fmaT(dz, dz, fmaT(dy, dy, dx * dx)));
+  };
+  const V3<Q> cq = cvt3<Q>(c);
+  V3<Q> bp = cq;
+  Q best = (Q)1e30;
+  int best_at = INT_MAX;
+  auto test = [&](int entry, int at) {
+    const float4* w = body + kRingBody * (long)entry;
+    const float4 r0 = __ldg(w), r1 = __ldg(w + 1), r2 = __ldg(w + 2);
+    if (__float_as_int(r2.y) < 0) return;  // an invalid entry
+    const V3<Q> A = {(Q)r0.x, (Q)r0.y, (Q)r0.z};
+    const V3<Q> B = {(Q)r0.w, (Q)r1.x, (Q)r1.y};
+    const V3<Q> C = {(Q)r1.z, (Q)r1.w, (Q)r2.x};
+    const V3<Q> p = closest_point_tri(cq, A, B, C);
+    const V3<Q> dd = sub3(p, cq);
+    const Q d2 = dot3(dd, dd);
+    if (d2 < best || (d2 == best && at < best_at && best_at != INT_MAX)) { best = d2; bp = p; best_at = at; }
+  };
+  // the nearest vertex's face with the nearest centre, tested by every lane
+  unsigned long long near = ~0ull;
+  for (int i = sub; i < end[0]; i += LANES) {
+    const unsigned long long k = ((unsigned long long)__float_as_uint(dist(__ldg(head + first[0] + i))) << 32) | (unsigned)i;
+    near = k < near ? k : near;
+  }
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1) {
+    const unsigned long long k = __shfl_xor_sync(full, near, o);
+    near = k < near ? k : near;
+  }
+  const int lead = near == ~0ull ? -1 : (int)(unsigned)near;
+  float limit = INFINITY;
+  if (lead >= 0) {
+    test(first[0] + lead, lead);
+    limit = approx_root((float)best) * 1.001f;
+  }
+  for (int i = sub; i < total; i += LANES) {
+    int t;
+    const int entry = entry_of(i, t);
+    const float4 h = __ldg(head + entry);
+    const float dc = dist(h);
+    if (i == lead || (dc <= 50.f * h.w && fmaT(0.9438f, dc, -slack) - 1.0501f * h.w > limit)) continue;
+    const float4 r2 = __ldg(body + kRingBody * (long)entry + 2);
+    const int ia = __float_as_int(r2.y), ib = __float_as_int(r2.z), ic = __float_as_int(r2.w);
+    bool seen = false;
+#pragma unroll
+    for (int s = 0; s + 1 < NV; ++s) {
+      const int w = knnv[s];
+      seen = seen || (s < t && (w == ia || w == ib || w == ic));
+    }
+    if (!seen) test(entry, i);
+  }
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1) {
+    const Q d = __shfl_xor_sync(full, best, o);
+    const int at = __shfl_xor_sync(full, best_at, o);
+    const V3<Q> p{__shfl_xor_sync(full, bp.x, o), __shfl_xor_sync(full, bp.y, o), __shfl_xor_sync(full, bp.z, o)};
+    if (d < best || (d == best && at < best_at)) { best = d; best_at = at; bp = p; }
+  }
+  return cvt3<T>(bp);
 }
 
 // --------------------------------------------------------------------------

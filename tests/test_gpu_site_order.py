@@ -168,3 +168,17 @@ def test_uneven_density_searches(eng, oracle, n, k, profile):
     r = oracle.lloyd_run(m.V, m.F, S0, k, 0, 3, profile=oracle.PROFILES[profile])
     assert np.array_equal(st["knn"], r["knn"])
     assert np.array_equal(S, r["S"])
+
+
+@pytest.mark.parametrize("n", [32768, 32769])
+@pytest.mark.parametrize("profile,mode", [("ref", 0), ("mixed", 1), ("fp64", 2)])
+def test_lanes_and_threads_meet(eng, oracle, n, profile, mode):
+    """The largest site set whose vertex search and projection run with lanes
+    per site, and the smallest with one thread each (thin faces among the
+    mesh's, which the projection never skips)."""
+    m = mg.torus(1.0, 0.3, 400, 40, noise_sigma=0.002, seed=4)
+    S0 = mg.sample_sites(m.V, m.F, n, seed=n)
+    S, st, _ = _run(eng, m, S0, 12, mode, 3, profile, True)
+    r = oracle.lloyd_run(m.V, m.F, S0, 12, mode, 3, profile=oracle.PROFILES[profile])
+    assert np.array_equal(st["knnv"], r["knnv"])
+    assert np.array_equal(S, r["S"])
