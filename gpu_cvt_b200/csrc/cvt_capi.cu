@@ -212,52 +212,73 @@ struct Scratch {
 // ---------------------------------------------------------------------------
 struct PointGrid {
   GridGeom* geom = nullptr;
-  int* cell_count = nullptr;
+  unsigned* zero = nullptr;  // 8 words: bounds and tickets (k_bbox_geom); one memset clears them, the
+  int* cell_count = nullptr; // cell counts behind them and rest[0]
+  int* rest = nullptr;       // stage searches: [0] = count, queries left to k_stage_knn_warp
   int* cell_start = nullptr;
   int* part = nullptr;
   int2* cellrank = nullptr;
   Pt4<float>* sorted = nullptr;
-  int* rest = nullptr;  // stage searches: [0] = count, queries left to k_stage_knn_warp
   int total_cells = 0;  // scan length (spatial capacity + NaN bucket)
+  // the arrays, one after another, for n points and n_rest queries; returns
+  // their bytes (base == NULL: only that)
+  size_t carve(unsigned char* base, int n, int n_rest) {
+    size_t at = 0;
+    auto take = [&](auto*& p, size_t count) {
+      p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at);
+      at += (count * sizeof(*p) + 255) & ~size_t(255);
+    };
+    take(zero, 8);
+    at = 32;
+    take(cell_count, (size_t)total_cells);
+    at = 32 + sizeof(int) * (size_t)total_cells;  // rest[0] right behind the counts
+    take(rest, (size_t)n_rest + 1);
+    at = (at + 255) & ~size_t(255);
+    take(geom, 1);
+    take(cell_start, (size_t)total_cells + 1);
+    take(part, (size_t)scan_blocks(total_cells) + 2);
+    take(cellrank, (size_t)n);
+    take(sorted, (size_t)n);
+    return at;
+  }
 };
 
-// geometry supplied by the host (hgeom != nullptr) or derived on the device
-// from the bbox with ~per_cell points per cell
-static cvt_status_t build_point_grid(Scratch& sc, const float* P, int n, float per_cell, const GridGeom* hgeom,
-                                     PointGrid& pg) {
-  cudaStream_t st = sc.st;
-  int cap = hgeom ? hgeom->ncell : std::max(64, 2 * n);
-  pg.total_cells = cap + 1;
-  CK(sc.get(&pg.geom, 1));
-  CK(sc.get(&pg.cell_count, (size_t)pg.total_cells));
-  CK(sc.get(&pg.cell_start, (size_t)pg.total_cells + 1));
-  CK(sc.get(&pg.part, (size_t)scan_blocks(pg.total_cells) + 2));
-  CK(sc.get(&pg.cellrank, (size_t)std::max(n, 1)));
-  CK(sc.get(&pg.sorted, (size_t)std::max(n, 1)));
+static int point_grid_cells(int n) { return std::max(64, 2 * n); }
+
+// The build into pg's arrays: one memset and five kernels (six with the
+// geometry supplied by the host); geometry derived on the device from the
+// bounds with ~per_cell points per cell when hgeom is NULL.
+static cvt_status_t enqueue_point_grid(const PointGrid& pg, const float* P, int n, float per_cell, const GridGeom* hgeom,
+                                       cudaStream_t st) {
+  CK(cudaMemsetAsync(pg.zero, 0, 32 + sizeof(int) * ((size_t)pg.total_cells + 1), st));
   if (hgeom) {
     CK(cudaMemcpyAsync(pg.geom, hgeom, sizeof(GridGeom), cudaMemcpyHostToDevice, st));
   } else {
-    int* bb;
-    CK(sc.get(&bb, 6));
-    k_bbox_init<<<1, 32, 0, st>>>(bb);
-    CKLAUNCH();
-    if (n > 0) { k_bbox<<<wave_blocks(n, kBboxThreads), kBboxThreads, 0, st>>>(n, P, bb); CKLAUNCH(); }
-    k_grid_geom<<<1, 32, 0, st>>>(bb, n, per_cell, cap, pg.geom);
+    k_bbox_geom<<<std::max(1, wave_blocks(n, kBboxThreads)), kBboxThreads, 0, st>>>(n, P, pg.zero, per_cell, pg.total_cells - 1,
+                                                                                   pg.geom);
     CKLAUNCH();
   }
-  CK(cudaMemsetAsync(pg.cell_count, 0, sizeof(int) * pg.total_cells, st));
   if (n > 0) {
     k_grid_count<float><<<cdiv(n, 256), 256, 0, st>>>(n, P, SegGrid{pg.geom, nullptr, nullptr}, pg.cell_count, pg.cellrank);
     CKLAUNCH();
   }
-  launch_exclusive_scan(pg.total_cells, pg.cell_count, pg.part, pg.cell_start, st);
-  LAUNCHED(3);
+  LAUNCHED(launch_exclusive_scan(pg.total_cells, pg.cell_count, pg.part, pg.cell_start, st, false, pg.zero + 7));
   CK(cudaGetLastError());
   if (n > 0) {
     k_grid_scatter<float><<<cdiv(n, 256), 256, 0, st>>>(n, P, pg.cellrank, pg.cell_start, pg.sorted);
     CKLAUNCH();
   }
   return CVT_OK;
+}
+
+// the same with its arrays from one stream-ordered allocation
+static cvt_status_t build_point_grid(Scratch& sc, const float* P, int n, float per_cell, const GridGeom* hgeom,
+                                     PointGrid& pg, int n_rest = 0) {
+  pg.total_cells = (hgeom ? hgeom->ncell : point_grid_cells(n)) + 1;
+  unsigned char* base;
+  CK(sc.get(&base, pg.carve(nullptr, std::max(n, 1), n_rest)));
+  pg.carve(base, std::max(n, 1), n_rest);
+  return enqueue_point_grid(pg, P, n, per_cell, hgeom, sc.st);
 }
 
 // ---------------------------------------------------------------------------
@@ -308,7 +329,7 @@ static void launch_knn_warp(const PointGrid& pg, const float* Q, int n, const in
 constexpr int kWarpPoints = 60000;
 constexpr int kWarpQueries = 50000;
 
-// the points' own neighbours; pg.rest[0] is zero
+// the points' own neighbours
 static cvt_status_t launch_knn_sites(const PointGrid& pg, int n, const uint8_t* frozen, int kk, uint32_t* knn, float* dist,
                                      cudaStream_t st) {
   if (n < kWarpPoints) {
@@ -333,16 +354,13 @@ static cvt_status_t launch_knn_sites(const PointGrid& pg, int n, const uint8_t* 
 }
 
 // the neighbours of nQ query points among n points
-static cvt_status_t launch_knn_queries(Scratch& sc, PointGrid& pg, const float* Q, int nQ, const uint8_t* frozen, int kk,
-                                       int ex, uint32_t* knn, float* dist) {
-  cudaStream_t st = sc.st;
+static cvt_status_t launch_knn_queries(const PointGrid& pg, const float* Q, int nQ, const uint8_t* frozen, int kk, int ex,
+                                       uint32_t* knn, float* dist, cudaStream_t st) {
   if (nQ < kWarpQueries) {
     launch_knn_warp(pg, Q, nQ, nullptr, frozen, kk, ex, knn, dist, st);
     CKLAUNCH();
     return CVT_OK;
   }
-  CK(sc.get(&pg.rest, (size_t)nQ + 1));
-  CK(cudaMemsetAsync(pg.rest, 0, sizeof(int), st));
   KK_DISPATCH(kk, launch_knn_query, pg, Q, nQ, frozen, kk, ex, knn, dist, st);
   CKLAUNCH();
   launch_knn_warp(pg, Q, nQ, pg.rest, frozen, kk, ex, knn, dist, st);
@@ -357,10 +375,8 @@ extern "C" cvt_status_t cvt_knn_sites(const float* pts, int n, int kk, const uin
   cudaStream_t st = S_(stream);
   Scratch sc(st);
   PointGrid pg;
-  cvt_status_t s = build_point_grid(sc, pts, n, 0.2f * kk, nullptr, pg);
+  cvt_status_t s = build_point_grid(sc, pts, n, 0.2f * kk, nullptr, pg, n);
   if (s != CVT_OK) return s;
-  CK(sc.get(&pg.rest, (size_t)n + 1));
-  CK(cudaMemsetAsync(pg.rest, 0, sizeof(int), st));
   return launch_knn_sites(pg, n, frozen, kk, knn, dist, st);
 }
 
@@ -372,9 +388,9 @@ extern "C" cvt_status_t cvt_knn_query_to_points(const float* cand, int n_cand, c
   cudaStream_t st = S_(stream);
   Scratch sc(st);
   PointGrid pg;
-  cvt_status_t s = build_point_grid(sc, cand, n_cand, 0.2f * kk + 1.f, nullptr, pg);
+  cvt_status_t s = build_point_grid(sc, cand, n_cand, 0.2f * kk + 1.f, nullptr, pg, n_query);
   if (s != CVT_OK) return s;
-  return launch_knn_queries(sc, pg, query, n_query, frozen, kk, 0, knn, dist);
+  return launch_knn_queries(pg, query, n_query, frozen, kk, 0, knn, dist, st);
 }
 
 extern "C" cvt_status_t cvt_knn_vertices(const float* V, int nV, const float* Q, int nQ, int k, int exclude_self,
@@ -385,10 +401,10 @@ extern "C" cvt_status_t cvt_knn_vertices(const float* V, int nV, const float* Q,
   cudaStream_t st = S_(stream);
   Scratch sc(st);
   PointGrid pg;
-  cvt_status_t s = build_point_grid(sc, V, nV, 0.2f * k + 1.f, nullptr, pg);
+  cvt_status_t s = build_point_grid(sc, V, nV, 0.2f * k + 1.f, nullptr, pg, nQ);
   if (s != CVT_OK) return s;
   // int output: the uint32 sentinel 0xFFFFFFFF reads as -1
-  return launch_knn_queries(sc, pg, Q, nQ, frozen, k, exclude_self ? 1 : 0, reinterpret_cast<uint32_t*>(out), nullptr);
+  return launch_knn_queries(pg, Q, nQ, frozen, k, exclude_self ? 1 : 0, reinterpret_cast<uint32_t*>(out), nullptr, st);
 }
 
 extern "C" cvt_status_t cvt_knn_drop_self(const uint32_t* in, int n, int kin, int kout, uint32_t* out, void* stream) {

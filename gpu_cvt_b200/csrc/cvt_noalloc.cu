@@ -15,7 +15,7 @@
 // Limits and rules:
 //   * at most CVT_NOALLOC_MAX_POINTS points per call (larger calls return
 //     CVT_ERR_CAPACITY and do nothing);
-//   * the array (~5.5 MB) is held by every GPU that loads the library, until
+//   * the array (~6 MB) is held by every GPU that loads the library, until
 //     the process exits;
 //   * all calls share that one array: calls whose work overlaps on the GPU
 //     (different streams, or different host threads without ordering) race
@@ -32,18 +32,10 @@
 namespace noalloc {
 
 constexpr int kMaxPoints = CVT_NOALLOC_MAX_POINTS;
-constexpr int kCap = 2 * kMaxPoints;  // spatial cells: the allocating path's max(64, 2n)
-constexpr size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
-constexpr size_t kScanParts = (size_t)(kCap + 1 + kScanTile - 1) / kScanTile + 2;
-constexpr size_t kOffBbox = 0;
-constexpr size_t kOffGeom = up256(kOffBbox + 6 * sizeof(int));
-constexpr size_t kOffCount = up256(kOffGeom + sizeof(GridGeom));
-constexpr size_t kOffStart = up256(kOffCount + (size_t)(kCap + 1) * sizeof(int));
-constexpr size_t kOffPart = up256(kOffStart + (size_t)(kCap + 2) * sizeof(int));
-constexpr size_t kOffRank = up256(kOffPart + kScanParts * sizeof(int));
-constexpr size_t kOffSorted = up256(kOffRank + (size_t)kMaxPoints * sizeof(int2));
-constexpr size_t kOffRest = up256(kOffSorted + (size_t)kMaxPoints * sizeof(Pt4<float>));
-constexpr size_t kBytes = up256(kOffRest + (size_t)(kMaxPoints + 1) * sizeof(int));
+constexpr int kCap = 2 * kMaxPoints;  // spatial cells: the allocating path's point_grid_cells
+// bytes of PointGrid::carve for kMaxPoints points and queries, rounded up
+constexpr size_t kBytes = 4096 + sizeof(int) * ((size_t)2 * (kCap + 2) + kCap / kScanTile + 8 + kMaxPoints) +
+                          (size_t)kMaxPoints * (sizeof(int2) + sizeof(Pt4<float>));
 
 }  // namespace noalloc
 
@@ -84,34 +76,13 @@ extern "C" cvt_status_t cvt_knn_sites_noalloc(const float* pts, int n, int kk, c
   cvt_status_t s = knn_scratch_address(&base);
   if (s != CVT_OK) return s;
   cudaStream_t st = S_(stream);
-  unsigned char* b = static_cast<unsigned char*>(base);
-  int* bb = reinterpret_cast<int*>(b + noalloc::kOffBbox);
   PointGrid pg;
-  pg.geom = reinterpret_cast<GridGeom*>(b + noalloc::kOffGeom);
-  pg.cell_count = reinterpret_cast<int*>(b + noalloc::kOffCount);
-  pg.cell_start = reinterpret_cast<int*>(b + noalloc::kOffStart);
-  pg.part = reinterpret_cast<int*>(b + noalloc::kOffPart);
-  pg.cellrank = reinterpret_cast<int2*>(b + noalloc::kOffRank);
-  pg.sorted = reinterpret_cast<Pt4<float>*>(b + noalloc::kOffSorted);
-  pg.rest = reinterpret_cast<int*>(b + noalloc::kOffRest);
-  const int cap = std::max(64, 2 * n);
-  pg.total_cells = cap + 1;
-  // the array keeps the previous call's contents: the bounding box and the
-  // cell counts must start from their initial values
-  k_bbox_init<<<1, 32, 0, st>>>(bb);
-  CKLAUNCH();
-  k_bbox<<<wave_blocks(n, kBboxThreads), kBboxThreads, 0, st>>>(n, pts, bb);
-  CKLAUNCH();
-  k_grid_geom<<<1, 32, 0, st>>>(bb, n, 0.2f * kk, cap, pg.geom);
-  CKLAUNCH();
-  CK(cudaMemsetAsync(pg.cell_count, 0, sizeof(int) * pg.total_cells, st));
-  CK(cudaMemsetAsync(pg.rest, 0, sizeof(int), st));
-  k_grid_count<float><<<cdiv(n, 256), 256, 0, st>>>(n, pts, SegGrid{pg.geom, nullptr, nullptr}, pg.cell_count, pg.cellrank);
-  CKLAUNCH();
-  launch_exclusive_scan(pg.total_cells, pg.cell_count, pg.part, pg.cell_start, st);
-  LAUNCHED(3);
-  CK(cudaGetLastError());
-  k_grid_scatter<float><<<cdiv(n, 256), 256, 0, st>>>(n, pts, pg.cellrank, pg.cell_start, pg.sorted);
-  CKLAUNCH();
+  pg.total_cells = point_grid_cells(n) + 1;
+  if (pg.carve(static_cast<unsigned char*>(base), n, n) > noalloc::kBytes)
+    return fail(CVT_ERR_CAPACITY, "cvt_knn_sites_noalloc: scratch array too small");
+  // the array keeps the previous call's contents; the build clears what must
+  // start at zero
+  s = enqueue_point_grid(pg, pts, n, 0.2f * kk, nullptr, st);
+  if (s != CVT_OK) return s;
   return launch_knn_sites(pg, n, frozen, kk, knn, dist, st);
 }

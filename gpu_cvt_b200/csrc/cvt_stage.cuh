@@ -49,14 +49,12 @@ __global__ void __launch_bounds__(kBboxThreads) k_bbox(int n, const float* __res
 }
 
 // Geometry for ~`per_cell` points per occupied cell on a surface, at most
-// max_cells spatial cells.
-__global__ void k_grid_geom(const int* bb, int n, float per_cell, int max_cells, GridGeom* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// max_cells spatial cells (lo, hi: bounds of the finite points, if any).
+__device__ inline GridGeom points_geom(bool any, const float* blo, const float* bhi, int n, float per_cell, int max_cells) {
   float lo[3], hi[3];
-  bool any = bb[0] != 0x7fffffff;
   for (int a = 0; a < 3; ++a) {
-    lo[a] = any ? ord2f(bb[a]) : 0.f;
-    hi[a] = any ? ord2f(bb[3 + a]) : 1.f;
+    lo[a] = any ? blo[a] : 0.f;
+    hi[a] = any ? bhi[a] : 1.f;
   }
   float ext[3] = {hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2]};
   float emax = fmaxf(fmaxf(ext[0], ext[1]), fmaxf(ext[2], 1e-20f));
@@ -78,7 +76,48 @@ __global__ void k_grid_geom(const int* bb, int n, float per_cell, int max_cells,
   g.inv_h = (float)(1.0 / h);
   g.cell_base = 0;
   g.ncell = g.dim[0] * g.dim[1] * g.dim[2];
-  *out = g;
+  return g;
+}
+
+// Bounds of n points and, by the last block to finish, their grid geometry.
+// zero: 8 words that start at zero, so that one memset prepares a whole grid
+// build: the bounds as maxima (of the ordered value, and of its complement for
+// the lower ones), the ticket in word 6.
+__global__ void __launch_bounds__(kBboxThreads) k_bbox_geom(int n, const float* __restrict__ P, unsigned* zero, float per_cell,
+                                                            int max_cells, GridGeom* out) {
+  __shared__ unsigned sb[6];
+  __shared__ bool last;
+  if (threadIdx.x < 6) sb[threadIdx.x] = 0u;
+  __syncthreads();
+  unsigned mx[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+  for (int i = blockIdx.x * kBboxThreads + threadIdx.x; i < n; i += gridDim.x * kBboxThreads) {
+    const V3<float> p = ld3(P, i);
+    if (!finite3(p)) continue;
+    const unsigned o[3] = {(unsigned)f2ord(p.x) ^ 0x80000000u, (unsigned)f2ord(p.y) ^ 0x80000000u,
+                           (unsigned)f2ord(p.z) ^ 0x80000000u};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) { mx[a] = max(mx[a], ~o[a]); mx[3 + a] = max(mx[3 + a], o[a]); }
+  }
+#pragma unroll
+  for (int a = 0; a < 6; ++a) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, mx[a]);
+    if ((threadIdx.x & 31) == 0) atomicMax(sb + a, m);
+  }
+  __syncthreads();
+  if (threadIdx.x < 6) atomicMax(zero + threadIdx.x, sb[threadIdx.x]);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(zero + 6, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last || threadIdx.x != 0) return;
+  __threadfence();
+  float lo[3], hi[3];
+  const volatile unsigned* z = zero;
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = ord2f((int)(~z[a] ^ 0x80000000u));
+    hi[a] = ord2f((int)(z[3 + a] ^ 0x80000000u));
+  }
+  *out = points_geom(z[3] != 0u, lo, hi, n, per_cell, max_cells);
 }
 
 // ---------------------------------------------------------------------------

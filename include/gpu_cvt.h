@@ -66,7 +66,7 @@ cvt_status_t cvt_knn_sites(const float* pts, int n, int kk, const uint8_t* froze
  * callers that cannot allocate device memory while they run (a serving
  * process that reserved a fixed HBM budget up front, or a host whose own
  * allocator owns the device heap): the search's temporaries live in one
- * fixed array compiled into the library (about 5 MB, held on every GPU that
+ * fixed array compiled into the library (about 6 MB, held on every GPU that
  * loads the library until the process exits), so the call allocates and
  * frees nothing.  At most CVT_NOALLOC_MAX_POINTS points (larger n returns
  * CVT_ERR_CAPACITY).  All calls share the array: calls that overlap on the
