@@ -1765,7 +1765,7 @@ static cvt_status_t enqueue_iteration_t(cvt_engine* e, int parity, cudaStream_t 
     }
     launch_site_proj<PROF>(a, parity, ns, e->p.proj_block, e->p.proj_mode, st);
   }
-  k_site_far<PROF><<<e->num_sms, 128, 0, st>>>(a, parity, e->d_segs, e->d_active, e->max_seg, e->d_tickets + 1);
+  k_site_far<PROF><<<e->num_sms, kFarThreads, 0, st>>>(a, parity, e->d_segs, e->d_active, e->max_seg, e->d_tickets + 1);
   L += 2;
   if (ev) CK(cudaEventRecord(ev[4], st));
   if (ev) CK(cudaEventRecord(ev[5], st));
