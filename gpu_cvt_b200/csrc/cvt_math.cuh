@@ -346,6 +346,11 @@ __global__ void k_build_ring_records(const float* __restrict__ V, const int* __r
 // over interleaved 64-byte records, 111 with heads apart, 105 so; an FP32
 // edge test before the FP64 one (109) and 32 warps (spills; 104) gain nothing.
 constexpr int kRingList = 32;
+// Entries of step 3 loaded together: one at a time each waits for its own
+// load.  Vertex search and projection of 300k sites: 165 us with 1, 158 with 2,
+// 157 with 4 (100k sites 76, 74, 76).  Loading the next face of step 4 ahead
+// costs spills (160 against 151 us, with the vertex search of grid_knn_box).
+constexpr int kRingBatch = 2;
 template <int BS> struct RingList { int e[kRingList][BS]; };  // entries, per thread
 
 template <class T, class Q>
@@ -434,18 +439,27 @@ __device__ __forceinline__ bool project_onering_rec(V3<T> c, const float4* __res
   }
   if (cnt > kRingList) return false;
   int m = 0, m0 = 0;
-  for (int k = 0; k < cnt; ++k) {
-    const int e = L.e[k][col];
-    const float4 r2 = __ldg(body + kRingBody * (long)e + 2);
-    const int ia = __float_as_int(r2.y), ib = __float_as_int(r2.z), ic = __float_as_int(r2.w);
-    bool seen = ia < 0;
+  for (int k0 = 0; k0 < cnt; k0 += kRingBatch) {
+    int e[kRingBatch];
+    float4 ids[kRingBatch];
 #pragma unroll
-    for (int s = 0; s + 1 < NV; ++s) {
-      const int w = knnv[s];
-      seen = seen || (k >= ends[s] && (w == ia || w == ib || w == ic));
+    for (int j = 0; j < kRingBatch; ++j) {
+      e[j] = L.e[min(k0 + j, cnt - 1)][col];
+      ids[j] = __ldg(body + kRingBody * (long)e[j] + 2);
     }
-    if (!seen) L.e[m++][col] = e;
-    if (k < ends[0]) m0 = m;
+#pragma unroll
+    for (int j = 0; j < kRingBatch; ++j) {
+      const int k = k0 + j;
+      const int ia = __float_as_int(ids[j].y), ib = __float_as_int(ids[j].z), ic = __float_as_int(ids[j].w);
+      bool seen = ia < 0 || k >= cnt;
+#pragma unroll
+      for (int s = 0; s + 1 < NV; ++s) {
+        const int w = knnv[s];
+        seen = seen || (k >= ends[s] && (w == ia || w == ib || w == ic));
+      }
+      if (!seen) L.e[m++][col] = e[j];
+      if (k < ends[0]) m0 = m;
+    }
   }
   for (int k = 0; k < m; ++k) {
     const int e = L.e[k][col];
