@@ -2390,15 +2390,18 @@ static cvt_status_t engine_eval_impl(cvt_engine_t e, int s, cvt_eval_t* out, int
   }
   float R2 = 2.0f * 0.5f * std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
   const FaceColumns nb{e->d_list + sd.site_base, label, (size_t)e->max_sites, (uint32_t)sd.site_base};
+  // before the first iteration there are no lists: the slots may still hold
+  // those of a segment that was there before
+  const int K = e->host_iters[s] == 0 ? 0 : e->K;
   int max_faces = 4 * n + 64;
   int* Fc;
   CK(sc.get(&Fc, 3 * (size_t)max_faces));
   int nf = 0;
-  cvt_status_t r = extract_faces(Sf, U, V, nb, Sc, n, e->K, R2, Fc, max_faces, &nf, st);
+  cvt_status_t r = extract_faces(Sf, U, V, nb, Sc, n, K, R2, Fc, max_faces, &nf, st);
   if (r == CVT_ERR_CAPACITY) {
     max_faces = nf;
     CK(sc.get(&Fc, 3 * (size_t)max_faces));
-    r = extract_faces(Sf, U, V, nb, Sc, n, e->K, R2, Fc, max_faces, &nf, st);
+    r = extract_faces(Sf, U, V, nb, Sc, n, K, R2, Fc, max_faces, &nf, st);
   }
   if (r != CVT_OK) return r;
   float q[6];
