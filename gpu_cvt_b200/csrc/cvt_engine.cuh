@@ -238,6 +238,17 @@ __device__ __forceinline__ bool halfplane_contains_disk(Q a, Q b, Q c, Q r2) {
   return c > (Q)1e-18 && fmaT(a, a, b * b) * r2 * (Q)1.0001 < c * c;
 }
 
+// Upper bound on ((d.u)^2 + (d.v)^2) / |d|^2 over all d, the largest eigenvalue
+// of the frame's Gram matrix by its row sums; at least 1, NaN for a frame with
+// NaN (then clip_cell skips nothing).  The stage calls take frames of any length
+// and skew from their caller.
+__device__ __forceinline__ float frame_gain(V3<float> u, V3<float> v) {
+  const float uv = fabsf(dot3(u, v));
+  const float x = (dot3(u, u) + uv) * 1.00001f, y = (dot3(v, v) + uv) * 1.00001f;
+  const float g = x > y ? x : y;
+  return x == x && g <= 1.00002f ? 1.f : x == x ? g : x;
+}
+
 // Neighbours of a site for clip_cell and pca_normal: id(t) is entry t of its
 // list, valid(id) whether it names a site, pos(id) that site's position.
 template <class T> struct RowNeighbours {  // row-major list of local indices into an AoS array
@@ -336,9 +347,10 @@ __device__ __forceinline__ int clip_cell_full(const NB& nb, V3<typename PT<PROF>
 // 9 u |d| r + 8 u c (u = 2^-24: difference, frame dots, half square and two
 // fma), and 2e-6 (|d| r + c) is left to the FP64 predicate itself; FP64
 // coefficients are only computed for those vertices and for real cuts.
-// Neighbours with |d|^2 > 4 r^2 (margin 2.5e-3) cannot cut whatever the frame
-// (its vectors have unit length to 1e-6): skipped, and on this iteration's
-// sorted list they end the loop (see clip_cell_full).
+// `gain` bounds (a^2 + b^2) / |d|^2 (frame_gain; 1 for the engine's frames, whose
+// vectors are orthonormal to 1e-6).  Neighbours with |d|^2 > 4 gain r^2 (margin
+// 2.5e-3) cannot cut: skipped, and on this iteration's sorted list they end the
+// loop (see clip_cell_full).  The FP32 error above grows with sqrt(gain) too.
 //
 // Bound by issue (63 %) and latency; 24 of 32 threads active.  Clip kernel,
 // mixed, 300k sites, K = 24: 57 us and 117 warp instructions per site, against
@@ -346,7 +358,7 @@ __device__ __forceinline__ int clip_cell_full(const NB& nb, V3<typename PT<PROF>
 // active, conversions 42 % of their pipe).
 template <int PROF, class NB>
 __device__ __forceinline__ int clip_cell(const NB& nb, V3<typename PT<PROF>::T> si, int K,
-                                         const Frame<typename PT<PROF>::T>& fr, float R,
+                                         const Frame<typename PT<PROF>::T>& fr, float gain, float R,
                                          const PolyRef<typename PT<PROF>::PP>& P, int cap, bool row_sorted) {
   using T = typename PT<PROF>::T;
   using Q = typename PT<PROF>::Q;
@@ -373,7 +385,7 @@ __device__ __forceinline__ int clip_cell(const NB& nb, V3<typename PT<PROF>::T> 
     const V3<T> d = sub3(sj, si);
     const V3<float> df = cvt3<float>(d);
     const float dd = dot3(df, df);
-    if (dd > 4.01f * r2 && dd > 2e-18f && dd < 1e30f) {
+    if (dd > 4.01f * gain * r2 && dd > 2e-18f && dd < 1e30f) {
       done = row_sorted;
       continue;
     }
@@ -394,7 +406,7 @@ __device__ __forceinline__ int clip_cell(const NB& nb, V3<typename PT<PROF>::T> 
     if (kFilter) {
       const float af = (float)dot3(d, fr.u), bf = (float)dot3(d, fr.v), cf = 0.5f * dd;
       float root;
-      asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"(dd * r2));
+      asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"(dd * r2 * gain));
       const float tol = 2e-6f * (root + cf) + 2e-12f;
       unsigned unsure = 0u;
       for (int i = 0; i < n; ++i) {
@@ -1041,7 +1053,7 @@ __device__ __forceinline__ bool site_clip(const EngineArgs<typename PT<PROF>::T>
   }
   PolyRef<PP> cur = A, nxt = B;
   const int np = FULL ? clip_cell_full<PROF>(nb, si, a.K, fr, md.R, cur, nxt, cap, !fz)
-                      : clip_cell<PROF>(nb, si, a.K, fr, md.R, A, cap, !fz);
+                      : clip_cell<PROF>(nb, si, a.K, fr, 1.f, md.R, A, cap, !fz);
   if (np < 0) return false;
   const V2<PP> c2 = poly_centroid<PP>(cur, np, PROF == PROF_MIXED);
   V3<T> cent;

@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(kFaceThreads) k_face_keys(const float* __restr
   const V3<float> si = ld3(S, i), ui = ld3(U, i), vi = ld3(Vv, i);
   P[0][c] = make_float2(-R2, -R2); P[1][c] = make_float2(R2, -R2); P[2][c] = make_float2(R2, R2); P[3][c] = make_float2(-R2, R2);
   int na = 4;
+  const float gain = frame_gain(ui, vi);
   float r2 = 2.f * R2 * R2 * 1.0001f;
   for (int t = 0; t < K; ++t) {
     if (na <= 0) continue;
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(kFaceThreads) k_face_keys(const float* __restr
     if ((unsigned)j >= (unsigned)n || j == i) continue;
     const V3<float> d = sub3(ld3(S, j), si);
     const float dd = dot3(d, d);
-    if (dd > 4.01f * r2 && dd > 2e-18f && dd < 1e30f) continue;  // cannot cut (clip_cell)
+    if (dd > 4.01f * gain * r2 && dd > 2e-18f && dd < 1e30f) continue;  // cannot cut (clip_cell)
     const float a = dot3(d, ui), b = dot3(d, vi), cc = 0.5f * dd;
     auto f = [&](float2 p) { return fmaT(a, p.x, fmaT(b, p.y, -cc)); };
     unsigned out = 0u;

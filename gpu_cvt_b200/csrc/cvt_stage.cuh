@@ -360,7 +360,8 @@ __global__ void __launch_bounds__(BLOCK) k_stage_clip(const float* __restrict__ 
   if (i >= n) return;
   V3<float> si = ld3(S, i);
   Frame<float> fr{ld3(U, i), ld3(Vv, i)};
-  int np = clip_cell<PROF>(RowNeighbours<float>{S, knn + (size_t)i * K, (uint32_t)n}, si, K, fr, R, cur, CAP, false);
+  int np = clip_cell<PROF>(RowNeighbours<float>{S, knn + (size_t)i * K, (uint32_t)n}, si, K, fr, frame_gain(fr.u, fr.v), R, cur,
+                           CAP, false);
   if (np < 0) {
     int k = atomicAdd(ovf, 1);
     ovf[1 + k] = i;
