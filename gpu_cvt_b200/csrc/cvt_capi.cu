@@ -309,14 +309,14 @@ static void launch_knn_query(const PointGrid& pg, const float* Q, int nQ, const 
     else FN<64>(__VA_ARGS__);                                    \
   } while (0)
 
-// one warp per query: all n of them, or those listed in rest
-static void launch_knn_warp(const PointGrid& pg, const float* Q, int n, const int* rest, const uint8_t* frozen, int kk,
-                            int ex, uint32_t* knn, float* dist, cudaStream_t st) {
+// one warp per query: all n of them, or those listed in rest (P: by k_stage_knn_query)
+static void launch_knn_warp(const PointGrid& pg, const float* Q, int n, const int* rest, const float* P,
+                            const uint8_t* frozen, int kk, int ex, uint32_t* knn, float* dist, cudaStream_t st) {
   const int blocks = std::min(cdiv(n, 4), 8 * sm_count());
   if (kk <= 32)
-    k_stage_knn_warp<1><<<blocks, 128, 0, st>>>(pg.geom, pg.cell_start, pg.sorted, Q, n, rest, frozen, kk, ex, knn, dist);
+    k_stage_knn_warp<1><<<blocks, 128, 0, st>>>(pg.geom, pg.cell_start, pg.sorted, Q, n, rest, P, frozen, kk, ex, knn, dist);
   else
-    k_stage_knn_warp<2><<<blocks, 128, 0, st>>>(pg.geom, pg.cell_start, pg.sorted, Q, n, rest, frozen, kk, ex, knn, dist);
+    k_stage_knn_warp<2><<<blocks, 128, 0, st>>>(pg.geom, pg.cell_start, pg.sorted, Q, n, rest, P, frozen, kk, ex, knn, dist);
 }
 
 // Which search: one warp per query for up to kWarpPoints points or kWarpQueries
@@ -333,7 +333,7 @@ constexpr int kWarpQueries = 50000;
 static cvt_status_t launch_knn_sites(const PointGrid& pg, int n, const uint8_t* frozen, int kk, uint32_t* knn, float* dist,
                                      cudaStream_t st) {
   if (n < kWarpPoints) {
-    launch_knn_warp(pg, nullptr, n, nullptr, frozen, kk, 0, knn, dist, st);
+    launch_knn_warp(pg, nullptr, n, nullptr, nullptr, frozen, kk, 0, knn, dist, st);
     CKLAUNCH();
     return CVT_OK;
   }
@@ -348,22 +348,22 @@ static cvt_status_t launch_knn_sites(const PointGrid& pg, int n, const uint8_t* 
   k_stage_knn_group<<<std::min(cdiv(n, 32), 20 * sm_count()), 32, 0, st>>>(pg.geom, pg.cell_start, pg.sorted, n, frozen, kk,
                                                                           knn, dist, pg.rest);
   CKLAUNCH();
-  launch_knn_warp(pg, nullptr, n, pg.rest, frozen, kk, 0, knn, dist, st);
+  launch_knn_warp(pg, nullptr, n, pg.rest, nullptr, frozen, kk, 0, knn, dist, st);
   CKLAUNCH();
   return CVT_OK;
 }
 
-// the neighbours of nQ query points among n points
-static cvt_status_t launch_knn_queries(const PointGrid& pg, const float* Q, int nQ, const uint8_t* frozen, int kk, int ex,
-                                       uint32_t* knn, float* dist, cudaStream_t st) {
+// the neighbours of nQ query points among the points P
+static cvt_status_t launch_knn_queries(const PointGrid& pg, const float* P, const float* Q, int nQ, const uint8_t* frozen,
+                                       int kk, int ex, uint32_t* knn, float* dist, cudaStream_t st) {
   if (nQ < kWarpQueries) {
-    launch_knn_warp(pg, Q, nQ, nullptr, frozen, kk, ex, knn, dist, st);
+    launch_knn_warp(pg, Q, nQ, nullptr, nullptr, frozen, kk, ex, knn, dist, st);
     CKLAUNCH();
     return CVT_OK;
   }
   KK_DISPATCH(kk, launch_knn_query, pg, Q, nQ, frozen, kk, ex, knn, dist, st);
   CKLAUNCH();
-  launch_knn_warp(pg, Q, nQ, pg.rest, frozen, kk, ex, knn, dist, st);
+  launch_knn_warp(pg, Q, nQ, pg.rest, P, frozen, kk, ex, knn, dist, st);
   CKLAUNCH();
   return CVT_OK;
 }
@@ -390,7 +390,7 @@ extern "C" cvt_status_t cvt_knn_query_to_points(const float* cand, int n_cand, c
   PointGrid pg;
   cvt_status_t s = build_point_grid(sc, cand, n_cand, 0.2f * kk + 1.f, nullptr, pg, n_query);
   if (s != CVT_OK) return s;
-  return launch_knn_queries(pg, query, n_query, frozen, kk, 0, knn, dist, st);
+  return launch_knn_queries(pg, cand, query, n_query, frozen, kk, 0, knn, dist, st);
 }
 
 extern "C" cvt_status_t cvt_knn_vertices(const float* V, int nV, const float* Q, int nQ, int k, int exclude_self,
@@ -404,7 +404,7 @@ extern "C" cvt_status_t cvt_knn_vertices(const float* V, int nV, const float* Q,
   cvt_status_t s = build_point_grid(sc, V, nV, 0.2f * k + 1.f, nullptr, pg, nQ);
   if (s != CVT_OK) return s;
   // int output: the uint32 sentinel 0xFFFFFFFF reads as -1
-  return launch_knn_queries(pg, Q, nQ, frozen, k, exclude_self ? 1 : 0, reinterpret_cast<uint32_t*>(out), nullptr, st);
+  return launch_knn_queries(pg, V, Q, nQ, frozen, k, exclude_self ? 1 : 0, reinterpret_cast<uint32_t*>(out), nullptr, st);
 }
 
 extern "C" cvt_status_t cvt_knn_drop_self(const uint32_t* in, int n, int kin, int kout, uint32_t* out, void* stream) {

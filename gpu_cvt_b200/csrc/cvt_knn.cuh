@@ -192,18 +192,19 @@ __device__ __forceinline__ bool group_knn(const GridGeom& g, int gkey, const int
 }
 
 // The k <= 32 R nearest of q by one warp, ring by ring as in warp_knn
-// (cvt_grid.cuh) with a run-time k; after rlim rings it scans all n_pts points
-// instead (a query far from them would visit the grid cell by cell).
+// (cvt_grid.cuh) with a run-time k, from ring `first` on (list: the nearest of
+// the rings before it; empty for first = 1).  far > 0: a query whose rings take
+// more than far look-ups of cell ranges scans all n_pts points instead; at once
+// when its distance from the grid alone asks for so many.
 template <class T, class PT, int R, class Accept>
 __device__ __forceinline__ void warp_knn_k(const GridGeom& g, const int* __restrict__ cell_start,
                                            const Pt4<PT>* __restrict__ pts, int n_pts, V3<T> q, int k, int lane,
-                                           Accept accept, int rlim, typename KeyOps<T>::Key (&list)[R]) {
+                                           Accept accept, int first, float far, typename KeyOps<T>::Key (&list)[R]) {
   using O = KeyOps<T>;
   using Key = typename O::Key;
-#pragma unroll
-  for (int r = 0; r < R; ++r) list[r] = O::empty();
   if (!finite3(q)) return;
-  Key kth = O::empty();
+  auto last_key = [&]() { return shfl_key((k - 1) / 32 == 0 ? list[0] : list[R - 1], (k - 1) % 32); };
+  Key kth = last_key();
   auto visit = [&](int pos) {
     Key key = O::empty();
     bool pass = false;
@@ -229,25 +230,39 @@ __device__ __forceinline__ void warp_knn_k(const GridGeom& g, const int* __restr
         list[r] = O::kmax(prev, O::kmin(list[r], x));
       }
     }
-    kth = shfl_key((k - 1) / 32 == 0 ? list[0] : list[R - 1], (k - 1) % 32);
+    kth = last_key();
   };
   const int c[3] = {grid_coord(g, q.x, 0), grid_coord(g, q.y, 1), grid_coord(g, q.z, 2)};
   const float qf[3] = {(float)q.x, (float)q.y, (float)q.z};
   const int rmax = max(g.dim[0], max(g.dim[1], g.dim[2]));
-  for (int ring = 1; ring <= rmax; ++ring) {
+  // ranges that warp_ring looks up in ring r: two per row
+  auto ranges = [&](int r) {
+    return 2.f * (float)((min(c[1] + r, g.dim[1] - 1) - max(c[1] - r, 0) + 1) *
+                         (min(c[2] + r, g.dim[2] - 1) - max(c[2] - r, 0) + 1));
+  };
+  float looked = 0.f;
+  if (far > 0.f) {
+    float out2 = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float d = fmaxf(fmaxf(g.lo[a] - qf[a], qf[a] - (g.lo[a] + (float)g.dim[a] * g.h)), 0.f);
+      out2 = fmaT(d, d, out2);
+    }
+    const int rings = (int)fminf(__fsqrt_rn(out2) * g.inv_h, (float)rmax);
+    if ((float)rings * ranges(rings) > 3.f * far) looked = INFINITY;
+  }
+  for (int ring = first; !(looked > far) && ring <= rmax; ++ring) {
     warp_ring(g, cell_start, c[0], c[1], c[2], ring, lane, visit);
     const float m = ring_margin(g, qf, c, ring) - 1e-3f * g.h;
     if (isinf(m)) return;
     if (!O::is_empty(kth) && m > 0.f && (double)O::dist(kth) < (double)m * (double)m) return;
-    if (ring == rlim) {
-      // a query far from the points: one pass over all of them
-#pragma unroll
-      for (int r = 0; r < R; ++r) list[r] = O::empty();
-      kth = O::empty();
-      for (int b = 0; b < n_pts; b += 32) visit(b + lane < n_pts ? b + lane : -1);
-      return;
-    }
+    if (far > 0.f) looked += ranges(ring);
   }
+  if (!(looked > far)) return;
+#pragma unroll
+  for (int r = 0; r < R; ++r) list[r] = O::empty();
+  kth = O::empty();
+  for (int b = 0; b < n_pts; b += 32) visit(b + lane < n_pts ? b + lane : -1);
 }
 
 }  // namespace cvt

@@ -147,8 +147,17 @@ __global__ void __launch_bounds__(128) k_stage_knn_points(const GridGeom* geom, 
 // queries are separate points; out_int != 0 writes int (-1 for missing).  A
 // query that has not ended after kQueryRings rings is far from the points (a
 // centroid of an unbounded cell: its thread would walk the whole grid, several
-// milliseconds) and is left to k_stage_knn_warp: rest[0] = count, then queries.
+// milliseconds) and is left to k_stage_knn_warp with what it found in its row
+// of knn: rest[0] = count, then queries.
 constexpr int kQueryRings = 4;
+
+// Cell ranges that a warp looks up for a query before it scans all points, per
+// point.  30k queries, k = 5, rings / scans / one thread each (ms): 14 cells off
+// 164k points 0.40, 10.6, 4.0; 40 cells off 1M points 2.7, 65, 36; a query with
+// only empty cells around it pays for the rings and the scan (60 cells inside
+// the sphere of 164k points 14.7, 11.0, 100; with 1/2 a query 60 cells off 20k
+// points takes 2.7 instead of 1.6).
+constexpr float kFarLookups = 0.125f;
 template <int KK>
 __global__ void __launch_bounds__(128) k_stage_knn_query(const GridGeom* geom, const int* __restrict__ cell_start,
                                                          const Pt4<float>* __restrict__ sorted, const float* __restrict__ Q,
@@ -161,10 +170,8 @@ __global__ void __launch_bounds__(128) k_stage_knn_query(const GridGeom* geom, c
   const GridGeom G = *geom;
   const int skip = exclude_self ? qi : -1;
   if (!grid_knn<float, float, KK>(G, cell_start, sorted, ld3(Q, qi), top, [skip](uint32_t id) { return (int)id != skip; },
-                                  kQueryRings)) {
+                                  kQueryRings))
     rest[1 + atomicAdd(rest, 1)] = qi;
-    return;
-  }
 #pragma unroll
   for (int k = 0; k < KK; ++k) {
     if (k >= kk) break;
@@ -177,11 +184,14 @@ __global__ void __launch_bounds__(128) k_stage_knn_query(const GridGeom* geom, c
 // rest == NULL all n.  Q == NULL: query w is the w-th of the cell-ordered
 // points.  Few queries (one thread each would leave most of the chip idle for
 // the length of one thread's search) and those that the other kernels leave.
+// P != NULL: the queries that k_stage_knn_query left, P the points by index;
+// the search goes on where that kernel stopped.
 template <int R>
 __global__ void __launch_bounds__(128) k_stage_knn_warp(const GridGeom* geom, const int* __restrict__ cell_start,
                                                         const Pt4<float>* __restrict__ sorted, const float* __restrict__ Q,
-                                                        int n, const int* __restrict__ rest, const uint8_t* frozen, int kk,
-                                                        int exclude_self, uint32_t* knn, float* dist) {
+                                                        int n, const int* __restrict__ rest, const float* __restrict__ P,
+                                                        const uint8_t* frozen, int kk, int exclude_self, uint32_t* knn,
+                                                        float* dist) {
   const int lane = threadIdx.x & 31;
   const int nw = (int)((gridDim.x * 128u) >> 5);
   const GridGeom G = *geom;
@@ -201,8 +211,17 @@ __global__ void __launch_bounds__(128) k_stage_knn_warp(const GridGeom* geom, co
     }
     if (frozen && frozen[row]) continue;
     unsigned long long list[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int e = 32 * r + lane;
+      list[r] = KeyOps<float>::empty();
+      if (P && e < kk) {
+        const uint32_t id = knn[(size_t)row * kk + e];
+        if (id != 0xffffffffu) list[r] = KeyOps<float>::make(dist2(ld3(P, id), q), id);
+      }
+    }
     warp_knn_k<float, float, R>(G, cell_start, sorted, n_pts, q, kk, lane, [skip](uint32_t id) { return (int)id != skip; },
-                                Q ? kQueryRings : 0, list);
+                                P ? kQueryRings + 1 : 1, Q ? kFarLookups * (float)n_pts : 0.f, list);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int e = 32 * r + lane;
