@@ -319,20 +319,30 @@ static void launch_knn_warp(const PointGrid& pg, const float* Q, int n, const in
     k_stage_knn_warp<2><<<blocks, 128, 0, st>>>(pg.geom, pg.cell_start, pg.sorted, Q, n, rest, P, frozen, kk, ex, knn, dist);
 }
 
-// Which search: one warp per query for up to kWarpPoints points or kWarpQueries
-// queries; more points with 10 to 40 neighbours each go in groups of 32, the
-// rest one thread each with its list in registers.  Measured, warp against the
-// other (us): 2k points, K = 21: 13, 67 (thread); 30k, K = 25: 73, 129
-// (group); 100k: about 240, 169 (group; thread 178); 1M, K = 33: group 1424,
-// thread 2174.  5 nearest of 250k vertices for 2k queries: 14, 135 (thread);
-// 30k: 60, 94; 60k: 112, 93.
-constexpr int kWarpPoints = 60000;
-constexpr int kWarpQueries = 50000;
+// Which search: one warp per query for few of them (one thread each leaves
+// most of the chip idle for the length of one thread's search), beyond that
+// groups of 32 points for 10 to 40 neighbours of the points themselves, else one
+// thread each with its list in registers.  The lines are where the measured
+// times of both sides cross (us; torus and sphere agree within 10 %):
+//   points, warp / thread: K = 1, 10k 84 / 81, 20k 98 / 83; K = 5, 20k 98 / 99,
+//     30k 114 / 99; K = 9, 30k 115 / 126, 40k 134 / 118; K = 64, 130k 1130 / 1261
+//   points, warp / group: K = 10, 45k 143 / 146, 55k 166 / 151; K = 25, 45k
+//     188 / 186, 55k 210 / 194; K = 33 (two list registers per lane from here
+//     on), 25k 195 / 204, 30k 220 / 203, 50k 309 / 237; K = 40, 30k 241 / 243
+//   queries on the surface, warp / thread (more points miss the caches, which
+//     threads hide less): K = 5, 800 points, 20k 69 / 71, 30k 83 / 67; 20k
+//     points, 30k 85 / 93, 40k 99 / 90; 252k points, 45k 134 / 141, 60k 161 /
+//     141; 1M points, 50k 186 / 223; K = 16, 800 points, 35k 129 / 117; 5k
+//     points, 60k 166 / 189, 80k 205 / 214
+static int warp_points(int kk) {
+  return kk <= 1 ? 10000 : kk <= 5 ? 20000 : kk <= 9 ? 32000 : kk <= 32 ? 50000 : kk <= 40 ? 30000 : 130000;
+}
+static int warp_queries(int n, int kk) { return (int)((kk <= 9 ? 8600.0 : 15000.0) * std::pow((double)n, 0.14)); }
 
 // the points' own neighbours
 static cvt_status_t launch_knn_sites(const PointGrid& pg, int n, const uint8_t* frozen, int kk, uint32_t* knn, float* dist,
                                      cudaStream_t st) {
-  if (n < kWarpPoints) {
+  if (n < warp_points(kk)) {
     launch_knn_warp(pg, nullptr, n, nullptr, nullptr, frozen, kk, 0, knn, dist, st);
     CKLAUNCH();
     return CVT_OK;
@@ -353,10 +363,10 @@ static cvt_status_t launch_knn_sites(const PointGrid& pg, int n, const uint8_t* 
   return CVT_OK;
 }
 
-// the neighbours of nQ query points among the points P
-static cvt_status_t launch_knn_queries(const PointGrid& pg, const float* P, const float* Q, int nQ, const uint8_t* frozen,
-                                       int kk, int ex, uint32_t* knn, float* dist, cudaStream_t st) {
-  if (nQ < kWarpQueries) {
+// the neighbours of nQ query points among the n points P
+static cvt_status_t launch_knn_queries(const PointGrid& pg, const float* P, int n, const float* Q, int nQ,
+                                       const uint8_t* frozen, int kk, int ex, uint32_t* knn, float* dist, cudaStream_t st) {
+  if (nQ < warp_queries(n, kk)) {
     launch_knn_warp(pg, Q, nQ, nullptr, nullptr, frozen, kk, ex, knn, dist, st);
     CKLAUNCH();
     return CVT_OK;
@@ -390,7 +400,7 @@ extern "C" cvt_status_t cvt_knn_query_to_points(const float* cand, int n_cand, c
   PointGrid pg;
   cvt_status_t s = build_point_grid(sc, cand, n_cand, 0.2f * kk + 1.f, nullptr, pg, n_query);
   if (s != CVT_OK) return s;
-  return launch_knn_queries(pg, cand, query, n_query, frozen, kk, 0, knn, dist, st);
+  return launch_knn_queries(pg, cand, n_cand, query, n_query, frozen, kk, 0, knn, dist, st);
 }
 
 extern "C" cvt_status_t cvt_knn_vertices(const float* V, int nV, const float* Q, int nQ, int k, int exclude_self,
@@ -404,7 +414,7 @@ extern "C" cvt_status_t cvt_knn_vertices(const float* V, int nV, const float* Q,
   cvt_status_t s = build_point_grid(sc, V, nV, 0.2f * k + 1.f, nullptr, pg, nQ);
   if (s != CVT_OK) return s;
   // int output: the uint32 sentinel 0xFFFFFFFF reads as -1
-  return launch_knn_queries(pg, V, Q, nQ, frozen, k, exclude_self ? 1 : 0, reinterpret_cast<uint32_t*>(out), nullptr, st);
+  return launch_knn_queries(pg, V, nV, Q, nQ, frozen, k, exclude_self ? 1 : 0, reinterpret_cast<uint32_t*>(out), nullptr, st);
 }
 
 extern "C" cvt_status_t cvt_knn_drop_self(const uint32_t* in, int n, int kin, int kout, uint32_t* out, void* stream) {

@@ -145,11 +145,13 @@ __global__ void __launch_bounds__(128) k_stage_knn_points(const GridGeom* geom, 
 }
 
 // queries are separate points; out_int != 0 writes int (-1 for missing).  A
-// query that has not ended after kQueryRings rings is far from the points (a
-// centroid of an unbounded cell: its thread would walk the whole grid, several
-// milliseconds) and is left to k_stage_knn_warp with what it found in its row
-// of knn: rest[0] = count, then queries.
-constexpr int kQueryRings = 4;
+// query that has not ended after kQueryRings rings is off the points and is left
+// to k_stage_knn_warp with what it found in its row of knn: rest[0] = count,
+// then queries.  One thread's ring costs what a warp's does, and a query near
+// the points ends with the first: 100k queries, k = 5, to 1M points (us), 1 ring
+// / 2 / 4: on the surface 226 / 231 / 229, 3 cells off 322 / 570 / 572, 10 cells
+// 795 / 1021 / 2458.
+constexpr int kQueryRings = 1;
 
 // Cell ranges that a warp looks up for a query before it scans all points, per
 // point.  30k queries, k = 5, rings / scans / one thread each (ms): 14 cells off
