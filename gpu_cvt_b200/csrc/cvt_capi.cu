@@ -109,10 +109,15 @@ static cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t st) {
 }
 
 // Held while an iteration is captured and its graph instantiated or updated,
-// and around every device-wide wait and release of this library: with one
-// thread capturing and another waiting for the device, tearing an engine down
-// or ending (its streams go), the driver failed the capture or crashed (two
-// threads that create, run and destroy engines: within 150 rounds).
+// and around the library's device-wide waits, the release of its long-lived
+// memory and of cached memory, and the creation and release of streams, events
+// and graphs: with one thread capturing and another waiting for the device,
+// tearing an engine down or ending (its streams go), the driver failed the
+// capture or crashed (two threads that create, run and destroy engines: within
+// 150 rounds).  One lock for the process: a thread that has a graph to capture
+// (twice per engine and covered extent) waits while another waits for its
+// device.  Taken before g_graph_mu and g_pool_mu; nothing that takes it is
+// called with it held.
 static std::mutex g_capture_mu;
 
 static cudaError_t device_sync() {
@@ -137,6 +142,7 @@ static void dev_free_sync(void* p) {
 static void graph_cache_clear();
 
 extern "C" cvt_status_t cvt_release_cached_memory(void) {
+  std::lock_guard<std::mutex> cap(g_capture_mu);
   graph_cache_clear();
   std::lock_guard<std::mutex> lk(g_pool_mu);
   for (cudaMemPool_t pool : g_pools)
@@ -1464,8 +1470,12 @@ extern "C" cvt_status_t cvt_engine_create(const cvt_params_t* p, int max_segment
   k_fill_int<<<cdiv((long)ns, 256), 256>>>(e->d_site_seg, (int)ns, -1);
   LAUNCHED(1);
   ECK(cudaGetLastError());
-  for (cudaEvent_t* ev : {&e->ev_fork, &e->ev_grid, &e->ev_join, &e->ev_cfork, &e->ev_cgrid, &e->ev_cjoin})
-    ECK(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+  {
+    std::lock_guard<std::mutex> lk(g_capture_mu);
+    for (cudaEvent_t* ev : {&e->ev_fork, &e->ev_grid, &e->ev_join, &e->ev_cfork, &e->ev_cgrid, &e->ev_cjoin})
+      if (err == cudaSuccess) err = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  }
+  ECK(err);
   ECK(device_sync());
 #undef ECK
   *out = e;
@@ -1822,9 +1832,12 @@ static cvt_status_t cover_segments(cvt_engine* e, cudaStream_t st) {
   };
   const int cs = fit(ns, e->cov_sites, e->max_sites), cc = fit(nc, e->cov_cells, e->max_cells);
   if (cs == e->cov_sites && cc == e->cov_cells) return CVT_OK;
-  if (e->gexec[0] || e->gexec[1]) CK(cudaStreamSynchronize(st));  // no replay in flight
-  for (int k = 0; k < 2; ++k)
-    if (e->gexec[k]) { graph_cache_put(graph_key(e), e->gexec[k]); e->gexec[k] = nullptr; }
+  if (e->gexec[0] || e->gexec[1]) {
+    CK(cudaStreamSynchronize(st));  // no replay in flight
+    std::lock_guard<std::mutex> lk(g_capture_mu);
+    for (int k = 0; k < 2; ++k)
+      if (e->gexec[k]) { graph_cache_put(graph_key(e), e->gexec[k]); e->gexec[k] = nullptr; }
+  }
   e->cov_sites = cs;
   e->cov_cells = cc;
   return CVT_OK;
@@ -1886,8 +1899,20 @@ extern "C" cvt_status_t cvt_engine_profile(cvt_engine_t e, int iters, float* ms,
   CK(thread_streams(&ts));
   s = cover_segments(e, st);
   if (s != CVT_OK) return s;
-  cudaEvent_t ev[6];
-  for (int k = 0; k < 6; ++k) CK(cudaEventCreate(&ev[k]));
+  // the six events of one call, released with it
+  struct Events {
+    cudaEvent_t e[6] = {};
+    ~Events() {
+      std::lock_guard<std::mutex> lk(g_capture_mu);
+      for (cudaEvent_t x : e)
+        if (x) cudaEventDestroy(x);
+    }
+  } events;
+  cudaEvent_t* ev = events.e;
+  {
+    std::lock_guard<std::mutex> lk(g_capture_mu);
+    for (int k = 0; k < 6; ++k) CK(cudaEventCreate(&ev[k]));
+  }
   double acc[5] = {0, 0, 0, 0, 0};
   for (int it = 0; it < iters; ++it) {
     int nl = 0;
@@ -1903,7 +1928,6 @@ extern "C" cvt_status_t cvt_engine_profile(cvt_engine_t e, int iters, float* ms,
       acc[k] += t;
     }
   }
-  for (int k = 0; k < 6; ++k) cudaEventDestroy(ev[k]);
   for (int k = 0; k < 5; ++k) ms[k] = (float)(acc[k] / iters);
   return s;
 }
@@ -2163,7 +2187,12 @@ extern "C" cvt_status_t cvt_remesh_batch(int n_meshes, const float* const* V, co
     std::atomic<int> next{0};
     auto ingest = [&]() {
       cudaStream_t st = nullptr;
-      if (cudaSetDevice(dev) != cudaSuccess || cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) {
+      cudaError_t made = cudaSetDevice(dev);
+      if (made == cudaSuccess) {
+        std::lock_guard<std::mutex> lk(g_capture_mu);
+        made = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+      }
+      if (made != cudaSuccess) {
         for (int i; (i = next++) < n_meshes;) { ms[i] = CVT_ERR_CUDA; merr[i] = "cvt_remesh_batch: stream creation failed"; }
         return;
       }
@@ -2171,6 +2200,7 @@ extern "C" cvt_status_t cvt_remesh_batch(int n_meshes, const float* const* V, co
         ms[i] = mesh_create_on(V[i], nV[i], F[i], nF[i], &meshes[i], st);
         if (ms[i] != CVT_OK) merr[i] = g_last_error;
       }
+      std::lock_guard<std::mutex> lk(g_capture_mu);
       cudaStreamDestroy(st);
     };
     const int nth = std::min(n_meshes, kIngestThreads);
