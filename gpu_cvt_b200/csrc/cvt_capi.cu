@@ -29,7 +29,10 @@ using namespace cvt;
 static thread_local std::string g_last_error;
 static std::atomic<unsigned long long> g_launches{0};
 
+// (a CUDA call's error also stays behind as the thread's last error, where the
+// next launch check would take it for its own)
 static cvt_status_t fail(cvt_status_t s, const std::string& msg) {
+  if (s == CVT_ERR_CUDA || s == CVT_ERR_OOM) cudaGetLastError();
   g_last_error = msg;
   return s;
 }
