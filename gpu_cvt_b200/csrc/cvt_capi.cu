@@ -6,7 +6,9 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -1492,10 +1494,35 @@ extern "C" cvt_status_t cvt_engine_destroy(cvt_engine_t e) {
   return CVT_OK;
 }
 
-// The sites of n consecutive slots from base on, cell-ordered copy in
-// `ordered`, into the engine with their initial state (k_place_sites).
-static cvt_status_t place_sites(cvt_engine* e, const Pt4<float>* ordered, int n, int base, int seg, const int* raw_seg,
-                                cudaStream_t st) {
+// Where the caller's sites of the slots from base on are put before they are
+// placed: the centroids' array, which every iteration fills before it reads it.
+static float* raw_sites(cvt_engine* e, int base) {
+  return reinterpret_cast<float*>(reinterpret_cast<char*>(e->d_cent) + (e->f64 ? sizeof(double) : sizeof(float)) * 3 * (size_t)base);
+}
+
+// Place the sites at raw_sites(base) in the n slots from base on, in the order
+// of the cells [cell0, cell0 + cells), with their initial state: of segment
+// seg, or with seg < 0 of all segments (placed in slot order).  Scratch are
+// arrays of the engine that an iteration fills before it reads them, so an
+// engine that holds its memory takes segments without any more; the scan
+// leaves the cell counts at zero again.
+static cvt_status_t place_sites(cvt_engine* e, int base, int n, int seg, int cell0, int cells, cudaStream_t st) {
+  const float* raw = raw_sites(e, base);
+  int2* rank = e->d_cellrank + base;
+  Pt4<float>* ordered = reinterpret_cast<Pt4<float>*>(reinterpret_cast<char*>(e->d_sorted) + pt_bytes(e) * (size_t)base);
+  const int* raw_seg = nullptr;
+  if (seg < 0) {
+    k_raw_segments<<<cdiv(n, 256), 256, 0, st>>>(e->d_segs, e->max_seg, n, e->d_act);
+    CKLAUNCH();
+    raw_seg = e->d_act;
+  }
+  const SegGrid sg{seg < 0 ? e->d_geom : e->d_geom + seg, raw_seg, nullptr};
+  k_grid_count<float><<<cdiv(n, 256), 256, 0, st>>>(n, raw, sg, e->d_cell_count, rank);
+  CKLAUNCH();
+  LAUNCHED(launch_exclusive_scan(cells, e->d_cell_count + cell0, e->d_part, e->d_cell_start + cell0, st, true, e->d_tickets));
+  CK(cudaGetLastError());
+  k_grid_scatter<float><<<cdiv(n, 256), 256, 0, st>>>(n, raw, rank, e->d_cell_start, ordered);
+  CKLAUNCH();
   if (e->f64)
     k_place_sites<double><<<cdiv(n, 256), 256, 0, st>>>(engine_args<double>(e), e->parity, n, ordered, base, seg, raw_seg,
                                                        e->d_site_seg, e->d_internal_of);
@@ -1506,9 +1533,9 @@ static cvt_status_t place_sites(cvt_engine* e, const Pt4<float>* ordered, int n,
   return CVT_OK;
 }
 
-// raw (remesh_batch): only reserve the segment's slots and cells in the host
-// mirrors of a freshly created engine; the caller has all segments' sites in
-// one device array and places them at once (place_all_segments).
+// reserve_only (remesh_batch): only take the segment's slots and cells in the
+// host mirrors of a freshly created engine; the caller places all segments at
+// once (place_all_segments).
 static cvt_status_t add_segment_impl(cvt_engine* e, cvt_mesh_t mesh, const float* sites, int n, int sites_on_device,
                                      int* seg_id, cudaStream_t st, bool reserve_only) {
   if (!e || !mesh || (!sites && !reserve_only) || n < 1 || !seg_id) return fail(CVT_ERR_INVALID, "cvt_engine_add_segment: bad arguments");
@@ -1558,22 +1585,10 @@ static cvt_status_t add_segment_impl(cvt_engine* e, cvt_mesh_t mesh, const float
   CK(cudaMemcpyAsync(e->d_segs + s, &e->segs[s], sizeof(SegDev), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(e->d_geom + s, &e->geom[s], sizeof(GridGeom), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(e->d_meshes + s, &md, sizeof(MeshDev), cudaMemcpyHostToDevice, st));
-  {
-    Scratch sc(st);
-    const float* src = sites;
-    if (!sites_on_device) {
-      float* tmp;
-      CK(sc.get(&tmp, 3 * (size_t)n));
-      CK(cudaMemcpyAsync(tmp, sites, sizeof(float) * 3 * (size_t)n, cudaMemcpyHostToDevice, st));
-      src = tmp;
-    }
-    GridGeom own = g;
-    own.cell_base = 0;
-    PointGrid pg;
-    cvt_status_t r = build_point_grid(sc, src, n, 0.f, &own, pg);
-    if (r == CVT_OK) r = place_sites(e, pg.sorted, n, base, s, nullptr, st);
-    if (r != CVT_OK) return r;
-  }
+  CK(cudaMemcpyAsync(raw_sites(e, base), sites, sizeof(float) * 3 * (size_t)n,
+                     sites_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
+  cvt_status_t r = place_sites(e, base, n, s, cbase, cells, st);
+  if (r != CVT_OK) return r;
   if (e->d_blockmax)  // no motion recorded in the segment's blocks
     CK(cudaMemsetAsync(e->d_blockmax + cbase, 0, sizeof(unsigned long long) * (size_t)cells, st));
   CK(cudaMemsetAsync(e->d_stats + (size_t)s * kStatsRing * kStatsWords, 0, sizeof(int) * kStatsRing * kStatsWords, st));
@@ -1588,11 +1603,11 @@ extern "C" cvt_status_t cvt_engine_add_segment(cvt_engine_t e, cvt_mesh_t mesh, 
   return add_segment_impl(e, mesh, sites, n, sites_on_device, seg_id, S_(stream), false);
 }
 
-// Fill a freshly created engine whose segments were reserved in slot order:
-// the device tables from the host mirrors in four copies (each small copy
-// from pageable memory waits for the stream), and every segment's sites (raw:
-// n sites in slot order) through one grid build over all of them.
-static cvt_status_t place_all_segments(cvt_engine* e, const float* raw, int n, cudaStream_t st) {
+// Fill a freshly created engine whose segments were reserved in slot order,
+// their sites at raw_sites: the device tables from the host mirrors in four
+// copies (each small copy from pageable memory waits for the stream), and
+// every segment's sites through one grid build over all of them.
+static cvt_status_t place_all_segments(cvt_engine* e, cudaStream_t st) {
   std::vector<MeshDev> md(e->max_seg);
   for (int k = 0; k < e->max_seg; ++k)
     if (e->seg_mesh[k]) md[k] = e->seg_mesh[k]->dev();
@@ -1600,22 +1615,7 @@ static cvt_status_t place_all_segments(cvt_engine* e, const float* raw, int n, c
   CK(cudaMemcpyAsync(e->d_geom, e->geom.data(), sizeof(GridGeom) * e->max_seg, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(e->d_meshes, md.data(), sizeof(MeshDev) * e->max_seg, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(e->d_active, e->active.data(), sizeof(int) * e->max_seg, cudaMemcpyHostToDevice, st));
-  Scratch sc(st);
-  int* seg;
-  int2* rank;
-  Pt4<float>* ordered;
-  CK(sc.get(&seg, (size_t)n));
-  CK(sc.get(&rank, (size_t)n));
-  CK(sc.get(&ordered, (size_t)n));
-  k_raw_segments<<<cdiv(n, 256), 256, 0, st>>>(e->d_segs, e->max_seg, n, seg);
-  CKLAUNCH();
-  // the engine's own cell arrays: the scan leaves the counts at zero again
-  k_grid_count<float><<<cdiv(n, 256), 256, 0, st>>>(n, raw, SegGrid{e->d_geom, seg, nullptr}, e->d_cell_count, rank);
-  CKLAUNCH();
-  LAUNCHED(launch_exclusive_scan(e->max_cells, e->d_cell_count, e->d_part, e->d_cell_start, st, true, e->d_tickets));
-  k_grid_scatter<float><<<cdiv(n, 256), 256, 0, st>>>(n, raw, rank, e->d_cell_start, ordered);
-  CKLAUNCH();
-  cvt_status_t r = place_sites(e, ordered, n, 0, -1, seg, st);
+  cvt_status_t r = place_sites(e, 0, e->max_sites, -1, 0, e->max_cells, st);
   if (r != CVT_OK) return r;
   CK(cudaStreamSynchronize(st));
   return CVT_OK;
@@ -1949,42 +1949,108 @@ static cvt_status_t seg_sites_buffer(cvt_engine* e, int s, cudaStream_t st, int*
   return CVT_OK;
 }
 
+// The same read into host memory without device memory: the segment's slots of
+// buffer par as they are, put into the caller's order here.
+template <class T, class O>
+static cvt_status_t read_sites(cvt_engine* e, const SegDev& sd, int par, O* out, cudaStream_t st) {
+  const size_t n = sd.n_sites;
+  std::unique_ptr<Pt4<T>[]> h(new (std::nothrow) Pt4<T>[n]);
+  if (!h) return fail(CVT_ERR_OOM, "cvt_engine_get_sites: out of host memory");
+  CK(cudaMemcpyAsync(h.get(), (const Pt4<T>*)e->d_S[par] + sd.site_base, sizeof(Pt4<T>) * n, cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  for (size_t i = 0; i < n; ++i) {
+    O* o = out + 3 * (size_t)(h[i].id - (uint32_t)sd.site_base);
+    o[0] = (O)h[i].x; o[1] = (O)h[i].y; o[2] = (O)h[i].z;
+  }
+  return CVT_OK;
+}
+
+// Sites of segment s as O, in the caller's order.  A kernel reorders them, on
+// the way through scratch unless it can write to out itself; where there is
+// no memory for that the host reorders them, so a program at its memory limit
+// still reads its sites.
+template <class T, class O>
+static cvt_status_t get_sites(cvt_engine* e, int s, O* out, bool on_device, cudaStream_t st) {
+  const SegDev& sd = e->segs[s];
+  const size_t bytes = sizeof(O) * 3 * (size_t)sd.n_sites;
+  bool direct = false;
+  if (on_device) {
+    cudaPointerAttributes at{};
+    CK(cudaPointerGetAttributes(&at, out));
+    if (at.type == cudaMemoryTypeUnregistered)
+      return fail(CVT_ERR_INVALID, "cvt_engine_get_sites: out is not memory that the device can write");
+    direct = at.type != cudaMemoryTypeDevice || at.device == e->dev;
+  }
+  Scratch sc(st);
+  O* to = out;
+  int par = 0;
+  if (!direct) {
+    const cudaError_t ae = sc.get(&to, 3 * (size_t)sd.n_sites);
+    if (ae == cudaErrorMemoryAllocation) {
+      cudaGetLastError();  // answered below
+      cvt_status_t r = seg_sites_buffer(e, s, st, &par);
+      if (r != CVT_OK) return r;
+      if (!on_device) return read_sites<T>(e, sd, par, out, st);
+      std::unique_ptr<O[]> h(new (std::nothrow) O[3 * (size_t)sd.n_sites]);
+      if (!h) return fail(CVT_ERR_OOM, "cvt_engine_get_sites: out of host memory");
+      r = read_sites<T>(e, sd, par, h.get(), st);
+      if (r != CVT_OK) return r;
+      CK(cudaMemcpy(out, h.get(), bytes, cudaMemcpyHostToDevice));
+      return CVT_OK;
+    }
+    CK(ae);
+  }
+  k_export_sites<<<cdiv(sd.n_sites, 256), 256, 0, st>>>(engine_args<T>(e), sd.site_base, sd.n_sites, to);
+  CKLAUNCH();
+  if (!direct) CK(cudaMemcpyAsync(out, to, bytes, on_device ? cudaMemcpyDefault : cudaMemcpyDeviceToHost, st));
+  return seg_sites_buffer(e, s, st, &par);  // the iteration count, and the wait
+}
+
 extern "C" cvt_status_t cvt_engine_get_sites(cvt_engine_t e, int s, float* out, int out_on_device, void* stream) {
   if (!e || !out || s < 0 || s >= e->max_seg || !e->seg_mesh[s]) return fail(CVT_ERR_INVALID, "cvt_engine_get_sites: bad arguments");
-  cudaStream_t st = S_(stream);
-  const SegDev& sd = e->segs[s];
-  size_t cnt = 3 * (size_t)sd.n_sites;
-  int par = 0;
-  cvt_status_t ps = seg_sites_buffer(e, s, st, &par);
-  if (ps != CVT_OK) return ps;
-  Scratch sc(st);
-  float* tmp = out;
-  if (!out_on_device) CK(sc.get(&tmp, cnt));
-  if (e->f64)
-    k_export_sites<<<cdiv(sd.n_sites, 256), 256, 0, st>>>(engine_args<double>(e), sd.site_base, sd.n_sites, tmp);
-  else
-    k_export_sites<<<cdiv(sd.n_sites, 256), 256, 0, st>>>(engine_args<float>(e), sd.site_base, sd.n_sites, tmp);
-  CKLAUNCH();
-  if (!out_on_device) CK(cudaMemcpyAsync(out, tmp, sizeof(float) * cnt, cudaMemcpyDeviceToHost, st));
-  if (!out_on_device) CK(cudaStreamSynchronize(st));
-  return CVT_OK;
+  if (e->f64) return get_sites<double>(e, s, out, out_on_device != 0, S_(stream));
+  return get_sites<float>(e, s, out, out_on_device != 0, S_(stream));
 }
 
 extern "C" cvt_status_t cvt_engine_get_sites_f64(cvt_engine_t e, int s, double* out, void* stream) {
   if (!e || !out || s < 0 || s >= e->max_seg || !e->seg_mesh[s] || !e->f64)
     return fail(CVT_ERR_INVALID, "cvt_engine_get_sites_f64: bad arguments (FP64 engines only)");
-  cudaStream_t st = S_(stream);
+  return get_sites<double>(e, s, out, false, S_(stream));
+}
+
+// cvt_engine_get_state without device memory: the arrays as they are, put into
+// the caller's order and indices here (see k_export_state).
+template <class T>
+static cvt_status_t read_state(cvt_engine* e, int s, uint32_t* knn, int* knnv, uint8_t* frozen, uint8_t* tier, cudaStream_t st) {
   const SegDev& sd = e->segs[s];
+  const size_t n = sd.n_sites, base = sd.site_base, row = sizeof(int) * n, pitch = sizeof(int) * (size_t)e->max_sites;
   int par = 0;
-  cvt_status_t ps = seg_sites_buffer(e, s, st, &par);
-  if (ps != CVT_OK) return ps;
-  Scratch sc(st);
-  double* tmp;
-  CK(sc.get(&tmp, 3 * (size_t)sd.n_sites));
-  k_export_sites<<<cdiv(sd.n_sites, 256), 256, 0, st>>>(engine_args<double>(e), sd.site_base, sd.n_sites, tmp);
-  CKLAUNCH();
-  CK(cudaMemcpyAsync(out, tmp, sizeof(double) * 3 * (size_t)sd.n_sites, cudaMemcpyDeviceToHost, st));
+  cvt_status_t r = seg_sites_buffer(e, s, st, &par);
+  if (r != CVT_OK) return r;
+  std::unique_ptr<Pt4<T>[]> S(new (std::nothrow) Pt4<T>[n]);
+  std::unique_ptr<uint32_t[]> list(new (std::nothrow) uint32_t[knn ? (size_t)e->K * n : 1]);
+  std::unique_ptr<int[]> kv(new (std::nothrow) int[knnv ? kKProj * n : 1]);
+  std::unique_ptr<uint8_t[]> fr(new (std::nothrow) uint8_t[n]), ti(new (std::nothrow) uint8_t[n]);
+  if (!S || !list || !kv || !fr || !ti) return fail(CVT_ERR_OOM, "cvt_engine_get_state: out of host memory");
+  CK(cudaMemcpyAsync(S.get(), (const Pt4<T>*)e->d_S[par] + base, sizeof(Pt4<T>) * n, cudaMemcpyDeviceToHost, st));
+  if (knn) CK(cudaMemcpy2DAsync(list.get(), row, e->d_list + base, pitch, row, e->K, cudaMemcpyDeviceToHost, st));
+  if (knnv) CK(cudaMemcpy2DAsync(kv.get(), row, e->d_knnv + base, pitch, row, kKProj, cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(fr.get(), e->d_frozen + base, n, cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(ti.get(), e->d_tier + base, n, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  const bool lists = e->host_iters[s] > 0;  // before the first iteration there are none
+  for (size_t i = 0; i < n; ++i) {
+    const size_t o = S[i].id - (uint32_t)base;
+    if (knn)
+      for (int t = 0; t < e->K; ++t) {
+        const uint32_t j = lists ? list[t * n + i] : 0u;
+        knn[o * e->K + t] = !lists || j == 0xffffffffu ? j : S[j - base].id - (uint32_t)base;
+      }
+    if (knnv)
+      for (int k = 0; k < kKProj; ++k) knnv[o * kKProj + k] = kv[k * n + i];
+    if (frozen) frozen[o] = fr[i];
+    if (tier) tier[o] = ti[i];
+  }
   return CVT_OK;
 }
 
@@ -1993,20 +2059,25 @@ extern "C" cvt_status_t cvt_engine_get_state(cvt_engine_t e, int s, uint32_t* kn
   if (!e || s < 0 || s >= e->max_seg || !e->seg_mesh[s]) return fail(CVT_ERR_INVALID, "cvt_engine_get_state: bad segment");
   cudaStream_t st = S_(stream);
   const SegDev& sd = e->segs[s];
-  const size_t n = sd.n_sites;
+  const size_t n = sd.n_sites, nk = knn ? e->K * n : 0, nv = knnv ? kKProj * n : 0;
   Scratch sc(st);
-  uint32_t* tk = nullptr;
-  int* tv = nullptr;
-  uint8_t *tf = nullptr, *tt = nullptr;
-  if (knn) CK(sc.get(&tk, (size_t)e->K * n));
-  if (knnv) CK(sc.get(&tv, kKProj * n));
-  if (frozen) CK(sc.get(&tf, n));
-  if (tier) CK(sc.get(&tt, n));
-  if (e->f64) k_export_state<<<cdiv((long)n, 128), 128, 0, st>>>(engine_args<double>(e), s, tk, tv, tf, tt);
-  else k_export_state<<<cdiv((long)n, 128), 128, 0, st>>>(engine_args<float>(e), s, tk, tv, tf, tt);
+  uint32_t* tk;  // the lists, then the vertices, frozen flags and tiers
+  const cudaError_t ae = sc.get(&tk, nk + nv + n / 2 + 1);
+  if (ae == cudaErrorMemoryAllocation) {
+    cudaGetLastError();  // the host reorders instead
+    return e->f64 ? read_state<double>(e, s, knn, knnv, frozen, tier, st) : read_state<float>(e, s, knn, knnv, frozen, tier, st);
+  }
+  CK(ae);
+  int* tv = reinterpret_cast<int*>(tk + nk);
+  uint8_t *tf = reinterpret_cast<uint8_t*>(tv + nv), *tt = tf + n;
+  uint32_t* dk = knn ? tk : nullptr;
+  int* dv = knnv ? tv : nullptr;
+  uint8_t *df = frozen ? tf : nullptr, *dt = tier ? tt : nullptr;
+  if (e->f64) k_export_state<<<cdiv((long)n, 128), 128, 0, st>>>(engine_args<double>(e), s, dk, dv, df, dt);
+  else k_export_state<<<cdiv((long)n, 128), 128, 0, st>>>(engine_args<float>(e), s, dk, dv, df, dt);
   CKLAUNCH();
-  if (knn) CK(cudaMemcpyAsync(knn, tk, sizeof(uint32_t) * e->K * n, cudaMemcpyDeviceToHost, st));
-  if (knnv) CK(cudaMemcpyAsync(knnv, tv, sizeof(int) * kKProj * n, cudaMemcpyDeviceToHost, st));
+  if (knn) CK(cudaMemcpyAsync(knn, tk, sizeof(uint32_t) * nk, cudaMemcpyDeviceToHost, st));
+  if (knnv) CK(cudaMemcpyAsync(knnv, tv, sizeof(int) * nv, cudaMemcpyDeviceToHost, st));
   if (frozen) CK(cudaMemcpyAsync(frozen, tf, n, cudaMemcpyDeviceToHost, st));
   if (tier) CK(cudaMemcpyAsync(tier, tt, n, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
@@ -2141,22 +2212,19 @@ constexpr int kIngestThreads = 8;
 // The sites of every reserved segment (slot order) from its host array.
 static cvt_status_t upload_and_place(cvt_engine* e, const int* seg, int n, const float* const* sites, const int* n_sites) {
   cudaStream_t st = S_(nullptr);
-  Scratch sc(st);
-  float* raw;
-  CK(sc.get(&raw, 3 * (size_t)e->max_sites));
+  float* raw = raw_sites(e, 0);
   for (int i = 0; i < n; ++i)
     CK(cudaMemcpyAsync(raw + 3 * (size_t)e->segs[seg[i]].site_base, sites[i], sizeof(float) * 3 * (size_t)n_sites[i],
                        cudaMemcpyHostToDevice, st));
-  return place_all_segments(e, raw, e->max_sites, st);
+  return place_all_segments(e, st);
 }
 
-// Every segment's sites into its host array: one kernel for all and one wait
-// at the end (cvt_engine_get_sites waits twice per segment).
+// Every segment's sites into its host array: one kernel for all, through the
+// centroids' array of the engine, which no iteration uses any more, and one
+// wait at the end (cvt_engine_get_sites waits twice per segment).
 static cvt_status_t engine_get_sites_all(cvt_engine* e, const int* seg, int n, float* const* out) {
   cudaStream_t st = S_(nullptr);
-  Scratch sc(st);
-  float* tmp;
-  CK(sc.get(&tmp, 3 * (size_t)e->max_sites));
+  float* tmp = raw_sites(e, 0);
   if (e->f64) k_export_sites<<<cdiv(e->max_sites, 256), 256, 0, st>>>(engine_args<double>(e), 0, e->max_sites, tmp);
   else k_export_sites<<<cdiv(e->max_sites, 256), 256, 0, st>>>(engine_args<float>(e), 0, e->max_sites, tmp);
   CKLAUNCH();

@@ -328,7 +328,11 @@ cvt_status_t cvt_engine_remove_segment(cvt_engine_t e, int seg_id);
  * from two threads at once. */
 cvt_status_t cvt_engine_run(cvt_engine_t e, int iters, void* stream);
 /* Copy a segment's current sites out (n*3 floats; FP64 engines convert).
- * Synchronous (it reads the segment's iteration count from the device). */
+ * Synchronous (it reads the segment's iteration count from the device).
+ * out_on_device: out is memory that the device can write, else
+ * CVT_ERR_INVALID.  This read and the two below reorder on the device through
+ * temporaries of the pool, or on the host when there is no device memory for
+ * them; placing a segment takes none beyond the engine's own. */
 cvt_status_t cvt_engine_get_sites(cvt_engine_t e, int seg_id, float* out, int out_on_device, void* stream);
 /* FP64 engines: the double-precision sites (n*3 doubles, host). */
 cvt_status_t cvt_engine_get_sites_f64(cvt_engine_t e, int seg_id, double* out, void* stream);
