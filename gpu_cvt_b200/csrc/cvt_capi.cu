@@ -1319,7 +1319,7 @@ static std::vector<std::pair<GraphKey, cudaGraphExec_t>> g_graph_cache;
 
 static GraphKey graph_key(const cvt_engine* e) {
   return {e->dev, e->p.profile, e->K, e->p.knn_block, e->p.clip_block, e->p.proj_block, e->p.proj_mode,
-          e->p.frame_mode, e->p.knn_reuse != 0, e->cov_sites <= kFewSites};
+          e->p.frame_mode, e->p.knn_reuse != 0, e->cov_sites <= kFewSites[e->p.profile]};
 }
 
 static cudaGraphExec_t graph_cache_take(const GraphKey& k) {
@@ -1777,7 +1777,7 @@ static cvt_status_t enqueue_iteration_t(cvt_engine* e, int parity, cudaStream_t 
   launch_site_clip<PROF>(a, parity, ns, e->p.clip_block, e->p.frame_mode, e->num_sms, st);
   L += 2;
   if (ev) CK(cudaEventRecord(ev[3], st));
-  if (e->p.proj_mode == CVT_PROJ_ONERING && ns <= kFewSites) {
+  if (e->p.proj_mode == CVT_PROJ_ONERING && ns <= kFewSites[PROF]) {
     k_site_vsearch_lanes<PROF><<<cdiv((long)ns * kVsearchLanes, 128), 128, 0, st>>>(a, parity);
     k_site_proj_lanes<PROF><<<cdiv((long)ns * kProjLanes, 128), 128, 0, st>>>(a, parity);
     L++;

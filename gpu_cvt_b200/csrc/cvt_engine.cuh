@@ -1239,14 +1239,16 @@ __global__ void __launch_bounds__(BS, PROF == PROF_FP64 ? 1 : 1536 / BS) k_site_
   for (int k = 0; k < kKProj; ++k) kv[k * a.stride] = (int)KeyOps<T>::idx(top.k[k]);
 }
 
-// Few sites (a.n_sites <= kFewSites): the vertex search and the projection with
-// 8 lanes per site each, which shorten a site's chain of loads where one
-// thread each would leave most of the chip idle.  The same results: the lanes'
-// candidates are merged by the keys that one thread compares.  Iteration of a
-// lone segment on a 40k-face torus, lanes against threads (us, ref, K = 20):
-// 2k sites 62, 94; 8k 66, 94; 16k 70, 94; 30k 83, 94; 60k (16 lanes) 126, 98.
-// 16 lanes for the projection: 60 at 2k, 75 at 16k; 4 for the search: 79 at 2k.
-constexpr int kFewSites = 32768;
+// Few sites (a.n_sites <= kFewSites[profile]): the vertex search and the
+// projection with 8 lanes per site each, which shorten a site's chain of loads
+// where one thread each would leave most of the chip idle.  The same results:
+// the lanes' candidates are merged by the keys that one thread compares.
+// Iteration of a lone segment on a 40k-face torus, K = 20, lanes / threads (us):
+// ref 2k sites 62 / 94, 16k 72 / 85, 32k 86 / 88, 40k 95 / 88; mixed 16k 83 / 92,
+// 24k 93 / 93, 28k 96 / 94, 40k 108 / 95; fp64 16k 83 / 93, 20k 89 / 94, 24k
+// 98 / 95, 32k 102 / 96 (K = 12 and 32 cross at the same places).  16 lanes for
+// the projection: 60 at 2k, 75 at 16k; 4 for the search: 79 at 2k.
+constexpr int kFewSites[3] = {32768, 25000, 22000};
 constexpr int kVsearchLanes = 8;
 constexpr int kProjLanes = 8;
 

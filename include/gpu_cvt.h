@@ -257,9 +257,9 @@ typedef struct {
   int use_graph;      /* capture iterations in a CUDA graph */
   /* launch shapes (threads per block); results do not depend on them:
    * knn_block 64|128|256 (one warp per site), clip_block 64|128 (FP64
-   * profile: 32|64), proj_block 64|128|256 (one-ring projection: engines that
-   * cover more than 32768 sites; fewer take 8 lanes per site in one shape);
-   * 0 = default. */
+   * profile: 32|64), proj_block 64|128|256 (one-ring projection of
+   * engines that cover more than 22000 (FP64), 25000 (MIXED) or 32768 (REF)
+   * sites; smaller ones take 8 lanes per site in one shape); 0 = default. */
   int knn_block, clip_block, proj_block;
   /* options beyond the reference (defaults reproduce it):
    * proj_mode  CVT_PROJ_ONERING (0): the closest point over the one-rings of
