@@ -1221,7 +1221,7 @@ __global__ void k_export_state(EngineArgs<T> a, int seg, uint32_t* __restrict__ 
   const size_t o = S[g].id - (uint32_t)base;
   if (knn)
     for (int t = 0; t < a.K; ++t) {
-      const uint32_t j = a.list[t * a.stride + g];
+      const uint32_t j = a.list[g * a.list_site + t * a.list_entry];
       // before the first iteration there is no list yet
       knn[o * a.K + t] = sd.iter == 0 ? 0u : j == 0xffffffffu ? j : S[j].id - (uint32_t)base;
     }
@@ -1258,7 +1258,7 @@ struct cvt_engine {
   int* d_site_seg = nullptr;
   void* d_S[2] = {nullptr, nullptr};
   uint32_t* d_internal_of = nullptr;
-  uint32_t* d_list = nullptr;   // list_len() entries per site: the K-list, with knn_reuse the candidate list
+  uint32_t* d_list = nullptr;   // per site its K-list, with knn_reuse its candidate list
   uint8_t* d_same = nullptr;
   float* d_kth = nullptr;
   int* d_act = nullptr;
@@ -1637,11 +1637,16 @@ extern "C" cvt_status_t cvt_engine_remove_segment(cvt_engine_t e, int s) {
 
 constexpr int kCellCap = 16;
 
+// where entry t of site g's list is: d_list[g * list_site + t * list_entry]
+static size_t list_site(const cvt_engine* e) { return e->p.knn_reuse ? 1 : (size_t)e->K; }
+static size_t list_entry(const cvt_engine* e) { return e->p.knn_reuse ? (size_t)e->max_sites : 1; }
+
 template <class T> static EngineArgs<T> engine_args(cvt_engine* e) {
   EngineArgs<T> a;
   a.segs = e->d_segs; a.geom = e->d_geom; a.active = e->d_active; a.meshes = e->d_meshes; a.site_seg = e->d_site_seg;
   a.S[0] = (Pt4<T>*)e->d_S[0]; a.S[1] = (Pt4<T>*)e->d_S[1];
   a.internal_of = e->d_internal_of; a.stride = (size_t)e->max_sites; a.list = e->d_list;
+  a.list_site = list_site(e); a.list_entry = list_entry(e);
   a.same = e->d_same; a.kth = e->d_kth; a.act = e->d_act; a.act_count = e->d_act_count;
   a.knnv = e->d_knnv; a.nnv = e->d_nnv;
   a.frozen = e->d_frozen; a.streak = e->d_streak; a.tier = e->d_tier;
@@ -2033,7 +2038,11 @@ static cvt_status_t read_state(cvt_engine* e, int s, uint32_t* knn, int* knnv, u
   std::unique_ptr<uint8_t[]> fr(new (std::nothrow) uint8_t[n]), ti(new (std::nothrow) uint8_t[n]);
   if (!S || !list || !kv || !fr || !ti) return fail(CVT_ERR_OOM, "cvt_engine_get_state: out of host memory");
   CK(cudaMemcpyAsync(S.get(), (const Pt4<T>*)e->d_S[par] + base, sizeof(Pt4<T>) * n, cudaMemcpyDeviceToHost, st));
-  if (knn) CK(cudaMemcpy2DAsync(list.get(), row, e->d_list + base, pitch, row, e->K, cudaMemcpyDeviceToHost, st));
+  const bool rows = list_entry(e) == 1;  // (a row per site, or K rows of one entry each)
+  if (knn && rows)
+    CK(cudaMemcpyAsync(list.get(), e->d_list + base * e->K, row * e->K, cudaMemcpyDeviceToHost, st));
+  else if (knn)
+    CK(cudaMemcpy2DAsync(list.get(), row, e->d_list + base, pitch, row, e->K, cudaMemcpyDeviceToHost, st));
   if (knnv) CK(cudaMemcpy2DAsync(kv.get(), row, e->d_knnv + base, pitch, row, kKProj, cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(fr.get(), e->d_frozen + base, n, cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(ti.get(), e->d_tier + base, n, cudaMemcpyDeviceToHost, st));
@@ -2043,7 +2052,7 @@ static cvt_status_t read_state(cvt_engine* e, int s, uint32_t* knn, int* knnv, u
     const size_t o = S[i].id - (uint32_t)base;
     if (knn)
       for (int t = 0; t < e->K; ++t) {
-        const uint32_t j = lists ? list[t * n + i] : 0u;
+        const uint32_t j = lists ? list[rows ? i * e->K + t : t * n + i] : 0u;
         knn[o * e->K + t] = !lists || j == 0xffffffffu ? j : S[j - base].id - (uint32_t)base;
       }
     if (knnv)
@@ -2500,7 +2509,7 @@ static cvt_status_t engine_eval_impl(cvt_engine_t e, int s, cvt_eval_t* out, int
     std::memcpy(&hi[a], &q, 4);
   }
   float R2 = 2.0f * 0.5f * std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
-  const FaceColumns nb{e->d_list + sd.site_base, label, (size_t)e->max_sites, (uint32_t)sd.site_base};
+  const FaceLists nb{e->d_list + sd.site_base * list_site(e), label, list_site(e), list_entry(e), (uint32_t)sd.site_base};
   // before the first iteration there are no lists: the slots may still hold
   // those of a segment that was there before
   const int K = e->host_iters[s] == 0 ? 0 : e->K;

@@ -117,7 +117,13 @@ template <class T> struct EngineArgs {
   // Neighbour list per site (internal indices, 0xffffffff: none): the K
   // nearest in order, and with candidate lists (MM > 0) MM - K further ones
   // in no order; the K-list is the candidate list's head.
+  // Entry e of site g at [g * list_site + e * list_entry]: entry by entry with
+  // candidate lists, where most lists are read and rewritten by one thread per
+  // site (k_knn_verify); a row per site without, where a warp writes each list
+  // in every iteration (100k sites, K = 24: full searches 196 us entry by entry,
+  // 152 as rows, the clip 26 and 24).
   uint32_t* list;
+  size_t list_site, list_entry;
   uint8_t* same;      // list unchanged vs the previous iteration (site KNN kernels)
   float* kth;         // last K-th neighbour's squared distance per site, < 0 unknown
   int* act;           // the sites whose list is recomputed
@@ -261,9 +267,9 @@ template <class T> struct RowNeighbours {  // row-major list of local indices in
 };
 template <class T> struct ListNeighbours {  // the engine's lists
   const Pt4<T>* S;
-  const uint32_t* col;  // list + g
-  size_t stride;
-  __device__ __forceinline__ uint32_t id(int t) const { return __ldg(col + t * stride); }
+  const uint32_t* own;  // the site's first entry
+  size_t step;
+  __device__ __forceinline__ uint32_t id(int t) const { return __ldg(own + t * step); }
   __device__ __forceinline__ bool valid(uint32_t j) const { return j != 0xffffffffu; }
   __device__ __forceinline__ V3<T> pos(uint32_t j) const { return ldp(S, j); }
 };
@@ -745,7 +751,8 @@ __device__ __forceinline__ void knn_search_site(const EngineArgs<T>& a, int pari
     mk[0] = kl[0];
   }
   const Key kth = shfl_key(mk[0], KK - 1);
-  uint32_t* col = a.list + g;
+  uint32_t* col = a.list + (MM > 0 ? (size_t)g : (size_t)g * KK);  // list_site, list_entry
+  const size_t step = MM > 0 ? a.stride : 1;
   bool diff = false;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -753,8 +760,8 @@ __device__ __forceinline__ void knn_search_site(const EngineArgs<T>& a, int pari
     if (e < LEN) {
       const uint32_t id = O::idx(mk[r]);
       const uint32_t v = id == 0xffffffffu ? id : __ldg(a.internal_of + id);
-      if (e < KK) diff = diff || col[e * a.stride] != v;
-      col[e * a.stride] = v;
+      if (e < KK) diff = diff || col[e * step] != v;
+      col[e * step] = v;
     }
   }
   const unsigned changed = __ballot_sync(0xffffffffu, diff);
@@ -1035,7 +1042,7 @@ __device__ __forceinline__ bool site_clip(const EngineArgs<typename PT<PROF>::T>
   const int s = __ldg(a.site_seg + g);
   const SegDev& sd = a.segs[s];
   const MeshDev& md = a.meshes[sd.mesh];
-  const ListNeighbours<T> nb{a.S[parity], a.list + g, a.stride};
+  const ListNeighbours<T> nb{a.S[parity], a.list + g * a.list_site, a.list_entry};
   const bool fz = sd.mode != 0 && a.frozen[g];
   const V3<T> si = ldp(a.S[parity], g);
   // frame from the nearest vertex normal (frozen sites: their kept vertex
@@ -1144,7 +1151,7 @@ __device__ __forceinline__ void site_settle(const EngineArgs<typename PT<PROF>::
       if (v < 0) { out[0] = out[1] = out[2] = 0.f; return; }
       out[0] = __ldg(md.N + 3 * v); out[1] = __ldg(md.N + 3 * v + 1); out[2] = __ldg(md.N + 3 * v + 2);
     };
-    auto row = [&](int t) { return (int)a.list[t * a.stride + g]; };
+    auto row = [&](int t) { return (int)a.list[g * a.list_site + t * a.list_entry]; };
     a.tier[g] = (uint8_t)tier_of(sd.mode, g, a.K, row, normal);
   }
 

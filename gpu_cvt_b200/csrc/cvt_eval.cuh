@@ -80,13 +80,13 @@ struct FaceRows {  // row-major lists
   __device__ __forceinline__ int get(int i, int t) const { return (int)knn[(size_t)i * K + t]; }
   __device__ __forceinline__ int label(int i) const { return i; }
 };
-struct FaceColumns {  // an engine segment's lists (from its first site on)
+struct FaceLists {  // an engine segment's lists (from its first site on)
   const uint32_t* list;
   const int* labels;
-  size_t stride;
+  size_t site, entry;  // EngineArgs::list_site, list_entry
   uint32_t base;
   __device__ __forceinline__ int get(int i, int t) const {
-    const uint32_t j = list[t * stride + i];
+    const uint32_t j = list[i * site + t * entry];
     return j == 0xffffffffu ? -1 : (int)(j - base);
   }
   __device__ __forceinline__ int label(int i) const { return labels[i]; }
