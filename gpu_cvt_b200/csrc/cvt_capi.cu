@@ -1971,9 +1971,12 @@ static cvt_status_t read_sites(cvt_engine* e, const SegDev& sd, int par, O* out,
 }
 
 // Sites of segment s as O, in the caller's order.  A kernel reorders them, on
-// the way through scratch unless it can write to out itself; where there is
-// no memory for that the host reorders them, so a program at its memory limit
-// still reads its sites.
+// the way through scratch unless it can write to out itself.  Up to kHostBytes,
+// and wherever there is no memory for the scratch, the host reorders a plain
+// copy, so a program at its memory limit still reads its sites (us, kernel /
+// host: FP32 300 sites 43 / 32, 8k 68 / 62, 16k 82 / 92; FP64 2k 48 / 43, 4k
+// 53 / 56).
+constexpr size_t kHostBytes = 128 << 10;
 template <class T, class O>
 static cvt_status_t get_sites(cvt_engine* e, int s, O* out, bool on_device, cudaStream_t st) {
   const SegDev& sd = e->segs[s];
@@ -1990,9 +1993,10 @@ static cvt_status_t get_sites(cvt_engine* e, int s, O* out, bool on_device, cuda
   O* to = out;
   int par = 0;
   if (!direct) {
-    const cudaError_t ae = sc.get(&to, 3 * (size_t)sd.n_sites);
-    if (ae == cudaErrorMemoryAllocation) {
-      cudaGetLastError();  // answered below
+    const bool few = !on_device && sizeof(Pt4<T>) * (size_t)sd.n_sites <= kHostBytes;
+    const cudaError_t ae = few ? cudaSuccess : sc.get(&to, 3 * (size_t)sd.n_sites);
+    if (few || ae == cudaErrorMemoryAllocation) {
+      if (!few) cudaGetLastError();  // answered below
       cvt_status_t r = seg_sites_buffer(e, s, st, &par);
       if (r != CVT_OK) return r;
       if (!on_device) return read_sites<T>(e, sd, par, out, st);
@@ -2063,6 +2067,10 @@ static cvt_status_t read_state(cvt_engine* e, int s, uint32_t* knn, int* knnv, u
   return CVT_OK;
 }
 
+// State up to this size comes back in one copy (K = 24, us, one / four copies:
+// 300 sites 53 / 93, 8k 213 / 286, 16k 388 / 418, 30k 683 / 619).
+constexpr size_t kStateBytes = 1 << 20;
+
 extern "C" cvt_status_t cvt_engine_get_state(cvt_engine_t e, int s, uint32_t* knn, int* knnv, uint8_t* frozen,
                                              uint8_t* tier, void* stream) {
   if (!e || s < 0 || s >= e->max_seg || !e->seg_mesh[s]) return fail(CVT_ERR_INVALID, "cvt_engine_get_state: bad segment");
@@ -2085,6 +2093,21 @@ extern "C" cvt_status_t cvt_engine_get_state(cvt_engine_t e, int s, uint32_t* kn
   if (e->f64) k_export_state<<<cdiv((long)n, 128), 128, 0, st>>>(engine_args<double>(e), s, dk, dv, df, dt);
   else k_export_state<<<cdiv((long)n, 128), 128, 0, st>>>(engine_args<float>(e), s, dk, dv, df, dt);
   CKLAUNCH();
+  // few bytes: one copy (each from pageable memory waits for the stream)
+  const size_t bytes = sizeof(int) * (nk + nv) + 2 * n;
+  std::unique_ptr<unsigned char[]> h(bytes <= kStateBytes ? new (std::nothrow) unsigned char[bytes] : nullptr);
+  if (h) {
+    CK(cudaMemcpyAsync(h.get(), tk, bytes, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    const unsigned char* at = h.get();
+    if (knn) std::memcpy(knn, at, sizeof(int) * nk);
+    at += sizeof(int) * nk;
+    if (knnv) std::memcpy(knnv, at, sizeof(int) * nv);
+    at += sizeof(int) * nv;
+    if (frozen) std::memcpy(frozen, at, n);
+    if (tier) std::memcpy(tier, at + n, n);
+    return CVT_OK;
+  }
   if (knn) CK(cudaMemcpyAsync(knn, tk, sizeof(uint32_t) * nk, cudaMemcpyDeviceToHost, st));
   if (knnv) CK(cudaMemcpyAsync(knnv, tv, sizeof(int) * nv, cudaMemcpyDeviceToHost, st));
   if (frozen) CK(cudaMemcpyAsync(frozen, tf, n, cudaMemcpyDeviceToHost, st));
