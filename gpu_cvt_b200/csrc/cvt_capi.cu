@@ -270,7 +270,7 @@ static cvt_status_t enqueue_point_grid(const PointGrid& pg, const float* P, int 
     CKLAUNCH();
   }
   if (n > 0) {
-    k_grid_count<float><<<cdiv(n, 256), 256, 0, st>>>(n, P, SegGrid{pg.geom, nullptr, nullptr}, pg.cell_count, pg.cellrank);
+    k_grid_count<float><<<cdiv(n, 256), 256, 0, st>>>(n, P, SegGrid{pg.geom, nullptr}, pg.cell_count, pg.cellrank);
     CKLAUNCH();
   }
   LAUNCHED(launch_exclusive_scan(pg.total_cells, pg.cell_count, pg.part, pg.cell_start, st, false, pg.zero + 7));
@@ -645,8 +645,9 @@ static cvt_status_t mesh_ensure_bvh(cvt_mesh* m) {
                 std::string("mesh BVH: ") + cudaGetErrorString(err));
   };
   if (e != cudaSuccess) return bail(e);
-  // segments of the upper levels, one level after another; the last level's
-  // go to k_bvh_subtree
+  // segments of the upper levels, one level after another; those of one level
+  // differ by at most one triangle, so all of them split; the last level's go
+  // to k_bvh_subtree
   std::vector<BvhSeg> table{{0, nF, 0, -1, -1}};
   std::vector<std::pair<int, int>> levels{{0, 1}};  // first segment, segments
   while (true) {
@@ -656,7 +657,6 @@ static cvt_status_t mesh_ensure_bvh(cvt_mesh* m) {
     if (!split) break;
     for (int k = first; k < first + nseg; ++k) {
       BvhSeg& g = table[k];
-      if (g.count <= leaf) continue;
       g.left = g.node + 1;
       g.right = g.node + 1 + bvh_subtree_nodes(g.count / 2, leaf, memo);
     }
@@ -668,7 +668,6 @@ static cvt_status_t mesh_ensure_bvh(cvt_mesh* m) {
     }
     levels.push_back({at, (int)table.size() - at});
   }
-  // (segments of one level differ by at most one triangle, so all split)
   int sub[kSubTris + 1];
   for (int k = 0; k <= kSubTris; ++k) sub[k] = k <= leaf ? 1 : 1 + sub[k / 2] + sub[k - k / 2];
   BVHNode root;
@@ -1516,7 +1515,7 @@ static cvt_status_t place_sites(cvt_engine* e, int base, int n, int seg, int cel
     CKLAUNCH();
     raw_seg = e->d_act;
   }
-  const SegGrid sg{seg < 0 ? e->d_geom : e->d_geom + seg, raw_seg, nullptr};
+  const SegGrid sg{seg < 0 ? e->d_geom : e->d_geom + seg, raw_seg};
   k_grid_count<float><<<cdiv(n, 256), 256, 0, st>>>(n, raw, sg, e->d_cell_count, rank);
   CKLAUNCH();
   LAUNCHED(launch_exclusive_scan(cells, e->d_cell_count + cell0, e->d_part, e->d_cell_start + cell0, st, true, e->d_tickets));

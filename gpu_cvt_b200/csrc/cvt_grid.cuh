@@ -597,7 +597,6 @@ __device__ __forceinline__ bool warp_radius_knn(const GridGeom& g, const int* __
 struct SegGrid {           // the minimal per-point view the build needs
   const GridGeom* geom;    // one geometry per segment
   const int* seg_of;       // segment of each point (nullptr: all segment 0)
-  const int* active;       // per-segment state, 1 = iterating (nullptr: all)
 };
 
 template <class T>
@@ -605,10 +604,7 @@ __global__ void k_grid_count(int n, const T* __restrict__ P, SegGrid sg, int* __
                              int2* __restrict__ cellrank) {
   int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= n) return;
-  int s = sg.seg_of ? sg.seg_of[g] : 0;
-  if (s < 0 || (sg.active && sg.active[s] != 1)) { cellrank[g] = make_int2(-1, 0); return; }
-  GridGeom G = sg.geom[s];
-  int cell = grid_cell(G, ld3(P, g));
+  int cell = grid_cell(sg.geom[sg.seg_of ? sg.seg_of[g] : 0], ld3(P, g));
   int rank = atomicAdd(cell_count + cell, 1);
   cellrank[g] = make_int2(cell, rank);
 }
@@ -619,7 +615,6 @@ __global__ void k_grid_scatter(int n, const T* __restrict__ P, const int2* __res
   int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= n) return;
   int2 cr = cellrank[g];
-  if (cr.x < 0) return;
   V3<T> p = ld3(P, g);
   Pt4<T> o;
   o.x = p.x; o.y = p.y; o.z = p.z; o.id = (uint32_t)g;

@@ -141,8 +141,7 @@ __global__ void k_tri_info(const float* __restrict__ V, const int* __restrict__ 
   }
 }
 
-// One frontier segment of the id array.  node < 0: a leaf finished on an
-// earlier level (carried so that the sort keeps its triangles in place).
+// One segment of a level of the id array: its node, and the nodes of its halves.
 struct BvhSeg {
   int start, count, node, left, right;
 };
@@ -194,7 +193,6 @@ __global__ void __launch_bounds__(256) k_seg_reduce(const int* __restrict__ tids
   if (p < n) {
     s = seg_of(segs, nseg, p);
     if (threadIdx.x == 0) s0 = s;
-    if (segs[s].node < 0) s = -1;   // finished leaf: nothing to emit
   }
   __syncthreads();
   const unsigned peers = __match_any_sync(0xffffffffu, s);
@@ -243,29 +241,24 @@ __device__ __forceinline__ unsigned centroid_key(const float* __restrict__ info,
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// Nodes of this level (pre-order slots), split axis per segment (-1: leaf).
+// Nodes of an upper level (pre-order slots), whose segments all split, and the
+// split axis of each.
 __global__ void k_seg_emit(const BvhSeg* __restrict__ segs, int nseg, const int* __restrict__ acc, int leaf,
                            BVHNode* __restrict__ nodes, int* __restrict__ axis) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nseg) return;
-  const BvhSeg g = segs[s];
-  if (g.node < 0) { axis[s] = -1; return; }
-  axis[s] = seg_node(g, acc + 12 * (size_t)s, leaf, nodes);
+  axis[s] = seg_node(segs[s], acc + 12 * (size_t)s, leaf, nodes);
 }
 
-// sort keys: segment rank in the high word; within a segment that splits the
-// centroid coordinate on its axis (-0 folded into +0, monotone unsigned map),
-// else 0 so that the stable sort leaves the segment as it is
+// sort keys: segment rank in the high word, then the centroid coordinate on the
+// segment's axis (-0 folded into +0, monotone unsigned map)
 __global__ void k_seg_keys(const int* __restrict__ tids, int n, const BvhSeg* __restrict__ segs, int nseg,
                            const int* __restrict__ axis, const float* __restrict__ info,
                            unsigned long long* __restrict__ keys) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   const int s = seg_of(segs, nseg, p);
-  const int ax = axis[s];
-  unsigned lo = 0;
-  if (ax >= 0) lo = centroid_key(info, tids[p], ax);
-  keys[p] = ((unsigned long long)(unsigned)s << 32) | lo;
+  keys[p] = ((unsigned long long)(unsigned)s << 32) | centroid_key(info, tids[p], axis[s]);
 }
 
 // ---------------------------------------------------------------------------
@@ -299,7 +292,6 @@ __global__ void __launch_bounds__(kSubThreads) k_bvh_subtree(int* __restrict__ t
   extern __shared__ __align__(16) unsigned char sub_raw[];
   SubTree& T = *reinterpret_cast<SubTree*>(sub_raw);
   const BvhSeg top = segs[blockIdx.x];
-  if (top.node < 0) return;
   const int n = top.count, tx = threadIdx.x;
   int pad = 64;  // elements sorted (a power of two; thread t holds 2t and 2t + 1)
   while (pad < n) pad <<= 1;

@@ -55,29 +55,25 @@ template <int LO, int LEN, int N> __device__ __forceinline__ void sort_words(uin
 }
 
 // Radius of a box query that covers every point within squared distance thr.
-template <class T>
-__device__ __forceinline__ float query_radius(const GridGeom& g, V3<T> q, float thr_ru) {
-  const float qm = fmaxf(fabsf((float)q.x), fmaxf(fabsf((float)q.y), fabsf((float)q.z)));
+__device__ __forceinline__ float query_radius(const GridGeom& g, V3<float> q, float thr_ru) {
+  const float qm = fmaxf(fabsf(q.x), fmaxf(fabsf(q.y), fabsf(q.z)));
   return __fsqrt_ru(thr_ru) * 1.0001f + 1e-3f * g.h + 4e-7f * qm;
 }
 
-// For each lane with valid set: the points other than `self` within squared
-// distance thr of q; afterwards the lane's column holds their places, the
-// first `want` of them the nearest in (distance, id) order.  gkey names the
-// lane's grid (lanes of different grids are not walked together).  Returns
-// whether the lane's query is answered: at least want and at most kGroupCap
-// points within thr.  Every point left out is farther than every one held.
-// Warp-collective.
-template <class T, class PT>
-__device__ __forceinline__ bool group_knn(const GridGeom& g, int gkey, const int* __restrict__ cell_start,
-                                          const Pt4<PT>* __restrict__ pts, bool valid, V3<T> q, T thr, float rad,
-                                          uint32_t self, int want, GroupPlaces& L) {
+// For each lane with valid set: the points within squared distance thr of q;
+// afterwards the lane's column holds their places, the first `want` of them the
+// nearest in (distance, id) order.  Returns whether the lane's query is
+// answered: at least want and at most kGroupCap points within thr.  Every point
+// left out is farther than every one held.  Warp-collective.
+__device__ __forceinline__ bool group_knn(const GridGeom& g, const int* __restrict__ cell_start,
+                                          const Pt4<float>* __restrict__ pts, bool valid, V3<float> q, float thr,
+                                          float rad, int want, GroupPlaces& L) {
   constexpr unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  valid = valid && finite3(q) && rad < INFINITY && thr > (T)0;
+  valid = valid && finite3(q) && rad < INFINITY && thr > 0.f;
   int at[3], lo[3], hi[3];
   {
-    const float qf[3] = {(float)q.x, (float)q.y, (float)q.z};
+    const float qf[3] = {q.x, q.y, q.z};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       at[a] = valid ? grid_coord(g, qf[a], a) : 0;
@@ -89,10 +85,8 @@ __device__ __forceinline__ bool group_knn(const GridGeom& g, int gkey, const int
   int cnt = 0;
   for (unsigned pending = __ballot_sync(full, valid); pending;) {
     const int leader = __ffs(pending) - 1;
-    // (every lane takes part in every shuffle)
-    const int lkey = __shfl_sync(full, gkey, leader);
-    bool member = ((pending >> lane) & 1u) != 0u && lkey == gkey;
-#pragma unroll
+    bool member = ((pending >> lane) & 1u) != 0u;
+#pragma unroll  // (every lane takes part in every shuffle)
     for (int a = 0; a < 3; ++a) {
       const int la = __shfl_sync(full, at[a], leader);
       member = member && abs(at[a] - la) <= kGroupReach;
@@ -104,14 +98,12 @@ __device__ __forceinline__ bool group_knn(const GridGeom& g, int gkey, const int
       ulo[a] = __reduce_min_sync(full, member ? lo[a] : INT_MAX);
       uhi[a] = __reduce_max_sync(full, member ? hi[a] : INT_MIN);
     }
-    const int dx = __shfl_sync(full, g.dim[0], leader), dy = __shfl_sync(full, g.dim[1], leader);
-    const int cbase = __shfl_sync(full, g.cell_base, leader);
     const int ny = uhi[1] - ulo[1] + 1, nrows = ny * (uhi[2] - ulo[2] + 1);
     for (int r0 = 0; r0 < nrows; r0 += 32) {
       const int r = r0 + lane;
       int b = 0, e = 0;
       if (r < nrows) {
-        const int row = cbase + ((ulo[2] + r / ny) * dy + ulo[1] + r % ny) * dx;
+        const int row = g.cell_base + ((ulo[2] + r / ny) * g.dim[1] + ulo[1] + r % ny) * g.dim[0];
         b = __ldg(cell_start + row + ulo[0]);
         e = __ldg(cell_start + row + uhi[0] + 1);
       }
@@ -121,15 +113,16 @@ __device__ __forceinline__ bool group_knn(const GridGeom& g, int gkey, const int
         filled &= filled - 1;
         const int re = __shfl_sync(full, e, src);
         int i = __shfl_sync(full, b, src);
-        auto look = [&](const Pt4<PT>& p, int place) {
-          const T d = dist2(V3<T>{(T)p.x, (T)p.y, (T)p.z}, q);
-          if (member && d <= thr && p.id != self) {
+        auto look = [&](const Pt4<float>& p, int place) {
+          // (before the condition: behind `member`, all 1M searches take 11 % longer)
+          const float d = dist2(V3<float>{p.x, p.y, p.z}, q);
+          if (member && d <= thr) {
             if (cnt < kGroupCap) L.at[cnt][lane] = place;
             ++cnt;
           }
         };
         for (; i + 4 <= re; i += 4) {
-          Pt4<PT> p[4];
+          Pt4<float> p[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) p[k] = pts[i + k];
 #pragma unroll
@@ -142,15 +135,15 @@ __device__ __forceinline__ bool group_knn(const GridGeom& g, int gkey, const int
   const bool ok = valid && cnt >= want && cnt <= kGroupCap;
   if (__any_sync(full, ok)) {
     const int n = ok ? cnt : 0;
-    const float scale = 67108863.f / (float)thr;
+    const float scale = 67108863.f / thr;
     uint32_t w[kGroupCap];
 #pragma unroll
     for (int k = 0; k < kGroupCap; ++k) {
       w[k] = 0xffffffffu;
       if (k < n) {
-        const Pt4<PT> p = pts[L.at[k][lane]];
-        const T d = dist2(V3<T>{(T)p.x, (T)p.y, (T)p.z}, q);
-        w[k] = (min((uint32_t)((float)d * scale), 0x3fffffeu) << 6) | (uint32_t)k;
+        const Pt4<float> p = pts[L.at[k][lane]];
+        const float d = dist2(V3<float>{p.x, p.y, p.z}, q);
+        w[k] = (min((uint32_t)(d * scale), 0x3fffffeu) << 6) | (uint32_t)k;
       }
     }
     sort_words<0, kGroupCap>(w);
@@ -164,20 +157,20 @@ __device__ __forceinline__ bool group_knn(const GridGeom& g, int gkey, const int
     for (int k = 0; k < kGroupCap; ++k)
       if (k < n) L.at[k][lane] = (int)w[k];
     if (tie) {
-      auto key = [&](int place, T& d, uint32_t& id) {
-        const Pt4<PT> p = pts[place];
-        d = dist2(V3<T>{(T)p.x, (T)p.y, (T)p.z}, q);
+      auto key = [&](int place, float& d, uint32_t& id) {
+        const Pt4<float> p = pts[place];
+        d = dist2(V3<float>{p.x, p.y, p.z}, q);
         id = p.id;
       };
       for (int t = 1; t < n; ++t) {
         const int place = L.at[t][lane];
-        T d;
+        float d;
         uint32_t id;
         key(place, d, id);
         int s = t;
         for (; s > 0; --s) {
           const int before = L.at[s - 1][lane];
-          T db;
+          float db;
           uint32_t ib;
           key(before, db, ib);
           if (db < d || (db == d && ib < id)) break;

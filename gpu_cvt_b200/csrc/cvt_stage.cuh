@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(32, 20) k_stage_knn_group(const GridGeom* geom
       thr = (1.3f * 11.f / 3.14159265f) * (float)kk * G.h * G.h / (float)near;
       rad = query_radius(G, q, thr);
     }
-    const bool ok = group_knn<float, float>(G, 0, cell_start, sorted, in, q, thr, rad, 0xffffffffu, kk, L);
+    const bool ok = group_knn(G, cell_start, sorted, in, q, thr, rad, kk, L);
     const unsigned left = __ballot_sync(0xffffffffu, in && !ok);
     if (left) {
       int base = 0;
