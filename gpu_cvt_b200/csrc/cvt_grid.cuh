@@ -228,57 +228,70 @@ __device__ __forceinline__ DKey shfl_up_key(DKey k) {
 __device__ __forceinline__ unsigned long long min_key(unsigned long long) { return 0ull; }
 __device__ __forceinline__ DKey min_key(DKey) { return {-INFINITY, 0u}; }
 
-// Visit the candidates of Chebyshev ring r around (cx,cy,cz) in chunks of 32:
-// every lane calls visit(pos) the same number of times, pos = a sorted
-// position or -1.  The ring's cell ranges (two slots per (z,y) row: the whole
-// x-range for rows on the shell's faces, else the two end cells) are spread
-// over the lanes, their lengths warp-scanned, and each lane finds the range of
-// its candidate by a shuffle binary search over the prefix sums.
+// Points of slot `slot` of Chebyshev ring r around (cx,cy,cz): two slots per
+// (z,y) row, the whole x-range for rows on the shell's faces, else the two end
+// cells.  nslots: slots of the ring.
+struct RingSlots {
+  int cx, cy, cz, r, x0, x1, y0, z0, ny, nslots;
+  __device__ __forceinline__ RingSlots(const GridGeom& g, int cx_, int cy_, int cz_, int r_)
+      : cx(cx_), cy(cy_), cz(cz_), r(r_), x0(max(cx_ - r_, 0)), x1(min(cx_ + r_, g.dim[0] - 1)), y0(max(cy_ - r_, 0)),
+        z0(max(cz_ - r_, 0)), ny(min(cy_ + r_, g.dim[1] - 1) - y0 + 1),
+        nslots(2 * (min(cz_ + r_, g.dim[2] - 1) - z0 + 1) * ny) {}
+  __device__ __forceinline__ void range(const GridGeom& g, const int* __restrict__ cell_start, int slot, int& b, int& e) const {
+    b = e = 0;
+    if (slot >= nslots) return;
+    const int rowi = slot >> 1, which = slot & 1;
+    const int z = z0 + rowi / ny, y = y0 + rowi % ny;
+    const int row = g.cell_base + (z * g.dim[1] + y) * g.dim[0];
+    const bool full_row = (r == 1) || abs(z - cz) == r || abs(y - cy) == r;
+    if (full_row) {
+      if (which == 0) { b = __ldg(cell_start + row + x0); e = __ldg(cell_start + row + x1 + 1); }
+    } else {
+      const int x = which == 0 ? cx - r : cx + r;
+      if (x >= 0 && x < g.dim[0]) { b = __ldg(cell_start + row + x); e = __ldg(cell_start + row + x + 1); }
+    }
+  }
+};
+
+// Visit the points of the lanes' ranges [b, e) in chunks of 32: every lane calls
+// visit(pos) the same number of times, pos = a sorted position or -1.  The
+// lengths are warp-scanned, and each lane finds the range of its candidate by a
+// shuffle binary search over the prefix sums.
+template <class Visit>
+__device__ __forceinline__ void warp_ranges(int b, int e, int lane, Visit&& visit) {
+  const int len = e - b;
+  int incl = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const int excl = incl - len;
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  for (int c = 0; c < total; c += 32) {
+    const int i = c + lane;
+    int lo = 0;
+#pragma unroll
+    for (int step = 16; step >= 1; step >>= 1) {
+      const int probe = lo + step;
+      const int ex = __shfl_sync(0xffffffffu, excl, probe & 31);
+      if (probe < 32 && ex <= i) lo = probe;
+    }
+    const int rb = __shfl_sync(0xffffffffu, b, lo);
+    const int rex = __shfl_sync(0xffffffffu, excl, lo);
+    visit(i < total ? rb + (i - rex) : -1);
+  }
+}
+
+// Visit the candidates of ring r, its slots spread over the lanes.
 template <class Visit>
 __device__ __forceinline__ void warp_ring(const GridGeom& g, const int* __restrict__ cell_start, int cx, int cy,
                                           int cz, int r, int lane, Visit&& visit) {
-  const int z0 = max(cz - r, 0), z1 = min(cz + r, g.dim[2] - 1);
-  const int y0 = max(cy - r, 0), y1 = min(cy + r, g.dim[1] - 1);
-  const int x0 = max(cx - r, 0), x1 = min(cx + r, g.dim[0] - 1);
-  const int ny = y1 - y0 + 1;
-  const int nslots = 2 * (z1 - z0 + 1) * ny;
-  for (int base = 0; base < nslots; base += 32) {
-    const int slot = base + lane;
-    int b = 0, e = 0;
-    if (slot < nslots) {
-      const int rowi = slot >> 1, which = slot & 1;
-      const int z = z0 + rowi / ny, y = y0 + rowi % ny;
-      const int row = g.cell_base + (z * g.dim[1] + y) * g.dim[0];
-      const bool full_row = (r == 1) || abs(z - cz) == r || abs(y - cy) == r;
-      if (full_row) {
-        if (which == 0) { b = __ldg(cell_start + row + x0); e = __ldg(cell_start + row + x1 + 1); }
-      } else {
-        const int x = which == 0 ? cx - r : cx + r;
-        if (x >= 0 && x < g.dim[0]) { b = __ldg(cell_start + row + x); e = __ldg(cell_start + row + x + 1); }
-      }
-    }
-    const int len = e - b;
-    int incl = len;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    const int excl = incl - len;
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    for (int c = 0; c < total; c += 32) {
-      const int i = c + lane;
-      int lo = 0;
-#pragma unroll
-      for (int step = 16; step >= 1; step >>= 1) {
-        const int probe = lo + step;
-        const int ex = __shfl_sync(0xffffffffu, excl, probe & 31);
-        if (probe < 32 && ex <= i) lo = probe;
-      }
-      const int rb = __shfl_sync(0xffffffffu, b, lo);
-      const int rex = __shfl_sync(0xffffffffu, excl, lo);
-      visit(i < total ? rb + (i - rex) : -1);
-    }
+  const RingSlots R(g, cx, cy, cz, r);
+  for (int base = 0; base < R.nslots; base += 32) {
+    int b, e;
+    R.range(g, cell_start, base + lane, b, e);
+    warp_ranges(b, e, lane, visit);
   }
 }
 
