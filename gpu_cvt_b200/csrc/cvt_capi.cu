@@ -179,14 +179,17 @@ static int wave_blocks(long n, int threads) { return std::min(cdiv(n, threads), 
 // remesh.)
 struct ThreadStreams {
   cudaStream_t side = nullptr, cap = nullptr, cap_side = nullptr;
+  std::vector<cudaStream_t> ingest;  // of cvt_remesh_batch's ingest threads, at most kIngestThreads
 };
 struct ThreadStreamSet {
   std::vector<ThreadStreams> dev;
   ~ThreadStreamSet() {
     std::lock_guard<std::mutex> lk(g_capture_mu);
-    for (ThreadStreams& t : dev)
+    for (ThreadStreams& t : dev) {
       for (cudaStream_t s : {t.side, t.cap, t.cap_side})
         if (s) cudaStreamDestroy(s);
+      for (cudaStream_t s : t.ingest) cudaStreamDestroy(s);
+    }
   }
 };
 static cudaError_t thread_streams(ThreadStreams** out) {
@@ -2280,35 +2283,37 @@ extern "C" cvt_status_t cvt_remesh_batch(int n_meshes, const float* const* V, co
   // Mesh ingest, many meshes at once: each host thread takes meshes off a
   // shared counter and ingests them on its own non-blocking stream (one
   // mesh's ingest is a chain of small kernels and host reads that leaves the
-  // GPU idle most of the time; 256 meshes took 83 ms one after another).
+  // GPU idle most of the time; 256 meshes took 83 ms one after another).  The
+  // streams belong to the calling thread and stay for its next call: made by
+  // each ingest thread, under the capture lock that the others take for every
+  // allocation, the last ones came milliseconds late.
   {
     int dev = 0;
+    ThreadStreams* ts = nullptr;
     if (cudaGetDevice(&dev) != cudaSuccess) return fail(CVT_ERR_CUDA, "cvt_remesh_batch: no device");
+    CK(thread_streams(&ts));
+    const int nth = std::min(n_meshes, kIngestThreads);
+    if ((int)ts->ingest.size() < nth) {
+      std::lock_guard<std::mutex> lk(g_capture_mu);
+      while ((int)ts->ingest.size() < nth) {
+        cudaStream_t st;
+        CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        ts->ingest.push_back(st);
+      }
+    }
     std::vector<cvt_status_t> ms(n_meshes, CVT_OK);
     std::vector<std::string> merr(n_meshes);
     std::atomic<int> next{0};
-    auto ingest = [&]() {
-      cudaStream_t st = nullptr;
-      cudaError_t made = cudaSetDevice(dev);
-      if (made == cudaSuccess) {
-        std::lock_guard<std::mutex> lk(g_capture_mu);
-        made = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-      }
-      if (made != cudaSuccess) {
-        for (int i; (i = next++) < n_meshes;) { ms[i] = CVT_ERR_CUDA; merr[i] = "cvt_remesh_batch: stream creation failed"; }
-        return;
-      }
+    auto ingest = [&](int t) {
+      const bool on = cudaSetDevice(dev) == cudaSuccess;
       for (int i; (i = next++) < n_meshes;) {
-        ms[i] = mesh_create_on(V[i], nV[i], F[i], nF[i], &meshes[i], st);
+        ms[i] = on ? mesh_create_on(V[i], nV[i], F[i], nF[i], &meshes[i], ts->ingest[t]) : fail(CVT_ERR_CUDA, "cvt_remesh_batch: no device");
         if (ms[i] != CVT_OK) merr[i] = g_last_error;
       }
-      std::lock_guard<std::mutex> lk(g_capture_mu);
-      cudaStreamDestroy(st);
     };
-    const int nth = std::min(n_meshes, kIngestThreads);
     std::vector<std::thread> pool;
-    for (int t = 1; t < nth; ++t) pool.emplace_back(ingest);
-    ingest();
+    for (int t = 1; t < nth; ++t) pool.emplace_back(ingest, t);
+    ingest(0);
     for (std::thread& t : pool) t.join();
     for (int i = 0; i < n_meshes && s == CVT_OK; ++i)
       if (ms[i] != CVT_OK) s = fail(ms[i], merr[i]);
