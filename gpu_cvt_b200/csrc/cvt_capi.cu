@@ -115,8 +115,8 @@ static cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t st) {
 
 // Held while an iteration is captured and its graph instantiated or updated,
 // and around the library's device-wide waits, the release of its long-lived
-// memory and of cached memory, and the creation and release of streams, events
-// and graphs: with one thread capturing and another waiting for the device,
+// memory and of cached memory, and the release of streams, events and graphs
+// (and where events and the threads' own streams are made): with one thread capturing and another waiting for the device,
 // tearing an engine down or ending (its streams go), the driver failed the
 // capture or crashed (two threads that create, run and destroy engines: within
 // 150 rounds).  One lock for the process: a thread that has a graph to capture
@@ -179,17 +179,14 @@ static int wave_blocks(long n, int threads) { return std::min(cdiv(n, threads), 
 // remesh.)
 struct ThreadStreams {
   cudaStream_t side = nullptr, cap = nullptr, cap_side = nullptr;
-  std::vector<cudaStream_t> ingest;  // of cvt_remesh_batch's ingest threads, at most kIngestThreads
 };
 struct ThreadStreamSet {
   std::vector<ThreadStreams> dev;
   ~ThreadStreamSet() {
     std::lock_guard<std::mutex> lk(g_capture_mu);
-    for (ThreadStreams& t : dev) {
+    for (ThreadStreams& t : dev)
       for (cudaStream_t s : {t.side, t.cap, t.cap_side})
         if (s) cudaStreamDestroy(s);
-      for (cudaStream_t s : t.ingest) cudaStreamDestroy(s);
-    }
   }
 };
 static cudaError_t thread_streams(ThreadStreams** out) {
@@ -2243,6 +2240,21 @@ extern "C" cvt_status_t cvt_remesh(const float* V, int nV, const int* F, int nF,
 // Host threads that ingest the meshes of one cvt_remesh_batch call.
 constexpr int kIngestThreads = 8;
 
+// Their streams: each thread makes its own, and the calling thread releases all
+// under one hold of the capture lock when the threads have ended.  (Made under
+// the lock, against threads that take it for every allocation, the last began
+// milliseconds late: 32 small meshes, one iteration 9.2 to 13.0 ms instead of
+// 8.0; kept for the next call, eight live streams made every evaluation 180 us
+// longer.)
+struct IngestStreams {
+  cudaStream_t st[kIngestThreads] = {};
+  ~IngestStreams() {
+    std::lock_guard<std::mutex> lk(g_capture_mu);
+    for (cudaStream_t s : st)
+      if (s) cudaStreamDestroy(s);
+  }
+};
+
 // The sites of every reserved segment (slot order) from its host array.
 static cvt_status_t upload_and_place(cvt_engine* e, const int* seg, int n, const float* const* sites, const int* n_sites) {
   cudaStream_t st = S_(nullptr);
@@ -2283,31 +2295,20 @@ extern "C" cvt_status_t cvt_remesh_batch(int n_meshes, const float* const* V, co
   // Mesh ingest, many meshes at once: each host thread takes meshes off a
   // shared counter and ingests them on its own non-blocking stream (one
   // mesh's ingest is a chain of small kernels and host reads that leaves the
-  // GPU idle most of the time; 256 meshes took 83 ms one after another).  The
-  // streams belong to the calling thread and stay for its next call: made by
-  // each ingest thread, under the capture lock that the others take for every
-  // allocation, the last ones came milliseconds late.
+  // GPU idle most of the time; 256 meshes took 83 ms one after another).
   {
     int dev = 0;
-    ThreadStreams* ts = nullptr;
     if (cudaGetDevice(&dev) != cudaSuccess) return fail(CVT_ERR_CUDA, "cvt_remesh_batch: no device");
-    CK(thread_streams(&ts));
     const int nth = std::min(n_meshes, kIngestThreads);
-    if ((int)ts->ingest.size() < nth) {
-      std::lock_guard<std::mutex> lk(g_capture_mu);
-      while ((int)ts->ingest.size() < nth) {
-        cudaStream_t st;
-        CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-        ts->ingest.push_back(st);
-      }
-    }
+    IngestStreams streams;
     std::vector<cvt_status_t> ms(n_meshes, CVT_OK);
     std::vector<std::string> merr(n_meshes);
     std::atomic<int> next{0};
     auto ingest = [&](int t) {
-      const bool on = cudaSetDevice(dev) == cudaSuccess;
+      const bool on = cudaSetDevice(dev) == cudaSuccess && cudaStreamCreateWithFlags(&streams.st[t], cudaStreamNonBlocking) == cudaSuccess;
       for (int i; (i = next++) < n_meshes;) {
-        ms[i] = on ? mesh_create_on(V[i], nV[i], F[i], nF[i], &meshes[i], ts->ingest[t]) : fail(CVT_ERR_CUDA, "cvt_remesh_batch: no device");
+        ms[i] = on ? mesh_create_on(V[i], nV[i], F[i], nF[i], &meshes[i], streams.st[t])
+                   : fail(CVT_ERR_CUDA, "cvt_remesh_batch: stream creation failed");
         if (ms[i] != CVT_OK) merr[i] = g_last_error;
       }
     };
