@@ -12,9 +12,9 @@
 // left to the caller (one warp per query).
 //
 // Bound by issue: of about 310 warp instructions per query (K = 33) half are
-// the walk.  1M points, K = 33: 1.05 ms and 0.10 for the queries left over; a
-// sorted list per thread in registers, one insertion per accepted candidate of
-// any lane, took 2.17.  (Tried for the engine's full searches too: its cells,
+// the walk.  1M points, K = 33: 1.05 ms and 0.10 for the queries left over
+// (1.25 with the grid build); a sorted list per thread in registers, one
+// insertion per accepted candidate of any lane, took 2.17.  (Tried for the engine's full searches too: its cells,
 // sized for K + 1 sites, make the union walk twice as long, no faster than a
 // warp per site.)
 #pragma once

@@ -154,12 +154,13 @@ __global__ void __launch_bounds__(128) k_stage_knn_points(const GridGeom* geom, 
 constexpr int kQueryRings = 1;
 
 // Cell ranges that a warp looks up for a query before it scans all points, per
-// point.  30k queries, k = 5, rings / scans / one thread each (ms): 14 cells off
-// 164k points 0.40, 10.6, 4.0; 40 cells off 1M points 2.7, 65, 36; a query with
-// only empty cells around it pays for the rings and the scan (60 cells inside
-// the sphere of 164k points 14.7, 11.0, 100; with 1/2 a query 60 cells off 20k
-// points takes 2.7 instead of 1.6).
+// point.  30k queries, k = 5 (ms), by rings, one thread each, scans alone: 14
+// cells off 164k points 0.42, 4.1, 10.5; 40 cells off 1M points 2.7, 36, 65.  A
+// query with only empty cells around it pays for the rings and the scan: 60
+// cells inside the sphere of 164k points 10.2 together (100 by one thread each).
+// 1/2 instead: 60 cells off 20k points 2.7 instead of 1.6.
 constexpr float kFarLookups = 0.125f;
+
 template <int KK>
 __global__ void __launch_bounds__(128) k_stage_knn_query(const GridGeom* geom, const int* __restrict__ cell_start,
                                                          const Pt4<float>* __restrict__ sorted, const float* __restrict__ Q,
